@@ -20,12 +20,11 @@ from types import SimpleNamespace
 
 import torch
 
-import infernum_b200 as ib
 from infernum_b200.cache import CacheManager
 from infernum_b200.engine.step import ModelRunner, StepContext, StepEntry
 from infernum_b200.models.model import Model
 from infernum_b200.ops import core
-from infernum_b200.parts.base import BLOCKS, EMBEDDINGS, NORMS, LayerSpec, PartSpec, Runtime, build_layer, build_part
+from infernum_b200.parts.base import EMBEDDINGS, NORMS, LayerSpec, PartSpec, Runtime, build_layer, build_part
 from infernum_b200.registry import resolve_config
 
 PAGE = 16
@@ -51,27 +50,27 @@ def listed():
     layer = dict(kind="layer", dtype="bfloat16")
     return [
         # one request of a small model being decoded: the least work a step can be, all of it latency
-        dict(layer, name="layer decode 1, 1B", width=2048, requests=1, tokens=1, past=700),
+        dict(layer, name="layer decode 1 1B", width=2048, requests=1, tokens=1, past=700),
         # a server's ordinary step: many requests of uneven lengths, a token each
-        dict(layer, name="layer decode 64, 8B", width=4096, requests=64, tokens=64, past=1100),
+        dict(layer, name="layer decode 64 8B", width=4096, requests=64, tokens=64, past=1100),
         # a long prompt, as large as a step gets
-        dict(layer, name="layer prompt 2048, 8B", width=4096, requests=1, tokens=2048, past=0),
+        dict(layer, name="layer prompt 2048 8B", width=4096, requests=1, tokens=2048, past=0),
         # the true 32-bit engine: two prompts in one step, and a few requests being decoded
-        dict(layer, name="layer prompts f32, 1B", dtype="float32", width=2048, requests=2, tokens=700, past=0),
-        dict(layer, name="layer decode 8 f32, 1B", dtype="float32", width=2048, requests=8, tokens=8, past=500),
+        dict(layer, name="layer prompts f32 1B", dtype="float32", width=2048, requests=2, tokens=700, past=0),
+        dict(layer, name="layer decode 8 f32 1B", dtype="float32", width=2048, requests=8, tokens=8, past=500),
         # attention through a latent: a long prompt, and eight requests being decoded
-        dict(kind="latent", name="latent prompt 2048, 8B", width=4096, requests=1, tokens=2048, past=0),
-        dict(kind="latent", name="latent decode 8, 8B", width=4096, requests=8, tokens=8, past=1024),
+        dict(kind="latent", name="latent prompt 2048 8B", width=4096, requests=1, tokens=2048, past=0),
+        dict(kind="latent", name="latent decode 8 8B", width=4096, requests=8, tokens=8, past=1024),
         # sixteen experts of which a token uses four: a long prompt; a few decoded tokens, with an expert for all
-        dict(kind="experts", name="experts prompt 2048, 8B", width=4096, rule="softmax_top", ff=3584, experts=16,
+        dict(kind="experts", name="experts prompt 2048 8B", width=4096, rule="softmax_top", ff=3584, experts=16,
              top=4, shared=0, tokens=2048),
-        dict(kind="experts", name="experts decode 8, 2B", width=2048, rule="softmax_all", ff=1024, experts=16,
+        dict(kind="experts", name="experts decode 8 2B", width=2048, rule="softmax_all", ff=1024, experts=16,
              top=4, shared=4096, tokens=8),
         # recurrent mixers: a long prompt through a state space layer, two prompts through a delta rule
-        dict(kind="state", name="ssd prompt 2048, 2B", width=2048, rule="ssd", requests=1, tokens=2048),
-        dict(kind="state", name="delta prompts 1500, 2B", width=2048, rule="delta", requests=2, tokens=1500),
+        dict(kind="state", name="ssd prompt 2048 2B", width=2048, rule="ssd", requests=1, tokens=2048),
+        dict(kind="state", name="delta prompts 1500 2B", width=2048, rule="delta", requests=2, tokens=1500),
         # a whole decoder: three prompts that arrive together, odd lengths
-        dict(kind="model", name="model prompts, 1B", width=2048, layers=8, vocab=32000, requests=3, tokens=1019),
+        dict(kind="model", name="model prompts 1B", width=2048, layers=8, vocab=32000, requests=3, tokens=1019),
     ]
 
 
