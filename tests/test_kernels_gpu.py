@@ -151,6 +151,27 @@ def test_gemm_plain(M, N, K, dt):
         assert torch.equal(one[0], out[M - 1])
 
 
+@pytest.mark.parametrize("M, N, K", [(1, 16, 4), (3, 8192, 64), (8, 2048, 2048), (7, 8200, 260), (9, 31, 128),
+                                     (16, 100, 132), (13, 9000, 128), (17, 48, 1024), (32, 33, 260), (30, 8300, 36),
+                                     (33, 3072, 516), (64, 2048, 64), (65, 64, 20), (130, 1030, 1024), (300, 129, 1028),
+                                     (700, 3072, 256), (257, 16384, 64)])
+def test_gemm_plain_in_32_bit_gives_the_same_bits_by_every_kernel(M, N, K):
+    """One ascending chain of multiply-adds an output: the kernels for few and for many rows, which take aligned
+    operands, against the general one, which an odd row stride asks for."""
+    c = core()
+    a, w = torch.randn(M, K, device=DEV), torch.randn(N, K, device=DEV)
+    odd = torch.full((N, K + 1), float("nan"), device=DEV)
+    odd[:, :K] = w
+    out = torch.full((M, N + 3), float("nan"), device=DEV)
+    ref = torch.empty(M, N, device=DEV)
+    c.gemm_plain(a, w, out[:, :N])       # rows of the result further apart than they are long
+    c.gemm_plain(a, odd[:, :K], ref)
+    assert torch.equal(out[:, :N], ref) and bool(out[:, N:].isnan().all())
+    even = torch.empty(M, N, device=DEV)
+    c.gemm_plain(a, w, even)
+    assert torch.equal(even, ref)
+
+
 def test_argmax_lowest_index_wins():
     c = core()
     x = torch.randn(6, 1000)
