@@ -1,0 +1,472 @@
+// Attention over the paged cache in true 32-bit, for heads of 64 and 128 whose keys and values have one size: the
+// arithmetic of attention_plain.cu (scores, running maximum, expf, sums all 32-bit; the same keys visible to a query),
+// spread so that the multiply-adds of a tile share their operands.  Two kernels:
+//
+//   attention_f32_tile_kernel  prompts.  A CTA owns 64 packed rows - query rows of one request times the query heads of
+//       one key/value head - and walks the keys in tiles of 64, two stages deep by cp.async.  A warp owns 16 rows, so
+//       the softmax needs no barrier; a thread has 4 rows x 8 keys of the scores and 4 rows x HD/8 of the result, and
+//       loads 12 pieces of 16 bytes from shared memory for 128 multiply-adds.  Bound by the multiply-adds.
+//       Where a query does not see all keys of a tile, unseen keys are left out of its sum (not multiplied by zero).
+//   attention_f32_rows_kernel  decoded tokens.  A CTA has a slice of one row's keys for up to four query heads of one
+//       key/value head: HD/4 lanes a key, four keys of each warp in flight, and the slices of a row are the CTAs of a
+//       cluster that merge through distributed shared memory.  Bound by the keys' and values' bytes.
+//
+// Both read past the L1 (see gemm_plain.cu: they may begin under an earlier kernel's tail).
+#include "common.cuh"
+
+using namespace ib;
+
+namespace {
+
+struct F32Params {
+    const float* q;
+    const float* k_pool;
+    const float* v_pool;
+    float* out;
+    const int* positions;   // [rows]
+    const int* row_entry;   // [rows]
+    const int* cu_rows;     // [entries + 1]
+    const int* q_start;     // [entries]
+    const int* tables;      // [entries][max_blocks]
+    const float* sink;      // [nh] or null
+    unsigned* err;
+    int q_stride, out_stride, max_blocks, nh, nkv, page_size, num_pages, window, keep_first;
+    float scale;
+};
+
+__device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void cp_async16(void* smem, const void* gmem, int bytes) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(smem_u32(smem)), "l"(gmem), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
+
+// Where key j of an entry lies (in units of a head's vectors); -1, and the error word, for a page that is none.
+__device__ __forceinline__ long long key_place(const F32Params& p, const int* table, int g, int j) {
+    const int b = j / p.page_size;
+    const int page = b < p.max_blocks ? table[b] : -1;
+    if (page < 0 || page >= p.num_pages) {
+        atomicOr(p.err, IB_FLAG_BAD_PAGE);
+        return -1;
+    }
+    return ((long long)page * p.nkv + g) * p.page_size + (j - b * p.page_size);
+}
+
+constexpr int ROWS = 64, KEYS = 64, P_PITCH = KEYS + 8;
+template <int HD>
+struct TileSmem {
+    static constexpr int PITCH = HD + 4;   // of queries and keys: eight keys' 16-byte loads lie in different banks
+    static constexpr int Q = ROWS * PITCH, K = KEYS * PITCH, V = KEYS * HD, P = 4 * 16 * P_PITCH;
+    static constexpr int BYTES = (Q + 2 * K + 2 * V + P + 2 * KEYS) * (int)sizeof(float);
+};
+
+template <int HD>
+__global__ void __launch_bounds__(128) attention_f32_tile_kernel(const F32Params p) {
+    using S = TileSmem<HD>;
+    extern __shared__ __align__(16) float smem[];
+    float* qs = smem;
+    float* ks = qs + S::Q;
+    float* vs = ks + 2 * S::K;
+    float* ps = vs + 2 * S::V;
+    int* held = reinterpret_cast<int*>(ps + S::P);  // [2][KEYS]: the key exists
+    const int g = blockIdx.x, e = blockIdx.y;
+    const int group = p.nh / p.nkv;
+    const int first = p.cu_rows[e], rows = p.cu_rows[e + 1] - first;
+    const int tiles = (rows * group + ROWS - 1) / ROWS;
+    const int tile = tiles - 1 - (int)blockIdx.z;   // the last rows, which see the most keys, begin first
+    if (tile < 0) return;
+    const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32, ly = lane / 8, lx = lane % 8;
+    const int packed0 = tile * ROWS, packed_end = min(packed0 + ROWS, rows * group);
+    const int start = p.q_start[e];
+    const int pos0 = start + packed0 / group, pos1 = start + (packed_end - 1) / group;  // first and last query's place
+    const int lo0 = p.window > 0 ? max(0, pos0 - p.window + 1) : 0;   // the first query's first key inside the window
+    const int kept = p.window > 0 ? max(p.keep_first, 0) : 0;         // keys below stay visible behind a window
+    const int kept_tiles = min(lo0, kept) > 0 ? (min(lo0, kept) + KEYS - 1) / KEYS : 0;
+    const int t_lo = max(lo0 / KEYS, kept_tiles), t_end = pos1 / KEYS + 1;
+    const int* table = p.tables + (size_t)e * p.max_blocks;
+
+    // queries of this tile (rows past the end repeat the last one)
+    for (int c = tid; c < ROWS * (HD / 4); c += 128) {
+        const int r = c / (HD / 4), d = (c % (HD / 4)) * 4;
+        const int pr = min(packed0 + r, packed_end - 1);
+        cp_async16(qs + r * S::PITCH + d,
+                   p.q + (size_t)(first + pr / group) * p.q_stride + (size_t)(g * group + pr % group) * HD + d, 16);
+    }
+    auto fetch = [&](int t, int buf) {
+        for (int i = tid / (HD / 4); i < KEYS; i += 128 / (HD / 4)) {
+            const int j = t * KEYS + i, d = (tid % (HD / 4)) * 4;
+            // (a key that some query of the tile sees: its page is followed; the others' are not looked up)
+            long long at = -1;
+            if (j <= pos1 && (j >= lo0 || j < kept)) at = key_place(p, table, g, j);
+            const size_t src = (size_t)(at < 0 ? 0 : at) * HD + d;
+            cp_async16(ks + buf * S::K + i * S::PITCH + d, p.k_pool + src, at < 0 ? 0 : 16);
+            cp_async16(vs + buf * S::V + i * HD + d, p.v_pool + src, at < 0 ? 0 : 16);
+            if (d == 0) held[buf * KEYS + i] = at >= 0;
+        }
+        cp_async_commit();
+    };
+    int row_pos[4];
+    float m[4], l[4], acc[4][HD / 8];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        row_pos[i] = start + min(packed0 + warp * 16 + i * 4 + ly, packed_end - 1) / group;
+        m[i] = -INFINITY;
+        l[i] = 0.f;
+#pragma unroll
+        for (int c = 0; c < HD / 8; ++c) acc[i][c] = 0.f;
+    }
+    const float* qw = qs + (warp * 16 + ly) * S::PITCH;
+    float* pw = ps + warp * 16 * P_PITCH;
+
+    int t = kept_tiles > 0 ? 0 : t_lo, buf = 0;
+    if (t < t_end) fetch(t, 0);
+    while (t < t_end) {
+        const int next = t + 1 == kept_tiles ? t_lo : t + 1;
+        cp_async_wait_all();
+        __syncthreads();   // the tile has come, and the other stage is read by all
+        if (next < t_end) fetch(next, buf ^ 1);
+        const float* kt = ks + buf * S::K + lx * S::PITCH;
+        float s[4][8];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 8; ++j) s[i][j] = 0.f;
+#pragma unroll 2
+        for (int d = 0; d < HD; d += 4) {
+            float4 a[4], b[8];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) a[i] = *reinterpret_cast<const float4*>(qw + i * 4 * S::PITCH + d);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) b[j] = *reinterpret_cast<const float4*>(kt + j * 8 * S::PITCH + d);
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    s[i][j] = fmaf(a[i].x, b[j].x, s[i][j]);
+                    s[i][j] = fmaf(a[i].y, b[j].y, s[i][j]);
+                    s[i][j] = fmaf(a[i].z, b[j].z, s[i][j]);
+                    s[i][j] = fmaf(a[i].w, b[j].w, s[i][j]);
+                }
+        }
+        // (all of the tile's keys are seen by every query of this warp, and exist)
+        const int wpos0 = start + min(packed0 + warp * 16, packed_end - 1) / group;
+        const int wpos1 = start + min(packed0 + warp * 16 + 15, packed_end - 1) / group;
+        bool mine = true;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) mine &= held[buf * KEYS + lx + 8 * j] != 0;
+        const bool whole = __all_sync(0xffffffffu, mine) && (t + 1) * KEYS - 1 <= wpos0 &&
+                           (p.window <= 0 || t * KEYS > wpos1 - p.window || (t + 1) * KEYS <= kept);
+        unsigned seen[4] = {0xffu, 0xffu, 0xffu, 0xffu};
+        if (!whole) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    const int key = t * KEYS + lx + 8 * j;
+                    const bool see = key <= row_pos[i] && held[buf * KEYS + lx + 8 * j] &&
+                                     (p.window <= 0 || key > row_pos[i] - p.window || key < kept);
+                    if (!see) seen[i] &= ~(1u << j);
+                }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            float top = m[i];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                s[i][j] = (seen[i] >> j) & 1u ? s[i][j] * p.scale : -INFINITY;
+                top = fmaxf(top, s[i][j]);
+            }
+#pragma unroll
+            for (int o = 1; o < 8; o <<= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+            const float ref = top == -INFINITY ? 0.f : top;   // (no key seen so far)
+            const float corr = expf(m[i] - ref);
+            m[i] = top;
+            float sum = 0.f;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const float w = expf(s[i][j] - ref);
+                sum += w;
+                pw[(i * 4 + ly) * P_PITCH + lx + 8 * j] = w;
+            }
+            l[i] = l[i] * corr + sum;
+#pragma unroll
+            for (int c = 0; c < HD / 8; ++c) acc[i][c] *= corr;
+        }
+        __syncwarp();
+        const float* vt = vs + buf * S::V + lx * 4;
+        const float* pr = pw + ly * P_PITCH;
+        if (whole) {
+#pragma unroll 2
+            for (int k = 0; k < KEYS; k += 4) {
+                float4 w[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) w[i] = *reinterpret_cast<const float4*>(pr + i * 4 * P_PITCH + k);
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+#pragma unroll
+                    for (int c = 0; c < HD / 32; ++c) {
+                        const float4 v = *reinterpret_cast<const float4*>(vt + (k + u) * HD + c * 32);
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            const float wi = u == 0 ? w[i].x : u == 1 ? w[i].y : u == 2 ? w[i].z : w[i].w;
+                            acc[i][4 * c] = fmaf(wi, v.x, acc[i][4 * c]);
+                            acc[i][4 * c + 1] = fmaf(wi, v.y, acc[i][4 * c + 1]);
+                            acc[i][4 * c + 2] = fmaf(wi, v.z, acc[i][4 * c + 2]);
+                            acc[i][4 * c + 3] = fmaf(wi, v.w, acc[i][4 * c + 3]);
+                        }
+                    }
+            }
+        } else {
+#pragma unroll 1
+            for (int k = 0; k < KEYS; ++k) {
+                const int key = t * KEYS + k;
+                if (!held[buf * KEYS + k]) continue;
+                float4 v[HD / 32];
+#pragma unroll
+                for (int c = 0; c < HD / 32; ++c) v[c] = *reinterpret_cast<const float4*>(vt + k * HD + c * 32);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    if (key > row_pos[i] || (p.window > 0 && key <= row_pos[i] - p.window && key >= kept)) continue;
+                    const float wi = pr[i * 4 * P_PITCH + k];
+#pragma unroll
+                    for (int c = 0; c < HD / 32; ++c) {
+                        acc[i][4 * c] = fmaf(wi, v[c].x, acc[i][4 * c]);
+                        acc[i][4 * c + 1] = fmaf(wi, v[c].y, acc[i][4 * c + 1]);
+                        acc[i][4 * c + 2] = fmaf(wi, v[c].z, acc[i][4 * c + 2]);
+                        acc[i][4 * c + 3] = fmaf(wi, v[c].w, acc[i][4 * c + 3]);
+                    }
+                }
+            }
+        }
+        __syncwarp();   // the warp's weights are read before the next tile's are written
+        t = next;
+        buf ^= 1;
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1) l[i] += __shfl_xor_sync(0xffffffffu, l[i], o);
+        const int pr = packed0 + warp * 16 + i * 4 + ly;
+        if (pr >= packed_end) continue;
+        const int head = g * group + pr % group;
+        float corr = 1.f;
+        if (p.sink) {
+            const float sk = p.sink[head], top = fmaxf(m[i], sk);
+            corr = expf(m[i] - top);
+            l[i] = l[i] * corr + expf(sk - top);
+        }
+        const float inv = l[i] > 0.f ? corr / l[i] : 0.f;
+        float* op = p.out + (size_t)(first + pr / group) * p.out_stride + (size_t)head * HD + lx * 4;
+#pragma unroll
+        for (int c = 0; c < HD / 32; ++c)
+            *reinterpret_cast<float4*>(op + c * 32) = make_float4(acc[i][4 * c] * inv, acc[i][4 * c + 1] * inv,
+                                                                  acc[i][4 * c + 2] * inv, acc[i][4 * c + 3] * inv);
+    }
+}
+
+template <int HD, int GB>
+__global__ void __launch_bounds__(128) attention_f32_rows_kernel(const F32Params p) {
+    pdl_trigger();
+    pdl_wait();
+    constexpr int LPK = HD / 4, SUBS = 32 / LPK, TEAMS = 4 * SUBS, AHEAD = 4;  // lanes a key, teams of them in a CTA
+    __shared__ __align__(16) float part_acc[TEAMS][GB][HD];
+    __shared__ float part_m[TEAMS][GB], part_l[TEAMS][GB];
+    __shared__ float all_acc[GB][HD], all_m[GB], all_l[GB];   // the CTA's share, read by the cluster's first CTA
+    const int splits = gridDim.x, slice = blockIdx.x;
+    const int group = p.nh / p.nkv, chunks = (group + GB - 1) / GB;
+    const int g = blockIdx.y / chunks, h0 = (blockIdx.y % chunks) * GB, heads = min(GB, group - h0);
+    const int row = blockIdx.z, tid = threadIdx.x, lane = tid % 32;
+    const int team = (tid / 32) * SUBS + lane / LPK, dl = (lane % LPK) * 4;
+    const int pos = p.positions[row];
+    const int* table = p.tables + (size_t)p.row_entry[row] * p.max_blocks;
+    const int lo = p.window > 0 ? max(0, pos - p.window + 1) : 0;
+    const int kept = min(max(p.keep_first, 0), lo);
+    const int n = pos < 0 ? 0 : kept + pos + 1 - lo;
+    const int per = (n + splits - 1) / splits, i0 = slice * per, i1 = min(n, i0 + per);
+
+    float4 q[GB];
+    float m[GB], l[GB];
+    float4 acc[GB];
+#pragma unroll
+    for (int h = 0; h < GB; ++h) {
+        q[h] = __ldcg(reinterpret_cast<const float4*>(p.q + (size_t)row * p.q_stride +
+                                                      (size_t)(g * group + h0 + min(h, heads - 1)) * HD + dl));
+        m[h] = -INFINITY;
+        l[h] = 0.f;
+        acc[h] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    for (int i = i0; i < i1; i += TEAMS * AHEAD) {   // (the same number of times for every lane: they shuffle)
+        float4 k[AHEAD], v[AHEAD];
+        bool in[AHEAD];
+#pragma unroll
+        for (int u = 0; u < AHEAD; ++u) {
+            const int at = i + u * TEAMS + team;
+            in[u] = at < i1;
+            k[u] = v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (in[u]) {
+                const long long place = key_place(p, table, g, at < kept ? at : lo + at - kept);
+                in[u] = place >= 0;
+                if (in[u]) {
+                    k[u] = __ldcg(reinterpret_cast<const float4*>(p.k_pool + (size_t)place * HD + dl));
+                    v[u] = __ldcg(reinterpret_cast<const float4*>(p.v_pool + (size_t)place * HD + dl));
+                }
+            }
+        }
+#pragma unroll
+        for (int h = 0; h < GB; ++h) {
+            float s[AHEAD], top = m[h];
+#pragma unroll
+            for (int u = 0; u < AHEAD; ++u) {
+                float d = q[h].x * k[u].x;
+                d = fmaf(q[h].y, k[u].y, d);
+                d = fmaf(q[h].z, k[u].z, d);
+                d = fmaf(q[h].w, k[u].w, d);
+#pragma unroll
+                for (int o = 1; o < LPK; o <<= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
+                s[u] = in[u] ? d * p.scale : -INFINITY;
+                top = fmaxf(top, s[u]);
+            }
+            const float ref = top == -INFINITY ? 0.f : top;
+            const float corr = expf(m[h] - ref);
+            m[h] = top;
+            l[h] *= corr;
+            acc[h].x *= corr; acc[h].y *= corr; acc[h].z *= corr; acc[h].w *= corr;
+#pragma unroll
+            for (int u = 0; u < AHEAD; ++u) {
+                const float w = expf(s[u] - ref);
+                l[h] += w;
+                acc[h].x = fmaf(w, v[u].x, acc[h].x);
+                acc[h].y = fmaf(w, v[u].y, acc[h].y);
+                acc[h].z = fmaf(w, v[u].z, acc[h].z);
+                acc[h].w = fmaf(w, v[u].w, acc[h].w);
+            }
+        }
+    }
+#pragma unroll
+    for (int h = 0; h < GB; ++h) {
+        *reinterpret_cast<float4*>(&part_acc[team][h][dl]) = acc[h];
+        if (dl == 0) {
+            part_m[team][h] = m[h];
+            part_l[team][h] = l[h];
+        }
+    }
+    __syncthreads();
+    for (int c = tid; c < GB * HD; c += 128) {
+        const int h = c / HD, d = c % HD;
+        float top = -INFINITY, sum = 0.f, a = 0.f;
+        for (int w = 0; w < TEAMS; ++w) top = fmaxf(top, part_m[w][h]);
+        const float ref = top == -INFINITY ? 0.f : top;
+        for (int w = 0; w < TEAMS; ++w) {
+            const float corr = expf(part_m[w][h] - ref);
+            sum = fmaf(part_l[w][h], corr, sum);
+            a = fmaf(part_acc[w][h][d], corr, a);
+        }
+        all_acc[h][d] = a;
+        if (d == 0) {
+            all_m[h] = top;
+            all_l[h] = sum;
+        }
+    }
+    // (a cluster of one CTA has the barrier of a block)
+    asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+    if (slice == 0) {
+        auto peer = [](const float* mine, int rank) {
+            unsigned at;
+            float v;
+            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(at) : "r"(smem_u32(mine)), "r"(rank));
+            asm volatile("ld.shared::cluster.f32 %0, [%1];\n" : "=f"(v) : "r"(at) : "memory");
+            return v;
+        };
+        for (int c = tid; c < heads * HD; c += 128) {
+            const int h = c / HD, d = c % HD, head = g * group + h0 + h;
+            float tops[8], top = p.sink ? p.sink[head] : -INFINITY;
+#pragma unroll
+            for (int r = 0; r < 8; ++r) {
+                tops[r] = r < splits ? peer(&all_m[h], r) : -INFINITY;
+                top = fmaxf(top, tops[r]);
+            }
+            const float ref = top == -INFINITY ? 0.f : top;
+            float sum = p.sink ? expf(p.sink[head] - ref) : 0.f, a = 0.f;
+#pragma unroll
+            for (int r = 0; r < 8; ++r)
+                if (r < splits) {
+                    const float corr = expf(tops[r] - ref);
+                    sum = fmaf(peer(&all_l[h], r), corr, sum);
+                    a = fmaf(peer(&all_acc[h][d], r), corr, a);
+                }
+            p.out[(size_t)row * p.out_stride + (size_t)head * HD + d] = sum > 0.f ? a / sum : 0.f;
+        }
+    }
+    asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");   // the shares are read
+    asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+}
+
+template <int HD>
+int launch_tiles(const F32Params& p, int n_entries, int max_rows, cudaStream_t s) {
+    static bool attr_done = false;
+    if (!attr_done) {
+        cudaError_t e = cudaFuncSetAttribute(attention_f32_tile_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             TileSmem<HD>::BYTES);
+        if (e != cudaSuccess) return (int)e;
+        attr_done = true;
+    }
+    const long long tiles = ((long long)max_rows * (p.nh / p.nkv) + ROWS - 1) / ROWS;
+    if (tiles > 65535 || n_entries > 65535) return IB_ERR_TOO_LARGE;
+    cudaError_t le = launch_kernel_in_order(attention_f32_tile_kernel<HD>, dim3(p.nkv, n_entries, (unsigned)tiles),
+                                            dim3(128), (size_t)TileSmem<HD>::BYTES, s, p);
+    if (le != cudaSuccess) return (int)le;
+    IB_LAUNCH_CHECK();
+    return IB_OK;
+}
+
+template <int HD, int GB>
+int launch_rows(const F32Params& p, int n_rows, int splits, cudaStream_t s) {
+    const int group = p.nh / p.nkv;
+    const long long y = (long long)p.nkv * ((group + GB - 1) / GB);
+    if (y > 65535 || n_rows > 65535) return IB_ERR_TOO_LARGE;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(splits, (unsigned)y, n_rows);
+    cfg.blockDim = dim3(128);
+    cfg.stream = s;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = splits;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = pdl_flag() ? 2 : 1;
+    cudaError_t le = cudaLaunchKernelEx(&cfg, attention_f32_rows_kernel<HD, GB>, p);
+    if (le != cudaSuccess) return (int)le;
+    IB_LAUNCH_CHECK();
+    return IB_OK;
+}
+
+}  // namespace
+
+// splits 1, 2, 4 or 8: the keys of each row in so many slices (decoded tokens); 0: tiles of 64 packed rows (prompts),
+// `max_rows` the most rows of an entry.  Pools contiguous [pages][nkv][page_size][hd]; rows of q and out 16-byte
+// aligned, hd 64 or 128.
+IB_EXPORT int ib_attention_f32(const float* q, int q_stride, const float* k_pool, const float* v_pool, float* out,
+                               int out_stride, const int* positions, const int* row_entry, const int* cu_rows,
+                               const int* q_start, const int* tables, int max_blocks, int n_entries, int n_rows,
+                               int max_rows, int nh, int nkv, int hd, int page_size, int num_pages, int window,
+                               float scale, const float* sink, int keep_first, int splits, unsigned* err, void* stream) {
+    if (n_rows <= 0 || n_entries <= 0) return IB_OK;
+    if (!q || !k_pool || !v_pool || !out || !positions || !row_entry || !cu_rows || !q_start || !tables || !err)
+        return IB_ERR_BAD_ARG;
+    if (nh <= 0 || nkv <= 0 || nh % nkv || page_size <= 0 || max_blocks <= 0 || num_pages <= 0 || max_rows <= 0)
+        return IB_ERR_BAD_ARG;
+    if ((hd != 64 && hd != 128) || q_stride % 4 || out_stride % 4 || ((uintptr_t)q & 15) || ((uintptr_t)out & 15) ||
+        ((uintptr_t)k_pool & 15) || ((uintptr_t)v_pool & 15))
+        return IB_ERR_UNSUPPORTED;
+    if (splits != 0 && splits != 1 && splits != 2 && splits != 4 && splits != 8) return IB_ERR_BAD_ARG;
+    const F32Params p{q, k_pool, v_pool, out, positions, row_entry, cu_rows, q_start, tables, sink, err, q_stride,
+                      out_stride, max_blocks, nh, nkv, page_size, num_pages, window, keep_first, scale};
+    cudaStream_t s = (cudaStream_t)stream;
+    if (splits == 0) return hd == 64 ? launch_tiles<64>(p, n_entries, max_rows, s) : launch_tiles<128>(p, n_entries, max_rows, s);
+    if (nh == nkv) return hd == 64 ? launch_rows<64, 1>(p, n_rows, splits, s) : launch_rows<128, 1>(p, n_rows, splits, s);
+    return hd == 64 ? launch_rows<64, 4>(p, n_rows, splits, s) : launch_rows<128, 4>(p, n_rows, splits, s);
+}

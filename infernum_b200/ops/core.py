@@ -16,7 +16,7 @@ import torch
 from ..csrc.build import load_module
 from ..errors import KernelError
 
-CORE_SOURCES = ["elementwise.cu", "attention_plain.cu", "gemm_plain.cu", "sampling.cu", "layernorm.cu",
+CORE_SOURCES = ["elementwise.cu", "attention_plain.cu", "attention_f32.cu", "gemm_plain.cu", "sampling.cu", "layernorm.cu",
                 "embed_hashed.cu", "latent.cu", "moe.cu", "hyper.cu", "recurrent.cu", "subnorm.cu", "shortconv.cu",
                 "attention_diff.cu", "attention_talk.cu"]
 
@@ -82,6 +82,11 @@ def core_lib() -> ctypes.CDLL:
                                           _c_void_p]
         lib.ib_feed_tokens.argtypes = [_c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_void_p, _c_int, _c_void_p,
                                        _c_void_p]
+        lib.ib_attention_f32.argtypes = [
+            _c_void_p, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_void_p,
+            _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_float,
+            _c_void_p, _c_int, _c_int, _c_void_p, _c_void_p]
+        lib.ib_attention_f32.restype = _c_int
         lib.ib_attention_plain_ex.argtypes = lib.ib_attention_plain.argtypes[:19] + [_c_int, _c_int, _c_int, _c_int,
                                                                                   _c_void_p, _c_void_p, _c_void_p]
         lib.ib_attention_plain_mask.argtypes = lib.ib_attention_plain.argtypes[:19] + [
@@ -536,6 +541,52 @@ def attention_plain(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor,
                                         block_tables.shape[1], N, n_heads, nkv, hd, page_size,
                                         num_pages, int(window), float(scale), err.data_ptr(),
                                         stream_ptr(q)), "attention_plain")
+
+
+def choose_f32_splits(max_rows_per_entry: int, n_rows: int, heads: int, kv_heads: int, max_kv_len: int,
+                      sm_count: int) -> int:
+    """How ``attention_f32`` spreads a step: 0 for tiles of 64 packed rows, or into how many slices (the CTAs of a
+    cluster: 1, 2, 4 or 8) the keys of every row are cut.  Up to four rows an entry go row by row: a tile would be
+    filled to a quarter at most with four query heads a key/value head, and its keys walked by one CTA (eight decoded
+    rows of the 1B shape at 500 keys: 12 us by rows in eight slices).  Slices as long as the SMs hold CTAs to take
+    them, and a slice keeps 64 keys."""
+    if max_rows_per_entry > 4:
+        return 0
+    group = heads // kv_heads
+    ctas = n_rows * kv_heads * (1 if group == 1 else -(-group // 4))
+    splits = 1
+    while splits < 8 and max_kv_len >= 128 * splits and ctas * splits < 4 * sm_count:
+        splits *= 2
+    return splits
+
+
+def attention_f32(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, out: torch.Tensor, ctx,
+                  block_tables: torch.Tensor, n_heads: int, scale: float, window: int, err: torch.Tensor,
+                  sink: Optional[torch.Tensor] = None, keep_first: int = 0, sm_count: int = 148) -> bool:
+    """``attention_plain`` for float32 steps whose keys and values have 64 or 128 elements, by the kernels of
+    ``attention_f32.cu``; False when the operands do not suit them (the caller then takes the plain kernel)."""
+    num_pages, nkv, page_size, hd = k_pool.shape
+    if q.dtype != torch.float32 or hd not in (64, 128) or v_pool.shape != k_pool.shape or n_heads % nkv \
+            or k_pool.dtype != torch.float32 or v_pool.dtype != torch.float32 or out.dtype != torch.float32 \
+            or not k_pool.is_contiguous() or not v_pool.is_contiguous() or q.stride(1) != 1 or out.stride(1) != 1 \
+            or q.stride(0) % 4 or out.stride(0) % 4 or q.shape[1] < n_heads * hd or out.shape[1] < n_heads * hd \
+            or any(t.data_ptr() % 16 for t in (q, k_pool, v_pool, out)) \
+            or max(q.shape[0], ctx.n_entries, n_heads) > 65535:
+        return False
+    require_cuda(q, k_pool, v_pool, out, ctx.positions, ctx.row_entry, block_tables, err, sink)
+    for t, name in ((ctx.positions, "positions"), (ctx.row_entry, "row_entry"), (ctx.cu_rows, "cu_rows"),
+                    (ctx.q_start, "q_start"), (block_tables, "block_tables")):
+        _int32(t, name)
+    if sink is not None and (sink.dtype != torch.float32 or sink.shape != (n_heads,) or not sink.is_contiguous()):
+        raise KernelError(f"attention_f32: sink must be contiguous float32 [{n_heads}]")
+    splits = choose_f32_splits(ctx.max_rows_per_entry, q.shape[0], n_heads, nkv, ctx.max_kv_len, sm_count)
+    check(core_lib().ib_attention_f32(
+        q.data_ptr(), q.stride(0), k_pool.data_ptr(), v_pool.data_ptr(), out.data_ptr(), out.stride(0),
+        ctx.positions.data_ptr(), ctx.row_entry.data_ptr(), ctx.cu_rows.data_ptr(), ctx.q_start.data_ptr(),
+        block_tables.data_ptr(), block_tables.shape[1], ctx.n_entries, q.shape[0], ctx.max_rows_per_entry, n_heads, nkv,
+        hd, page_size, num_pages, int(window), float(scale), _ptr(sink), int(keep_first), splits, err.data_ptr(),
+        stream_ptr(q)), "attention_f32")
+    return True
 
 
 def gemm_plain(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:

@@ -324,6 +324,37 @@ def test_attention_plain(dtype, nh, nkv, hd, ps, window):
     assert rel_err(out, plain_result(refs, window)) < (2e-6 if dtype == torch.float32 else 1e-2)
 
 
+@pytest.mark.parametrize("nh, nkv, hd, ps", [(8, 2, 64, 16), (4, 4, 128, 8), (5, 1, 64, 4), (6, 2, 128, 32), (8, 1, 64, 3)])
+@pytest.mark.parametrize("lens, rows", [([37, 1, 64, 5], [37, 1, 3, 2]), ([130, 65, 200, 128], [130, 64, 6, 1]),
+                                        ([700, 3, 129, 64], [1, 1, 1, 1]), ([300, 17], [4, 2])])
+@pytest.mark.parametrize("window, keep_first, sink", [(0, 0, False), (7, 0, True), (70, 3, False), (64, 66, True)])
+def test_attention_in_32_bit_tiles_and_rows(nh, nkv, hd, ps, lens, rows, window, keep_first, sink):
+    """The tile kernel (prompts) and the row kernel (few rows an entry) against the plain kernel, which rounds the same
+    sums in another order: 32-bit sums of some hundred terms, 2e-6 of the largest value.  Pages behind a window are
+    given back (-1) and every slot without a key is NaN; a key a query does not see may hold anything."""
+    c = core()
+    q, kp, vp, tables, ctx, _ = paged_case(lens, rows, nh, nkv, hd, ps, torch.float32, 3, poison=True)
+    for e, (L, n) in enumerate(zip(lens, rows)):
+        for b in range(tables.shape[1]):
+            if window and keep_first <= b * ps and (b + 1) * ps <= L - n - window + 1:
+                tables[e, b] = -1
+    s = torch.linspace(-1, 2, nh, device=DEV) if sink else None
+    err = c.new_error_word(DEV)
+    ref = torch.empty(q.shape[0], nh * hd, device=DEV)
+    c.attention_plain(q, kp, vp, ref, ctx.positions, ctx.row_entry, tables, nh, hd ** -0.5, window, err, sink=s,
+                      keep_first=keep_first)
+    out = torch.full_like(ref, float("nan"))
+    assert c.attention_f32(q, kp, vp, out, ctx, tables, nh, hd ** -0.5, window, err, sink=s, keep_first=keep_first)
+    assert err.item() == 0
+    assert rel_err(out, ref) < 2e-6
+    # the last token's value is an infinity: only the last query sees it
+    last = lens[0] - 1
+    vp[tables[0, last // ps], :, last % ps] = float("inf")
+    c.attention_f32(q, kp, vp, out, ctx, tables, nh, hd ** -0.5, window, err, sink=s, keep_first=keep_first)
+    rest = [r for r in range(q.shape[0]) if r != rows[0] - 1]
+    assert rel_err(out[rest], ref[rest]) < 2e-6 and not bool(out[rows[0] - 1].isfinite().any())
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_attention_plain_finds_a_far_key(dtype):
     """Among hundreds of keys one far key carries the answer."""
