@@ -35,6 +35,9 @@
 #define IB_SITE_ATTN_TC_LAYOUT 9     // attention_tcgen05: shared memory window not where the budget assumes
 #define IB_SITE_SPLIT_PRODUCER 10    // attention_mma split mode: TMA producer
 #define IB_SITE_SPLIT_COMPUTE 11     // attention_mma split mode: computing warps
+#define IB_SITE_GROUPED_PRODUCER 12  // gemm_grouped: TMA producer
+#define IB_SITE_GROUPED_MMA 13       // gemm_grouped: MMA issuer
+#define IB_SITE_GROUPED_EPILOGUE 14  // gemm_grouped: epilogue
 #define IB_TIMEOUT_AT(site) (IB_FLAG_WAIT_TIMEOUT | (1u << (8 + (site))))
 
 #define IB_EXPORT extern "C" __attribute__((visibility("default")))

@@ -1,0 +1,452 @@
+// Products of a mixture of experts, bf16, for steps of many tokens: every expert's rows (the tokens that chose it, side
+// by side) by that expert's weights, all experts in one launch:
+//
+//     out[s, n] = sum_k X[s, k] * W_e[n, k]      s in [offsets[e], offsets[e + 1])
+//
+// Tiles of 256 weight rows x up to `w_max` tokens, each computed by two CTAs of a cluster as one with
+// tcgen05.mma.cta_group::2.  The weight rows ride on the M side (128 a CTA) and the tokens on the N side, whose width
+// is any multiple of 16: an expert's tokens are cut into tiles of one width, so little is computed for padding (tokens
+// on the M side would be padded to 256 an expert, 25 % at 512 tokens an expert).  Which tiles there are is known to the
+// device only: every CTA works the list out from `offsets` and the pairs take the tiles in turn, so a recorded step
+// replays for other routings.
+//
+//   warp 0      TMA producer: its CTA's weight and token boxes of every k block, counted on the leader's barrier
+//   warp 1      allocates tensor memory; in the leader CTA one lane issues the MMAs
+//   warps 2..9  epilogue (two warps per 32 TMEM lanes, half of the tokens each), under the next tile's MMAs:
+//               lane = weight row, register = token.
+//               gated: a CTA's 128 weight rows are 64 gates and their 64 ups, which lie in other warps' lanes; the
+//               two warps of a pair hand each other half of sixteen tokens through shared memory, and each stores
+//               act(gate) * up * scale[token] as bf16;
+//               otherwise the accumulator is stored as it is, in float32, 128 bytes a warp and token.
+//
+// Every wait on an mbarrier is bounded; on a time-out the CTA sets IB_FLAG_WAIT_TIMEOUT, stops, frees its tensor memory
+// and returns.  Launched in order, as gemm_tcgen05_2cta.cu is and for its reason.
+#include "common.cuh"
+
+#include <cuda.h>
+
+using namespace ib;
+
+namespace {
+
+constexpr int BW = 128;        // weight rows per CTA (256 per pair): the M side
+constexpr int TILE = 256;      // weight rows, and most tokens, of a tile
+constexpr int BK = 64;
+constexpr int UMMA_K = 16;
+constexpr int STAGES = 6;
+constexpr int W_BYTES = BW * BK * 2;
+constexpr int STAGE_BYTES = W_BYTES + (TILE / 2) * BK * 2;   // 32 KiB
+constexpr int XCH_BYTES = 4 * 2 * 2 * 8 * 32 * 4;            // [pair of warps][buffer][direction][8 tokens][32 lanes]
+constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + XCH_BYTES + 1024;
+constexpr int NUM_THREADS = 320;
+constexpr unsigned TMEM_COLS = 512;   // two accumulators of 256 columns
+constexpr int MAX_EXPERTS = 256;
+constexpr unsigned PEER_BIT_MASK = 0xFEFFFFFFu;  // clears the CTA-rank bit of a shared::cluster address
+
+__device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ bool elect_one() {
+    unsigned pred = 0;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}\n" : "=r"(pred));
+    return pred != 0;
+}
+__device__ __forceinline__ unsigned cluster_ctarank() {
+    unsigned r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;\n" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void cluster_sync_all() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+}
+__device__ __forceinline__ void mbar_init(void* bar, unsigned count) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_u32(bar)), "r"(count));
+}
+__device__ __forceinline__ void mbar_expect_tx(void* bar, unsigned bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
+}
+// One arrival on the barrier at this offset in the leader CTA's shared memory.
+__device__ __forceinline__ void mbar_arrive_leader(void* bar) {
+    unsigned remote;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(remote) : "r"(smem_u32(bar)), "r"(0u));
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];\n" ::"r"(remote) : "memory");
+}
+__device__ __forceinline__ bool mbar_wait(void* bar, unsigned parity) {
+    return mbar_wait_bounded<false>(smem_u32(bar), parity);
+}
+// The same, when arrivals come from the other CTA of the pair too.
+__device__ __forceinline__ bool mbar_wait_cluster(void* bar, unsigned parity) {
+    return mbar_wait_bounded<true>(smem_u32(bar), parity);
+}
+// A box into this CTA's shared memory; the bytes are counted on the barrier at
+// the same offset in the leader CTA (rank bit cleared).
+__device__ __forceinline__ void tma_load_2d_pair(void* dst, const CUtensorMap* map, void* bar, int x, int y) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes "
+        "[%0], [%1, {%3, %4}], [%2];\n"
+        ::"r"(smem_u32(dst)), "l"(map), "r"(smem_u32(bar) & PEER_BIT_MASK), "r"(x), "r"(y) : "memory");
+}
+__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory"); }
+__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory"); }
+__device__ __forceinline__ void umma_bf16_pair(unsigned tmem_d, uint64_t adesc, uint64_t bdesc, unsigned idesc,
+                                               unsigned accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}\n"
+        ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
+}
+// Arrives, when the MMAs issued so far are done, on the barrier at this offset in
+// both CTAs of the pair.
+__device__ __forceinline__ void umma_commit_pair(void* bar) {
+    asm volatile(
+        "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n"
+        ::"r"(smem_u32(bar)), "h"((unsigned short)3) : "memory");
+}
+__device__ __forceinline__ void tmem_ld16(unsigned addr, unsigned (&r)[16]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(addr));
+}
+__device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory"); }
+
+__device__ __forceinline__ uint64_t desc_k_major(const void* tile) {
+    uint64_t d = 0;
+    d |= (uint64_t)((smem_u32(tile) >> 4) & 0x3FFF);
+    d |= (uint64_t)1 << 16;
+    d |= (uint64_t)(1024 >> 4) << 32;
+    d |= (uint64_t)1 << 46;
+    d |= (uint64_t)2 << 61;
+    return d;
+}
+// float32 accumulator, bf16 operands, both K-major, M = 256 (the pair), N = width.
+__device__ __forceinline__ unsigned instr_desc(int bn) {
+    return (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(bn >> 3) << 17) | ((unsigned)(TILE >> 4) << 24);
+}
+
+// Two warps agree on whether both go on.
+__device__ __forceinline__ bool pair_agrees(int id, bool ok) {
+    unsigned all;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.and.pred q, %2, 64, p;\n\t"
+        "selp.u32 %0, 1, 0, q;\n\t}\n"
+        : "=r"(all) : "r"(ok ? 1u : 0u), "r"(id) : "memory");
+    return all != 0;
+}
+__device__ __forceinline__ void pair_sync(int id) { asm volatile("bar.sync %0, 64;\n" ::"r"(id) : "memory"); }
+
+struct Params {
+    void* out;              // gated: bf16 [slots, ldo]; else float32
+    const int* offsets;     // [n_experts + 1]: where each expert's rows begin
+    const float* scale;     // gated, optional: out[s] *= scale[s * scale_stride]
+    unsigned* err;
+    int n_experts, N, K, ldo;   // N weight rows of an expert
+    int w_row_step, w_col_step; // where expert e's weights begin in W: row e * w_row_step, column e * w_col_step
+    int w_max;              // most tokens of a tile
+    int scale_stride;
+    int act;
+    float act_limit, act_alpha;
+};
+
+struct TileWalk {
+    // The tiles of expert e are start[e] .. start[e + 1): its weight tiles, and for each its token tiles.
+    const int* start;
+    const int* offsets;
+    int n_experts, w_max, e;
+    __device__ TileWalk(const int* s, const int* o, int n, int w) : start(s), offsets(o), n_experts(n), w_max(w), e(0) {}
+    struct Place { int e, row, t0, width, count; };   // row: first weight row; count: tokens there are
+    __device__ __forceinline__ Place at(int tile) {   // tiles are asked for in rising order
+        while (tile >= start[e + 1]) ++e;
+        const int rows = offsets[e + 1] - offsets[e], cuts = (rows + w_max - 1) / w_max;
+        const int width = max(32, ((rows + cuts - 1) / cuts + 15) & ~15);
+        const int r = tile - start[e], j = r % cuts;
+        Place p;
+        p.e = e;
+        p.row = (r / cuts) * TILE;
+        p.t0 = offsets[e] + j * width;
+        p.width = width;
+        p.count = min(width, offsets[e + 1] - p.t0);
+        return p;
+    }
+};
+
+template <bool GATED>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
+gemm_grouped_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
+                    const Params p) {
+    extern __shared__ unsigned char smem_dyn[];
+    unsigned char* smem = (unsigned char*)(((uintptr_t)smem_dyn + 1023) & ~(uintptr_t)1023);
+    __shared__ __align__(8) unsigned long long full_bar[STAGES];
+    __shared__ __align__(8) unsigned long long empty_bar[STAGES];
+    __shared__ __align__(8) unsigned long long acc_full[2];    // MMAs of a tile are done (both CTAs)
+    __shared__ __align__(8) unsigned long long acc_empty[2];   // leader: both epilogues have read it
+    __shared__ unsigned tmem_slot;
+    __shared__ int s_start[MAX_EXPERTS + 1], s_offsets[MAX_EXPERTS + 1];
+
+    pdl_trigger();
+    pdl_wait();   // every thread: the offsets, the tokens, and whoever still reads `out`
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const unsigned rank = cluster_ctarank();           // 0 = leader
+    const int n_pairs = gridDim.x >> 1;
+    const int first = blockIdx.x >> 1;
+    const int n_kblocks = (p.K + BK - 1) / BK;
+    const int x_box = p.w_max / 2;                     // token rows of a box
+
+    for (int i = threadIdx.x; i <= p.n_experts; i += NUM_THREADS) s_offsets[i] = __ldcg(p.offsets + i);
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < STAGES; ++s) {
+            mbar_init(&full_bar[s], 1);
+            mbar_init(&empty_bar[s], 1);
+        }
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(&acc_full[b], 1);
+            mbar_init(&acc_empty[b], 16);   // eight epilogue warps in each CTA
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+    }
+    __syncthreads();
+    if (warp == 2) {   // the tiles before each expert: a running sum by one warp
+        const int w_tiles = (p.N + TILE - 1) / TILE;
+        int before = 0;
+        for (int e0 = 0; e0 < p.n_experts; e0 += 32) {
+            const int e = e0 + lane;
+            int mine = e < p.n_experts ? (s_offsets[e + 1] - s_offsets[e] + p.w_max - 1) / p.w_max * w_tiles : 0;
+            const int own = mine;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int up = __shfl_up_sync(0xffffffffu, mine, o);
+                if (lane >= o) mine += up;
+            }
+            if (e < p.n_experts) s_start[e] = before + mine - own;
+            before += __shfl_sync(0xffffffffu, mine, 31);
+        }
+        if (lane == 0) s_start[p.n_experts] = before;
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;\n"
+                     ::"r"(smem_u32(&tmem_slot)), "r"(TMEM_COLS));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;\n" ::);
+    }
+    __syncwarp();
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync_all();   // both CTAs' barriers are initialised before anyone signals them
+    tc_fence_after();
+    const unsigned tmem = tmem_slot;
+    const int tiles = s_start[p.n_experts];
+    TileWalk walk(s_start, s_offsets, p.n_experts, p.w_max);
+
+    if (warp == 0) {
+        // ---- producer (both CTAs) ---------------------------------------------------
+        if (elect_one()) {
+            bool ok = true;
+            unsigned it = 0;   // k blocks loaded so far, over all tiles
+            for (int tile = first; tile < tiles && ok; tile += n_pairs) {
+                const TileWalk::Place at = walk.at(tile);
+                const int wr = at.e * p.w_row_step + at.row + (int)rank * BW, wc = at.e * p.w_col_step;
+                const int xr = at.t0 + (int)rank * (at.width >> 1);
+                for (int i = 0; i < n_kblocks; ++i, ++it) {
+                    const int s = it % STAGES;
+                    const unsigned round = it / STAGES;
+                    if (round > 0 && !mbar_wait(&empty_bar[s], (round - 1) & 1)) { ok = false; break; }
+                    unsigned char* ws = smem + (size_t)s * STAGE_BYTES;
+                    // the leader's barrier counts the bytes of both CTAs
+                    if (rank == 0) mbar_expect_tx(&full_bar[s], 2 * (W_BYTES + x_box * BK * 2));
+                    tma_load_2d_pair(ws, &map_w, &full_bar[s], wc + i * BK, wr);
+                    tma_load_2d_pair(ws + W_BYTES, &map_x, &full_bar[s], i * BK, xr);
+                }
+            }
+            if (!ok) atomicOr(p.err, IB_TIMEOUT_AT(IB_SITE_GROUPED_PRODUCER));
+        }
+    } else if (warp == 1) {
+        // ---- MMA issuer (leader CTA only) -----------------------------------------------
+        if (rank == 0 && elect_one()) {
+            bool ok = true;
+            unsigned it = 0, j = 0;
+            for (int tile = first; tile < tiles && ok; tile += n_pairs, ++j) {
+                const unsigned buf = j & 1;
+                const unsigned idesc = instr_desc(walk.at(tile).width);
+                if (j >= 2 && !mbar_wait_cluster(&acc_empty[buf], ((j >> 1) - 1) & 1)) { ok = false; break; }
+                tc_fence_after();
+                const unsigned acc = tmem + buf * TILE;
+                for (int i = 0; i < n_kblocks; ++i, ++it) {
+                    const int s = it % STAGES;
+                    if (!mbar_wait(&full_bar[s], (it / STAGES) & 1)) { ok = false; break; }
+                    tc_fence_after();
+                    unsigned char* ws = smem + (size_t)s * STAGE_BYTES;
+                    const uint64_t adesc = desc_k_major(ws);
+                    const uint64_t bdesc = desc_k_major(ws + W_BYTES);
+#pragma unroll
+                    for (int kk = 0; kk < BK / UMMA_K; ++kk)
+                        umma_bf16_pair(acc, adesc + 2 * kk, bdesc + 2 * kk, idesc, (i > 0 || kk > 0) ? 1u : 0u);
+                    umma_commit_pair(&empty_bar[s]);
+                }
+                if (ok) umma_commit_pair(&acc_full[buf]);
+            }
+            if (!ok) atomicOr(p.err, IB_TIMEOUT_AT(IB_SITE_GROUPED_MMA));
+        }
+    } else {
+        // ---- epilogue: my 128 weight rows x the tile's tokens, half of them per warp --------------
+        const int quad = warp & 3;
+        const int half = (warp - 2) >> 2;
+        const int id = 1 + half * 2 + (quad & 1);   // the barrier of the warps with a block's gates and their ups
+        float* xch = reinterpret_cast<float*>(smem + STAGES * STAGE_BYTES) + (id - 1) * (2 * 2 * 8 * 32);
+        bool ok = true;
+        unsigned j = 0, turn = 0;
+        for (int tile = first; tile < tiles && ok; tile += n_pairs, ++j) {
+            const unsigned buf = j & 1;
+            ok = mbar_wait(&acc_full[buf], (j >> 1) & 1);
+            if (GATED) ok = pair_agrees(id, ok);
+            if (!ok) break;
+            tc_fence_after();
+            const TileWalk::Place at = walk.at(tile);
+            const unsigned taddr = tmem + buf * TILE + ((unsigned)(quad * 32) << 16);
+            const int split = ((at.width >> 1) + 15) & ~15;   // tokens of the first half of the warps
+            const int c_end = min(half ? at.width : split, (at.count + 15) & ~15);
+            const int row = at.row + (int)rank * BW;           // first weight row of this CTA
+            for (int c = half ? split : 0; c < c_end; c += 16) {
+                unsigned v[16];
+                tmem_ld16(taddr + c, v);
+                tmem_ld_wait();
+                if (GATED) {
+                    // lanes of quads 0 and 1 hold gates, those of 2 and 3 their ups: the first keep tokens
+                    // 0..7 of the sixteen and hand over 8..15, the others the reverse
+                    const bool up = quad >= 2;
+                    float* give = xch + ((turn & 1) * 2 + (up ? 1 : 0)) * (8 * 32) + lane;
+                    const float* take = xch + ((turn & 1) * 2 + (up ? 0 : 1)) * (8 * 32) + lane;
+                    ++turn;
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) give[q * 32] = __uint_as_float(up ? v[q] : v[8 + q]);
+                    pair_sync(id);   // (two buffers: the one after next is written behind the next barrier)
+                    const int col = row / 2 + (quad & 1) * 32 + lane;
+                    bf16* out = (bf16*)p.out + col;
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) {
+                        const int t = c + (up ? 8 + q : q);
+                        const float mine = __uint_as_float(up ? v[8 + q] : v[q]), other = take[q * 32];
+                        if (t < at.count && row < p.N) {
+                            const size_t s = (size_t)(at.t0 + t);
+                            const float sc = p.scale ? __ldcg(p.scale + s * p.scale_stride) : 1.f;
+                            const float y = gate_times(up ? other : mine, up ? mine : other, p.act, p.act_limit, p.act_alpha);
+                            out[s * p.ldo] = __float2bfloat16_rn(y * sc);
+                        }
+                    }
+                } else {
+                    const int n = row + quad * 32 + lane;
+                    float* out = (float*)p.out + n;
+#pragma unroll
+                    for (int q = 0; q < 16; ++q)
+                        if (c + q < at.count && n < p.N) out[(size_t)(at.t0 + c + q) * p.ldo] = __uint_as_float(v[q]);
+                }
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_leader(&acc_empty[buf]);
+        }
+        if (!ok && lane == 0) atomicOr(p.err, IB_TIMEOUT_AT(IB_SITE_GROUPED_EPILOGUE));
+    }
+    __syncwarp();   // the elected lanes are back with their warps before the aligned instructions below
+    tc_fence_before();
+    cluster_sync_all();   // neither CTA leaves (or frees tensor memory) while the other may still use it
+    if (warp == 1) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(TMEM_COLS));
+    }
+}
+
+typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
+                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*,
+                                  CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion,
+                                  CUtensorMapFloatOOBfill);
+
+EncodeTiledFn get_encode_fn() {
+    static EncodeTiledFn fn = nullptr;
+    if (!fn) {
+        void* ptr = nullptr;
+        cudaDriverEntryPointQueryResult qres;
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &qres) == cudaSuccess &&
+            qres == cudaDriverEntryPointSuccess)
+            fn = (EncodeTiledFn)ptr;
+    }
+    return fn;
+}
+
+int make_map(CUtensorMap* map, const void* base, long long rows, long long cols, long long ld, int box_rows) {
+    EncodeTiledFn fn = get_encode_fn();
+    if (!fn) return IB_ERR_UNSUPPORTED;
+    cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
+    cuuint64_t strides[1] = {(cuuint64_t)ld * 2};
+    cuuint32_t box[2] = {(cuuint32_t)BK, (cuuint32_t)box_rows};
+    cuuint32_t estr[2] = {1, 1};
+    CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
+                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? IB_OK : IB_ERR_BAD_ARG;
+}
+
+template <bool GATED>
+int launch_grouped(const CUtensorMap& mw, const CUtensorMap& mx, const Params& p, int pairs, cudaStream_t stream) {
+    static bool attr_done = false;
+    if (!attr_done) {
+        cudaError_t e = cudaFuncSetAttribute(gemm_grouped_kernel<GATED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             SMEM_BYTES);
+        if (e != cudaSuccess) return (int)e;
+        attr_done = true;
+    }
+    cudaError_t le = launch_kernel_in_order(gemm_grouped_kernel<GATED>, dim3((unsigned)(pairs * 2)), dim3(NUM_THREADS),
+                                            (size_t)SMEM_BYTES, stream, mw, mx, p);
+    if (le != cudaSuccess) return (int)le;
+    IB_LAUNCH_CHECK();
+    return IB_OK;
+}
+
+}  // namespace
+
+// x bf16 [slots, K] (rows ldx apart), the rows of expert e from offsets[e] (int32 [n_experts + 1], on the device, rising,
+// offsets[n_experts] <= slots) on; W bf16 of `w_rows` x `w_cols` (rows ldw apart), expert e's N x K weights at row
+// e * w_row_step and column e * w_col_step (a multiple of 8).  act > 0 (gate_times' codes): N rows of 64 gates and their
+// 64 ups in turn, out bf16 [slots, ldo] of N / 2 columns, times scale[s * scale_stride] where given; act 0: out float32
+// [slots, ldo].  w_max: most tokens of a tile, 64, 128 or 256.
+IB_EXPORT int ib_gemm_grouped(const void* x, int ldx, int slots, const void* w, int ldw, int w_rows, int w_cols, void* out,
+                              int ldo, const int* offsets, int n_experts, int N, int K, int w_row_step, int w_col_step,
+                              int w_max, int act, float act_limit, float act_alpha, const float* scale, int scale_stride,
+                              int sm_count, unsigned* err, void* stream) {
+    if (slots <= 0 || N <= 0) return IB_OK;
+    if (!x || !w || !out || !offsets || !err || K <= 0 || n_experts <= 0 || sm_count < 2 || act < 0 || act > 3 ||
+        w_row_step < 0 || w_col_step < 0 || (w_max != 64 && w_max != 128 && w_max != 256))
+        return IB_ERR_BAD_ARG;
+    if (n_experts > MAX_EXPERTS) return IB_ERR_TOO_LARGE;
+    // expert e's weights lie inside W; a box that reaches past them (K no multiple of 64, N none of 256) meets the
+    // matrix's end (zeros), another expert's rows (not stored) or - columns - would meet another expert's values
+    if ((long long)(n_experts - 1) * w_row_step + N > w_rows || (long long)(n_experts - 1) * w_col_step + K > w_cols)
+        return IB_ERR_BAD_ARG;
+    if (((uintptr_t)x & 15) || ((uintptr_t)w & 15) || (ldx % 8) || (ldw % 8) || ldx < K || ldw < w_cols ||
+        (w_col_step % 8) || (w_col_step && K % BK) || (act && N % 128) || ldo < (act ? N / 2 : N))
+        return IB_ERR_UNSUPPORTED;
+    Params p;
+    p.out = out;
+    p.offsets = offsets;
+    p.scale = scale;
+    p.err = err;
+    p.n_experts = n_experts;
+    p.N = N;
+    p.K = K;
+    p.ldo = ldo;
+    p.w_row_step = w_row_step;
+    p.w_col_step = w_col_step;
+    p.w_max = w_max;
+    p.scale_stride = scale_stride;
+    p.act = act;
+    p.act_limit = act_limit;
+    p.act_alpha = act_alpha;
+    CUtensorMap mw, mx;
+    int rc = make_map(&mw, w, w_rows, w_cols, ldw, BW);
+    if (rc != IB_OK) return rc;
+    rc = make_map(&mx, x, slots, K, ldx, w_max / 2);
+    if (rc != IB_OK) return rc;
+    const long long most = ((long long)slots / w_max + n_experts) * ((N + TILE - 1) / TILE);
+    if (most > 0x3fffffffLL) return IB_ERR_TOO_LARGE;
+    const int pairs = (int)(most < sm_count / 2 ? most : sm_count / 2);
+    return act ? launch_grouped<true>(mw, mx, p, pairs, (cudaStream_t)stream)
+               : launch_grouped<false>(mw, mx, p, pairs, (cudaStream_t)stream);
+}

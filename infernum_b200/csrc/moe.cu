@@ -378,3 +378,167 @@ IB_EXPORT int ib_moe_combine(const void* routed, const void* h, int h_stride, co
     IB_LAUNCH_CHECK();
     return IB_OK;
 }
+
+// Who goes where: the (token, choice) pairs side by side expert by expert, in the order of the tokens.  By one CTA: a warp
+// takes a run of tokens, counts its pairs per expert, and - once the counts before it are known - hands out places.
+//   offsets[E + 3]    where each expert's rows begin, the last one's end; then 0 and N, the same for one expert of all rows
+//   slot_of[N, top]   a pair's row, -1 where there is none (an output without an expert; an expert named again later in
+//                     the row, whose last weight counts, as in the dense row of weights)
+//   slot_scale[...]   a row's weight
+constexpr int SORT_WARPS = 32;
+__global__ void __launch_bounds__(SORT_WARPS * 32)
+moe_sort_kernel(const int* __restrict__ ids, const float* __restrict__ weights, int n_rows, int top, int E,
+                int* __restrict__ offsets, int* __restrict__ slot_of, float* __restrict__ slot_scale) {
+    pdl_trigger();
+    pdl_wait();
+    extern __shared__ int place[];   // [SORT_WARPS][E]: a warp's pairs of an expert, then its next free row
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    int* mine = place + warp * E;
+    for (int e = lane; e < E; e += 32) mine[e] = 0;
+    __syncwarp();
+    const int groups = (n_rows + 31) / 32, per = (groups + SORT_WARPS - 1) / SORT_WARPS;
+    const int g0 = warp * per, g1 = min(groups, g0 + per);
+    auto chosen = [&](int row, int k) {   // the pair's expert, E for none
+        if (row >= n_rows) return E;
+        const int* r = ids + (size_t)row * top;
+        const int e = __ldcg(r + k);
+        if (e < 0 || e >= E) return E;
+        for (int j = k + 1; j < top; ++j)
+            if (__ldcg(r + j) == e) return E;
+        return e;
+    };
+    for (int g = g0; g < g1; ++g)
+        for (int k = 0; k < top; ++k) {
+            const int e = chosen(g * 32 + lane, k);
+            const unsigned same = __match_any_sync(0xffffffffu, e);
+            if (e < E && lane == __ffs(same) - 1) mine[e] += __popc(same);
+            __syncwarp();
+        }
+    __syncthreads();
+    if (warp == 0) {
+        int before = 0;
+        for (int e0 = 0; e0 < E; e0 += 32) {
+            const int e = e0 + lane;
+            int total = 0;
+            if (e < E)
+                for (int w = 0; w < SORT_WARPS; ++w) total += place[w * E + e];
+            int sum = total;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int up = __shfl_up_sync(0xffffffffu, sum, o);
+                if (lane >= o) sum += up;
+            }
+            int at = before + sum - total;
+            if (e < E) {
+                offsets[e] = at;
+                for (int w = 0; w < SORT_WARPS; ++w) {
+                    const int n = place[w * E + e];
+                    place[w * E + e] = at;
+                    at += n;
+                }
+            }
+            before += __shfl_sync(0xffffffffu, sum, 31);
+        }
+        if (lane == 0) {
+            offsets[E] = before;
+            offsets[E + 1] = 0;
+            offsets[E + 2] = n_rows;
+        }
+    }
+    __syncthreads();
+    for (int g = g0; g < g1; ++g)
+        for (int k = 0; k < top; ++k) {
+            const int row = g * 32 + lane, e = chosen(row, k);
+            const unsigned same = __match_any_sync(0xffffffffu, e);
+            const int rank = __popc(same & ((1u << lane) - 1u));
+            const int at = e < E ? mine[e] + rank : -1;
+            __syncwarp();
+            if (e < E && rank == 0) mine[e] += __popc(same);
+            __syncwarp();
+            if (row < n_rows) {
+                slot_of[(size_t)row * top + k] = at;
+                if (at >= 0) slot_scale[at] = __ldcg(weights + (size_t)row * top + k);
+            }
+        }
+}
+
+IB_EXPORT int ib_moe_sort(const int* ids, const float* weights, int n_rows, int top, int E, int* offsets, int* slot_of,
+                          float* slot_scale, void* stream) {
+    if (n_rows <= 0) return IB_OK;
+    if (!ids || !weights || !offsets || !slot_of || !slot_scale || top <= 0 || E <= 0) return IB_ERR_BAD_ARG;
+    if (E > 256) return IB_ERR_TOO_LARGE;
+    cudaError_t le = launch_kernel(moe_sort_kernel, dim3(1), dim3(SORT_WARPS * 32), (size_t)SORT_WARPS * E * sizeof(int),
+                                   (cudaStream_t)stream, ids, weights, n_rows, top, E, offsets, slot_of, slot_scale);
+    if (le != cudaSuccess) return (int)le;
+    IB_LAUNCH_CHECK();
+    return IB_OK;
+}
+
+// Every token's row to the places of its pairs: xs[slot_of[n, k], :] = x[n, :], bf16, sixteen bytes a thread.
+__global__ void moe_scatter_rows_kernel(const bf16* __restrict__ x, int ldx, const int* __restrict__ slot_of, int top,
+                                        bf16* __restrict__ xs, int W) {
+    pdl_trigger();
+    pdl_wait();
+    const int row = blockIdx.x;
+    const int* to = slot_of + (size_t)row * top;
+    for (int c = threadIdx.x * 8; c < W; c += blockDim.x * 8) {
+        const uint4 v = __ldcg(reinterpret_cast<const uint4*>(x + (size_t)row * ldx + c));
+        for (int k = 0; k < top; ++k) {
+            const int s = __ldcg(to + k);
+            if (s >= 0) *reinterpret_cast<uint4*>(xs + (size_t)s * W + c) = v;
+        }
+    }
+}
+
+IB_EXPORT int ib_moe_scatter_rows(const void* x, int ldx, const int* slot_of, int top, void* xs, int n_rows, int W,
+                                  void* stream) {
+    if (n_rows <= 0) return IB_OK;
+    if (!x || !slot_of || !xs || top <= 0 || W <= 0 || ldx < W) return IB_ERR_BAD_ARG;
+    if (W % 8 || ldx % 8 || ((uintptr_t)x & 15) || ((uintptr_t)xs & 15)) return IB_ERR_UNSUPPORTED;
+    cudaError_t le = launch_kernel(moe_scatter_rows_kernel, dim3(n_rows), dim3(W >= 4096 ? 512 : W >= 2048 ? 256 : 128), 0,
+                                   (cudaStream_t)stream, (const bf16*)x, ldx, slot_of, top, (bf16*)xs, W);
+    if (le != cudaSuccess) return (int)le;
+    IB_LAUNCH_CHECK();
+    return IB_OK;
+}
+
+// out[n, :] = sum_k parts[slot_of[n, k], :] (+ shared[n, :]), the float32 results of a token's experts in the order of
+// its choices, one rounding to bf16 at the store.
+__global__ void moe_gather_sum_kernel(const float* __restrict__ parts, const int* __restrict__ slot_of, int top,
+                                      const float* __restrict__ shared, bf16* __restrict__ out, int W) {
+    pdl_trigger();
+    pdl_wait();
+    const int row = blockIdx.x;
+    const int* from = slot_of + (size_t)row * top;
+    for (int c = threadIdx.x * 4; c < W; c += blockDim.x * 4) {
+        float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+        for (int k = 0; k < top; ++k) {
+            const int s = __ldcg(from + k);
+            if (s < 0) continue;
+            const float4 v = __ldcg(reinterpret_cast<const float4*>(parts + (size_t)s * W + c));
+            a.x += v.x; a.y += v.y; a.z += v.z; a.w += v.w;
+        }
+        if (shared) {
+            const float4 v = __ldcg(reinterpret_cast<const float4*>(shared + (size_t)row * W + c));
+            a.x += v.x; a.y += v.y; a.z += v.z; a.w += v.w;
+        }
+        __nv_bfloat162 lo = __floats2bfloat162_rn(a.x, a.y), hi = __floats2bfloat162_rn(a.z, a.w);
+        uint2 packed;
+        packed.x = *reinterpret_cast<unsigned*>(&lo);
+        packed.y = *reinterpret_cast<unsigned*>(&hi);
+        *reinterpret_cast<uint2*>(out + (size_t)row * W + c) = packed;
+    }
+}
+
+IB_EXPORT int ib_moe_gather_sum(const float* parts, const int* slot_of, int top, const float* shared, void* out, int n_rows,
+                                int W, void* stream) {
+    if (n_rows <= 0) return IB_OK;
+    if (!parts || !slot_of || !out || top <= 0 || W <= 0) return IB_ERR_BAD_ARG;
+    if (W % 4 || ((uintptr_t)parts & 15) || ((uintptr_t)shared & 15) || ((uintptr_t)out & 7)) return IB_ERR_UNSUPPORTED;
+    cudaError_t le = launch_kernel(moe_gather_sum_kernel, dim3(n_rows), dim3(W >= 4096 ? 512 : W >= 2048 ? 256 : 128), 0,
+                                   (cudaStream_t)stream, parts, slot_of, top, shared, (bf16*)out, W);
+    if (le != cudaSuccess) return (int)le;
+    IB_LAUNCH_CHECK();
+    return IB_OK;
+}

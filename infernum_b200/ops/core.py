@@ -34,7 +34,8 @@ TIMEOUT_SITES = ["product for few tokens: producer", "product for few tokens: MM
                  "product on SM pairs: MMA issuer", "product on SM pairs: epilogue",
                  "prompt attention: producer", "prompt attention: MMA issuer", "prompt attention: softmax",
                  "prompt attention: shared memory window misplaced", "decode attention: producer",
-                 "decode attention: computing warps"]
+                 "decode attention: computing warps",
+                 "experts' product: producer", "experts' product: MMA issuer", "experts' product: epilogue"]
 
 
 def describe_flags(flags: int) -> str:
@@ -82,6 +83,11 @@ def core_lib() -> ctypes.CDLL:
                                           _c_void_p]
         lib.ib_feed_tokens.argtypes = [_c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_void_p, _c_int, _c_void_p,
                                        _c_void_p]
+        lib.ib_moe_sort.argtypes = [_c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_void_p]
+        lib.ib_moe_scatter_rows.argtypes = [_c_void_p, _c_int, _c_void_p, _c_int, _c_void_p, _c_int, _c_int, _c_void_p]
+        lib.ib_moe_gather_sum.argtypes = [_c_void_p, _c_void_p, _c_int, _c_void_p, _c_void_p, _c_int, _c_int, _c_void_p]
+        for fn in ("ib_moe_sort", "ib_moe_scatter_rows", "ib_moe_gather_sum"):
+            getattr(lib, fn).restype = _c_int
         lib.ib_attention_f32.argtypes = [
             _c_void_p, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_void_p,
             _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_float,
@@ -1418,6 +1424,46 @@ def moe_route_softmax_all(logits: torch.Tensor, correction: Optional[torch.Tenso
                                               gate.shape[1] if gate is not None else int(experts), int(groups), int(keep),
                                               int(group_top), 1 if renorm else 0, N, stream_ptr(logits)),
           "moe_route_softmax_all")
+
+
+def moe_sort(ids: torch.Tensor, weights: torch.Tensor, experts: int):
+    """The (token, choice) pairs of ``ids`` / ``weights`` [N, top] side by side expert by expert: ``offsets`` int32
+    [experts + 1], ``whole`` int32 (0, N), ``slot_of`` int32 [N, top] (a pair's row, -1 where it has none) and ``scale``
+    float32 [N top], a row's weight."""
+    require_cuda(ids, weights)
+    N, top = ids.shape
+    _int32(ids, "ids")
+    if weights.shape != (N, top) or weights.dtype != torch.float32 or not weights.is_contiguous():
+        raise KernelError("moe_sort: weights must be contiguous float32 [N, top]")
+    ints = torch.empty(experts + 3 + N * top, dtype=torch.int32, device=ids.device)
+    offsets, slot_of = ints[: experts + 3], ints[experts + 3:].view(N, top)
+    scale = torch.empty(N * top, dtype=torch.float32, device=ids.device)
+    check(core_lib().ib_moe_sort(ids.data_ptr(), weights.data_ptr(), N, top, int(experts), offsets.data_ptr(),
+                                 slot_of.data_ptr(), scale.data_ptr(), stream_ptr(ids)), "moe_sort")
+    return offsets[: experts + 1], offsets[experts + 1:], slot_of, scale
+
+
+def moe_scatter_rows(x: torch.Tensor, slot_of: torch.Tensor, out: torch.Tensor) -> None:
+    """out[slot_of[n, k]] = x[n] (bfloat16 rows; places of -1 are left out)."""
+    require_cuda(x, slot_of, out)
+    N, W = x.shape
+    if x.dtype != torch.bfloat16 or out.dtype != x.dtype or x.stride(1) != 1 or out.shape != (slot_of.numel(), W) \
+            or not out.is_contiguous() or not slot_of.is_contiguous():
+        raise KernelError("moe_scatter_rows: x bfloat16 [N, W], out contiguous bfloat16 [N top, W]")
+    check(core_lib().ib_moe_scatter_rows(x.data_ptr(), x.stride(0), slot_of.data_ptr(), slot_of.shape[1], out.data_ptr(),
+                                         N, W, stream_ptr(out)), "moe_scatter_rows")
+
+
+def moe_gather_sum(parts: torch.Tensor, slot_of: torch.Tensor, shared: Optional[torch.Tensor], out: torch.Tensor) -> None:
+    """out[n] = sum_k parts[slot_of[n, k]] (+ shared[n]): float32 rows summed in 32-bit, rounded once to bfloat16."""
+    require_cuda(parts, slot_of, shared, out)
+    N, W = out.shape
+    if parts.dtype != torch.float32 or parts.shape != (slot_of.numel(), W) or not parts.is_contiguous() \
+            or slot_of.shape[0] != N or not slot_of.is_contiguous() or out.dtype != torch.bfloat16 or not out.is_contiguous() \
+            or (shared is not None and (shared.shape != (N, W) or shared.dtype != torch.float32 or not shared.is_contiguous())):
+        raise KernelError("moe_gather_sum: parts float32 [N top, W], shared float32 [N, W], out bfloat16 [N, W]")
+    check(core_lib().ib_moe_gather_sum(parts.data_ptr(), slot_of.data_ptr(), slot_of.shape[1], _ptr(shared), out.data_ptr(),
+                                       N, W, stream_ptr(out)), "moe_gather_sum")
 
 
 def moe_combine(routed: Optional[torch.Tensor], h: torch.Tensor, shared: Optional[torch.Tensor], extra: torch.Tensor,

@@ -26,6 +26,7 @@ from . import core
 _c_int, _c_void_p, _c_ll, _c_float = ctypes.c_int, ctypes.c_void_p, ctypes.c_longlong, ctypes.c_float
 _lib: Optional[ctypes.CDLL] = None
 _pair_lib: Optional[ctypes.CDLL] = None
+_grouped_lib: Optional[ctypes.CDLL] = None
 _workspaces: Dict[torch.device, dict] = {}
 
 BM, BK = 128, 64
@@ -89,6 +90,20 @@ def pair_lib() -> ctypes.CDLL:
         lib()  # the SM count
         _pair_lib = l
     return _pair_lib
+
+
+def grouped_lib() -> ctypes.CDLL:
+    """The experts' products (``gemm_grouped.cu``)."""
+    global _grouped_lib
+    if _grouped_lib is None:
+        l = load_module("gemm_grouped", ["gemm_grouped.cu"])
+        l.ib_gemm_grouped.argtypes = [_c_void_p, _c_int, _c_int, _c_void_p, _c_int, _c_int, _c_int, _c_void_p, _c_int,
+                                      _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_float, _c_float,
+                                      _c_void_p, _c_int, _c_int, _c_void_p, _c_void_p]
+        l.ib_gemm_grouped.restype = _c_int
+        lib()  # the SM count
+        _grouped_lib = l
+    return _grouped_lib
 
 
 def _error_word(device) -> torch.Tensor:
@@ -226,6 +241,51 @@ def gemm_pair(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor,
                                           core.stream_ptr(x), float(act_limit), float(act_alpha),
                                           -(-N // 16) * 16 if limit_col is None else int(limit_col), float(act_limit2))
     core.check(code, "gemm_pair")
+
+
+def grouped_tile(rows: int, experts: int) -> int:
+    """Most tokens of a tile of ``gemm_grouped``: as many as an expert has on average, so that the boxes of tokens that
+    are fetched are not mostly another expert's."""
+    mean = rows / max(experts, 1)
+    return 256 if mean > 96 else 128 if mean > 40 else 64
+
+
+def gemm_grouped(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, offsets: torch.Tensor, n: int, row_step: int,
+                 col_step: int, tile: int, err: Optional[torch.Tensor] = None, act: int = 0, act_limit: float = 0.0,
+                 act_alpha: float = 0.0, scale: Optional[torch.Tensor] = None) -> None:
+    """``out[s] = x[s] @ W_e^T`` for the rows ``s`` in ``[offsets[e], offsets[e + 1])`` of every expert: ``W_e`` are the
+    ``n`` rows of ``w`` from ``e * row_step`` on, ``x``'s width of its columns from ``e * col_step`` on.  ``act`` (a code
+    of ``GATE_CODES``): 64 gate rows and their 64 up rows in turn, out bfloat16, every row times ``scale[s]``
+    (float32, any stride); 0: out float32."""
+    core.require_cuda(x, w, out, offsets, scale)
+    slots, K = x.shape
+    E = offsets.numel() - 1
+    if offsets.dtype != torch.int32 or not offsets.is_contiguous() or E < 1:
+        raise KernelError("gemm_grouped: offsets must be contiguous int32 [experts + 1]")
+    if x.dtype != torch.bfloat16 or w.dtype != torch.bfloat16 or x.stride(1) != 1 or w.stride(1) != 1 or out.stride(1) != 1 \
+            or out.shape != (slots, n // 2 if act else n) or out.dtype != (torch.bfloat16 if act else torch.float32):
+        raise KernelError("gemm_grouped: x and w bfloat16, out bfloat16 [rows, n / 2] with a gate, else float32 [rows, n]")
+    if scale is not None and (scale.dtype != torch.float32 or scale.dim() != 1 or scale.shape[0] < slots):
+        raise KernelError("gemm_grouped: scale must be float32 with a value a row")
+    code = grouped_lib().ib_gemm_grouped(
+        x.data_ptr(), x.stride(0), slots, w.data_ptr(), w.stride(0), w.shape[0], w.shape[1], out.data_ptr(), out.stride(0),
+        offsets.data_ptr(), E, int(n), K, int(row_step), int(col_step), int(tile), int(act), float(act_limit),
+        float(act_alpha), scale.data_ptr() if scale is not None else None, scale.stride(0) if scale is not None else 0,
+        POLICY["sm_count"], (err if err is not None else _error_word(x.device)).data_ptr(), core.stream_ptr(x))
+    core.check(code, "gemm_grouped")
+
+
+def grouped_suits(x: torch.Tensor, w1: torch.Tensor, w2: torch.Tensor, expert_size: int, experts: int, top: int,
+                  activation: str) -> bool:
+    """Whether a step's experts run by ``gemm_grouped`` (each token through the experts it chose) instead of as one wide
+    feed-forward (every expert for every token, times a zero where it was not chosen).  Above the tokens that the
+    weight-streaming kernel takes, and where at most half of the experts are chosen: the rows are copied to their
+    experts and the results come back in float32, 20 bytes a chosen expert and value of a row."""
+    return (POLICY["mode"] not in ("none", "cublas", "library") and activation in GATE_CODES
+            and x.shape[0] > POLICY["max_tokens"] and 2 * top <= experts <= 256 and expert_size % 64 == 0
+            and x.dtype == w1.dtype == w2.dtype == torch.bfloat16 and x.shape[1] % 8 == 0
+            and x.stride(1) == 1 and x.stride(0) % 8 == 0 and w1.stride(0) % 8 == 0 and w2.stride(0) % 8 == 0
+            and not any(t.data_ptr() % 16 for t in (x, w1, w2)))
 
 
 def route(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, err: Optional[torch.Tensor] = None) -> bool:

@@ -12,8 +12,8 @@ as ``[hidden, experts * ff]``; one product gives every expert's gate and up
 values, the activation kernel multiplies each expert's run of ``ff`` outputs by
 the token's weight for that expert (0 where it was not chosen), and the down
 product sums over all experts at once: ``sum_e Wd_e (w_e a_e)`` is one product
-with the concatenated vector.  Every expert is computed for every token; what
-a token did not choose is multiplied by an exact 0.
+with the concatenated vector.  What a token did not choose is multiplied by an exact 0.
+Steps of many tokens run each token through the experts it chose only (``grouped``).
 
 Parameters: ``hidden_size``, ``expert_size`` (ff), ``experts``, ``top``,
 ``activation`` ("silu" | "gelu_tanh" | "clamped_swish" with ``limit`` and ``alpha``), ``prefix``, ``expert_names`` (format of
@@ -203,16 +203,51 @@ class MixtureOfExperts(FeedForward):
             core.moe_route(logits, self.router_bias, self.top, ids, wts, gate)
         return ids, wts, gate
 
-    def forward(self, x: torch.Tensor, ctx=None) -> torch.Tensor:
-        _ids, _wts, gate = self.route(x)
+    def grouped(self, x: torch.Tensor, ids: torch.Tensor, wts: torch.Tensor, gate: torch.Tensor) -> torch.Tensor:
+        """The experts' weighted sum with every token run through the experts it chose only: the tokens' rows side by
+        side expert by expert, two products over all experts, the float32 results summed token by token.  An
+        expert that every token uses runs as one more pair of products on the rows as they are."""
+        from ..ops import gemm_tc
+
+        E, f, h, N = self.experts, self.expert_size, self.hidden_size, x.shape[0]
+        w1, w2, dev = self.gate_up.weight, self.down.weight, x.device
+        act = {"act": gemm_tc.GATE_CODES[self.activation], "act_alpha": self.alpha}
+        offsets, whole, slot_of, scale = core.moe_sort(ids, wts, E)
+        rows = slot_of.numel()
+        tile = gemm_tc.grouped_tile(rows, E)
+        xs = torch.empty((rows, h), dtype=x.dtype, device=dev)
+        core.moe_scatter_rows(x, slot_of, xs)
+        a = torch.empty((rows, f), dtype=x.dtype, device=dev)
+        gemm_tc.gemm_grouped(xs, w1[: 2 * E * f], a, offsets, 2 * f, 2 * f, 0, tile, err=self.gate_up.err, scale=scale,
+                             act_limit=self.limit, **act)
+        parts = torch.empty((rows, h), dtype=torch.float32, device=dev)
+        gemm_tc.gemm_grouped(a, w2[:, : E * f], parts, offsets, h, 0, f, tile, err=self.down.err)
+        shared = None
+        if self.shared_runs:
+            sf = self.shared_runs * f
+            sa = torch.empty((N, sf), dtype=x.dtype, device=dev)
+            tile = gemm_tc.grouped_tile(N, 1)
+            gemm_tc.gemm_grouped(x, w1[2 * E * f:], sa, whole, 2 * sf, 0, 0, tile, err=self.gate_up.err, scale=gate[:, E],
+                                 act_limit=self.shared["limit"], **act)
+            shared = torch.empty((N, h), dtype=torch.float32, device=dev)
+            gemm_tc.gemm_grouped(sa, w2[:, E * f:], shared, whole, h, 0, 0, tile, err=self.down.err)
+        out = torch.empty((N, h), dtype=x.dtype, device=dev)
+        core.moe_gather_sum(parts, slot_of, shared, out)
+        return out
+
+    def routed(self, x: torch.Tensor, ids: torch.Tensor, wts: torch.Tensor, gate: torch.Tensor) -> torch.Tensor:
+        """The chosen experts' weighted sum, with the expert that every token uses where it runs beside them."""
+        from ..ops import gemm_tc
+
+        if self.block == 64 and gemm_tc.grouped_suits(x, self.gate_up.weight, self.down.weight, self.expert_size,
+                                                      self.experts, self.top, self.activation):
+            return self.grouped(x, ids, wts, gate)
         act = torch.empty((x.shape[0], gate.shape[1] * self.expert_size), dtype=x.dtype, device=x.device)
         fused = False
         # the columns of an expert that every token uses may have a limit of their own
         limit_col = self.experts * self.expert_size if self.shared_runs and self.shared["limit"] != self.limit else None
         limit2 = self.shared["limit"] if limit_col is not None else 0.0
         if self.block == 64 and x.dtype == torch.bfloat16 and self.gate_up.weight.dtype == torch.bfloat16:
-            from ..ops import gemm_tc
-
             # prompts: activation and the router's weights in the product's epilogue
             fused = gemm_tc.swiglu_route(x, self.gate_up.weight, act, self.gate_up.err, activation=self.activation,
                                          scale=gate, cols_per_scale=self.expert_size, act_limit=self.limit,
@@ -221,7 +256,11 @@ class MixtureOfExperts(FeedForward):
             core.gated_act(self.gate_up(x), act, self.activation, block=self.block, scale=gate,
                            cols_per_scale=self.expert_size, limit=self.limit, alpha=self.alpha, limit_col=limit_col,
                            limit2=limit2)
-        routed = self.down(act)
+        return self.down(act)
+
+    def forward(self, x: torch.Tensor, ctx=None) -> torch.Tensor:
+        ids, wts, gate = self.route(x)
+        routed = self.routed(x, ids, wts, gate)
         if self.scoring != "softmax_all" or not (self.identity or self.shared_ffn is not None):
             return routed  # (an expert for every token that ran as columns of the products is in there)
         # the input handed on by the outputs without an expert, and the expert that every token uses

@@ -292,3 +292,43 @@ def test_random_weights_are_the_same_on_the_device_and_in_a_written_folder(tmp_p
         assert torch.equal(t.cpu(), stored[name]), name
     other = random_tensors(specs, 22, DEV, torch.bfloat16)
     assert not torch.equal(other["model.embed_tokens.weight"], drawn["model.embed_tokens.weight"])
+
+
+@pytest.mark.parametrize("scoring, experts, top, ff, shared, identity", [
+    ("softmax_top", 16, 4, 192, 0, 0), ("softmax_top", 8, 2, 64, 0, 0), ("sigmoid", 16, 2, 128, 0, 0),
+    ("softmax_all", 16, 4, 64, 128, 0), ("softmax_all", 40, 3, 128, 0, 2), ("softmax_all", 8, 4, 64, 64, 1)])
+@pytest.mark.parametrize("rows, hidden", [(65, 72), (100, 264), (300, 256), (1030, 128)])
+def test_experts_of_the_chosen_tokens_only_against_every_expert_for_every_token(scoring, experts, top, ff, shared, identity,
+                                                                                  rows, hidden):
+    """The grouped products (above 64 rows) against the one wide feed-forward that multiplies by zeros.  The activated
+    rows are the same bits but for the products' order of sums, and both add up in 32-bit and round once: two
+    roundings to bfloat16 apart."""
+    from infernum_b200.ops import gemm_tc
+    from infernum_b200.parts.base import PartSpec, build_part
+
+    rt = runtime(torch.bfloat16)
+    params = dict(hidden_size=hidden, expert_size=ff, experts=experts, top=top, scoring=scoring, identity=identity,
+                  router_bias="router.b" if scoring != "softmax_all" else None)
+    if scoring == "sigmoid":
+        params["groups"] = {"count": 4, "keep": 2}
+    if shared:
+        params["shared"] = {"size": shared, "gate": "g"}
+    part = build_part("ffn", PartSpec("moe", params), rt)
+    g = torch.Generator(device=DEV).manual_seed(rows + experts)
+    part.bind({n: (torch.randn(s.shape, generator=g, device=DEV) * (0.3 if "router" in n else 0.1)).to(torch.bfloat16)
+               for n, s in part.weight_specs().items()})
+    x = torch.randn(rows, hidden, generator=g, device=DEV).to(torch.bfloat16)
+    x[rows // 2:] = x[: rows - rows // 2].clone()  # (crowds: half of the rows go where the others go)
+    x[: rows // 4] = x[0]                          # (and one place gets a quarter of them)
+    got = part.forward(x)
+    mode = gemm_tc.POLICY["mode"]
+    gemm_tc.POLICY["mode"] = "none"
+    try:
+        ref = part.forward(x)
+    finally:
+        gemm_tc.POLICY["mode"] = mode
+    assert int(rt.error_word().item()) == 0
+    assert got.isfinite().all()
+    assert float((got.float() - ref.float()).abs().max()) < 2 ** -7 * float(ref.float().abs().max())
+    again = part.forward(x)
+    assert torch.equal(got, again)
