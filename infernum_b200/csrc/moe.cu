@@ -37,20 +37,104 @@ __global__ void router_logits_kernel(const TX* __restrict__ x, int ldx, const TW
     if (lane == 0) z[(size_t)n * E + e] = acc;
 }
 
+// Eight neighbouring values of a row in 32-bit (16-byte aligned).
+__device__ __forceinline__ void load8(const bf16* p, float (&v)[8]) {
+    const uint4 r = __ldcg(reinterpret_cast<const uint4*>(p));
+    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&r);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const float2 f = __bfloat1622float2(h[i]);
+        v[2 * i] = f.x;
+        v[2 * i + 1] = f.y;
+    }
+}
+__device__ __forceinline__ void load8(const float* p, float (&v)[8]) {
+    const float4 a = __ldcg(reinterpret_cast<const float4*>(p)), b = __ldcg(reinterpret_cast<const float4*>(p) + 1);
+    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+    v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+}
+
+// The same for rows of eights: a CTA takes four rows by eight experts, its four warps every fourth run of 256 k, a lane
+// eight neighbouring k of a run.  An expert's values are converted once for four rows, a row's once for eight experts.
+// The lanes' sums meet by halves (31 shuffles for 32 logits) and the warps' in their order: a fixed order per logit,
+// whatever the batch.  2,048 rows of 4,096, 16 experts: 64 us a warp a (row, expert) -> 8 us; eight rows 11 -> 5 us.
+template <typename TX, typename TW>
+__global__ void __launch_bounds__(128) router_logits_tile_kernel(const TX* __restrict__ x, int ldx, const TW* __restrict__ w,
+                                                                 int ldw, float* __restrict__ z, int n_rows, int E, int K) {
+    pdl_trigger();
+    pdl_wait();
+    __shared__ float sums[4][32];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int row0 = blockIdx.x * 4, e0 = blockIdx.y * 8;
+    const TX* xr[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) xr[r] = x + (size_t)min(row0 + r, n_rows - 1) * ldx;
+    float v[32];   // [row][expert]
+#pragma unroll
+    for (int i = 0; i < 32; ++i) v[i] = 0.f;
+    for (int k = warp * 256 + lane * 8; k < K; k += 1024) {
+        float a[4][8];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) load8(xr[r] + k, a[r]);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            float b[8];
+            load8(w + (size_t)min(e0 + e, E - 1) * ldw + k, b);
+#pragma unroll
+            for (int r = 0; r < 4; ++r)
+#pragma unroll
+                for (int i = 0; i < 8; ++i) v[r * 8 + e] = fmaf(a[r][i], b[i], v[r * 8 + e]);
+        }
+    }
+    int o = 1;
+#pragma unroll
+    for (int n = 16; n >= 1; n >>= 1, o <<= 1) {
+        const bool upper = lane & o;
+#pragma unroll
+        for (int i = 0; i < n; ++i) {
+            const float give = upper ? v[i] : v[i + n], keep = upper ? v[i + n] : v[i];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+        }
+    }
+    sums[warp][__brev((unsigned)lane) >> 27] = v[0];   // (the logit a lane is left with: its bits reversed)
+    __syncthreads();
+    if (warp == 0) {
+        const int row = row0 + lane / 8, e = e0 + lane % 8;
+        if (row < n_rows && e < E)
+            z[(size_t)row * E + e] = ((sums[0][lane] + sums[1][lane]) + sums[2][lane]) + sums[3][lane];
+    }
+}
+
+template <typename TX, typename TW>
+static bool rows_of_eights(const void* x, int ldx, const void* w, int ldw, int K) {
+    return K % 8 == 0 && (size_t)ldx * sizeof(TX) % 16 == 0 && (size_t)ldw * sizeof(TW) % 16 == 0 && !((uintptr_t)x & 15) &&
+           !((uintptr_t)w & 15);
+}
+
 IB_EXPORT int ib_router_logits(const void* x, int x_dtype, int ldx, const void* w, int w_dtype, int ldw, float* z,
                                int n_rows, int E, int K, void* stream) {
     if (n_rows <= 0) return IB_OK;
     if (!x || !w || !z || E <= 0 || K <= 0 || ldx < K || ldw < K) return IB_ERR_BAD_ARG;
     const long long warps = (long long)n_rows * E;
     const unsigned blocks = (unsigned)((warps + 7) / 8);
+    const dim3 tiles((n_rows + 3) / 4, (E + 7) / 8);
     cudaStream_t s = (cudaStream_t)stream;
     cudaError_t le;
-    if (x_dtype == 0 && w_dtype == 0)
+    if (x_dtype == 0 && w_dtype == 0 && rows_of_eights<float, float>(x, ldx, w, ldw, K))
+        le = launch_kernel(router_logits_tile_kernel<float, float>, tiles, dim3(128), 0, s, (const float*)x, ldx,
+                           (const float*)w, ldw, z, n_rows, E, K);
+    else if (x_dtype == 0 && w_dtype == 0)
         le = launch_kernel(router_logits_kernel<float, float>, dim3(blocks), dim3(256), 0, s, (const float*)x, ldx,
                            (const float*)w, ldw, z, n_rows, E, K);
+    else if (x_dtype == 1 && w_dtype == 1 && rows_of_eights<bf16, bf16>(x, ldx, w, ldw, K))
+        le = launch_kernel(router_logits_tile_kernel<bf16, bf16>, tiles, dim3(128), 0, s, (const bf16*)x, ldx,
+                           (const bf16*)w, ldw, z, n_rows, E, K);
     else if (x_dtype == 1 && w_dtype == 1)
         le = launch_kernel(router_logits_kernel<bf16, bf16>, dim3(blocks), dim3(256), 0, s, (const bf16*)x, ldx,
                            (const bf16*)w, ldw, z, n_rows, E, K);
+    else if (x_dtype == 1 && w_dtype == 0 && rows_of_eights<bf16, float>(x, ldx, w, ldw, K))
+        le = launch_kernel(router_logits_tile_kernel<bf16, float>, tiles, dim3(128), 0, s, (const bf16*)x, ldx,
+                           (const float*)w, ldw, z, n_rows, E, K);
     else if (x_dtype == 1 && w_dtype == 0)
         le = launch_kernel(router_logits_kernel<bf16, float>, dim3(blocks), dim3(256), 0, s, (const bf16*)x, ldx,
                            (const float*)w, ldw, z, n_rows, E, K);
@@ -398,30 +482,50 @@ moe_sort_kernel(const int* __restrict__ ids, const float* __restrict__ weights, 
     __syncwarp();
     const int groups = (n_rows + 31) / 32, per = (groups + SORT_WARPS - 1) / SORT_WARPS;
     const int g0 = warp * per, g1 = min(groups, g0 + per);
-    auto chosen = [&](int row, int k) {   // the pair's expert, E for none
-        if (row >= n_rows) return E;
+    // Up to eight choices a token are read together; more one by one.  A pair's expert (E for none) waits in slot_of
+    // until its place is known.
+    constexpr int FIRST = 8;
+    for (int g = g0; g < g1; ++g) {
+        const int row = g * 32 + lane;
         const int* r = ids + (size_t)row * top;
-        const int e = __ldcg(r + k);
-        if (e < 0 || e >= E) return E;
-        for (int j = k + 1; j < top; ++j)
-            if (__ldcg(r + j) == e) return E;
-        return e;
-    };
-    for (int g = g0; g < g1; ++g)
-        for (int k = 0; k < top; ++k) {
-            const int e = chosen(g * 32 + lane, k);
+        int first[FIRST];
+#pragma unroll
+        for (int j = 0; j < FIRST; ++j) first[j] = row < n_rows && j < top ? __ldcg(r + j) : -1;
+        auto count = [&](int k, int e, bool again) {
+            if (row >= n_rows || e < 0 || e >= E || again) e = E;
+            if (row < n_rows) slot_of[(size_t)row * top + k] = e;
             const unsigned same = __match_any_sync(0xffffffffu, e);
             if (e < E && lane == __ffs(same) - 1) mine[e] += __popc(same);
             __syncwarp();
+        };
+#pragma unroll
+        for (int k = 0; k < FIRST; ++k) {
+            if (k >= top) break;
+            bool again = false;
+#pragma unroll
+            for (int j = k + 1; j < FIRST; ++j) again |= first[j] == first[k];
+            if (row < n_rows)
+                for (int j = FIRST; j < top; ++j) again |= __ldcg(r + j) == first[k];
+            count(k, first[k], again);
         }
+        for (int k = FIRST; k < top; ++k) {
+            const int e = row < n_rows ? __ldcg(r + k) : E;
+            bool again = false;
+            if (row < n_rows)
+                for (int j = k + 1; j < top; ++j) again |= __ldcg(r + j) == e;
+            count(k, e, again);
+        }
+    }
     __syncthreads();
     if (warp == 0) {
         int before = 0;
         for (int e0 = 0; e0 < E; e0 += 32) {
             const int e = e0 + lane;
             int total = 0;
-            if (e < E)
+            if (e < E) {
+#pragma unroll
                 for (int w = 0; w < SORT_WARPS; ++w) total += place[w * E + e];
+            }
             int sum = total;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
@@ -446,9 +550,12 @@ moe_sort_kernel(const int* __restrict__ ids, const float* __restrict__ weights, 
         }
     }
     __syncthreads();
-    for (int g = g0; g < g1; ++g)
+    for (int g = g0; g < g1; ++g) {
+        const int row = g * 32 + lane;
+#pragma unroll 4
         for (int k = 0; k < top; ++k) {
-            const int row = g * 32 + lane, e = chosen(row, k);
+            const int e = row < n_rows ? slot_of[(size_t)row * top + k] : E;   // (this thread's own)
+            const float wt = row < n_rows ? __ldcg(weights + (size_t)row * top + k) : 0.f;
             const unsigned same = __match_any_sync(0xffffffffu, e);
             const int rank = __popc(same & ((1u << lane) - 1u));
             const int at = e < E ? mine[e] + rank : -1;
@@ -457,9 +564,10 @@ moe_sort_kernel(const int* __restrict__ ids, const float* __restrict__ weights, 
             __syncwarp();
             if (row < n_rows) {
                 slot_of[(size_t)row * top + k] = at;
-                if (at >= 0) slot_scale[at] = __ldcg(weights + (size_t)row * top + k);
+                if (at >= 0) slot_scale[at] = wt;
             }
         }
+    }
 }
 
 IB_EXPORT int ib_moe_sort(const int* ids, const float* weights, int n_rows, int top, int E, int* offsets, int* slot_of,

@@ -296,13 +296,14 @@ def test_random_weights_are_the_same_on_the_device_and_in_a_written_folder(tmp_p
 
 @pytest.mark.parametrize("scoring, experts, top, ff, shared, identity", [
     ("softmax_top", 16, 4, 192, 0, 0), ("softmax_top", 8, 2, 64, 0, 0), ("sigmoid", 16, 2, 128, 0, 0),
-    ("softmax_all", 16, 4, 64, 128, 0), ("softmax_all", 40, 3, 128, 0, 2), ("softmax_all", 8, 4, 64, 64, 1)])
+    ("softmax_all", 16, 4, 64, 128, 0), ("softmax_all", 40, 3, 128, 0, 2), ("softmax_all", 8, 4, 64, 64, 1),
+    ("softmax_top", 40, 12, 64, 0, 0)])
 @pytest.mark.parametrize("rows, hidden", [(65, 72), (100, 264), (300, 256), (1030, 128)])
 def test_experts_of_the_chosen_tokens_only_against_every_expert_for_every_token(scoring, experts, top, ff, shared, identity,
                                                                                   rows, hidden):
-    """The grouped products (above 64 rows) against the one wide feed-forward that multiplies by zeros.  The activated
-    rows are the same bits but for the products' order of sums, and both add up in 32-bit and round once: two
-    roundings to bfloat16 apart."""
+    """The grouped products (above 64 rows) against 64 bits: with S the sum of the sizes of what an output adds up, an
+    activated value rounds to bfloat16, eight bits, once (2^-8 of S in all), the result once (2^-8 of itself); the 32-bit sums of up
+    to some hundred terms add less than a tenth to either."""
     from infernum_b200.ops import gemm_tc
     from infernum_b200.parts.base import PartSpec, build_part
 
@@ -315,20 +316,46 @@ def test_experts_of_the_chosen_tokens_only_against_every_expert_for_every_token(
         params["shared"] = {"size": shared, "gate": "g"}
     part = build_part("ffn", PartSpec("moe", params), rt)
     g = torch.Generator(device=DEV).manual_seed(rows + experts)
-    part.bind({n: (torch.randn(s.shape, generator=g, device=DEV) * (0.3 if "router" in n else 0.1)).to(torch.bfloat16)
-               for n, s in part.weight_specs().items()})
+    w = {n: (torch.randn(s.shape, generator=g, device=DEV) * (0.3 if "router" in n else 0.1)).to(torch.bfloat16)
+         for n, s in part.weight_specs().items()}
+    part.bind(w)
     x = torch.randn(rows, hidden, generator=g, device=DEV).to(torch.bfloat16)
     x[rows // 2:] = x[: rows - rows // 2].clone()  # (crowds: half of the rows go where the others go)
     x[: rows // 4] = x[0]                          # (and one place gets a quarter of them)
+    assert gemm_tc.grouped_suits(x, part.gate_up.weight, part.down.weight, ff, experts, top, "silu")
     got = part.forward(x)
-    mode = gemm_tc.POLICY["mode"]
-    gemm_tc.POLICY["mode"] = "none"
-    try:
-        ref = part.forward(x)
-    finally:
-        gemm_tc.POLICY["mode"] = mode
     assert int(rt.error_word().item()) == 0
-    assert got.isfinite().all()
-    assert float((got.float() - ref.float()).abs().max()) < 2 ** -7 * float(ref.float().abs().max())
+    ids, wts, gate = part.route(x)
+    xd, ref, size = x.double(), torch.zeros(rows, hidden, dtype=torch.float64, device=DEV), 0
+    every = [(f"e{e}.", (wts.double() * (ids == e)).sum(1)) for e in range(experts)]
+    if shared:
+        every.append(("shared.", torch.sigmoid(xd @ w["shared.g"].double().T)[:, 0]))
+    for p, by in every:
+        a = torch.nn.functional.silu(xd @ w[p + "gate"].double().T) * (xd @ w[p + "up"].double().T) * by[:, None]
+        ref += a @ w[p + "down"].double().T
+        size = size + a.abs() @ w[p + "down"].double().abs().T
+    bound = 1.1 * 2 ** -8 * (size + ref.abs())
+    if identity:  # (the input handed on is added to the rounded sum, and the whole rounds again)
+        passed = (wts.double() * (ids >= experts)).sum(1)[:, None] * xd
+        bound = bound + 1.1 * 2 ** -8 * (ref + passed).abs()
+        ref = ref + passed
+    assert bool(((got.double() - ref).abs() <= bound + 1e-6).all())
     again = part.forward(x)
     assert torch.equal(got, again)
+
+
+@pytest.mark.parametrize("rows, experts, hidden", [(1, 1, 8), (3, 17, 264), (8, 16, 2048), (70, 9, 1032), (2049, 16, 320)])
+@pytest.mark.parametrize("dx, dw", [(torch.bfloat16,) * 2, (torch.float32,) * 2, (torch.bfloat16, torch.float32)])
+def test_router_logits_of_rows_of_eights(rows, experts, hidden, dx, dw):
+    """32-bit sums of ``hidden`` products in a fixed order: within sqrt(hidden) roundings of the sum of their sizes, and
+    a row's logits do not depend on the batch."""
+    from infernum_b200.ops import core
+
+    x, w = torch.randn(rows, hidden, device=DEV).to(dx), torch.randn(experts, hidden, device=DEV).to(dw)
+    out, one = torch.full((rows, experts), float("nan"), device=DEV), torch.empty(1, experts, device=DEV)
+    core.router_logits(x, w, out)
+    ref = x.double() @ w.double().T
+    size = x.double().abs() @ w.double().abs().T
+    assert bool(((out.double() - ref).abs() <= size * 2 ** -24 * max(4.0, hidden ** 0.5)).all())
+    core.router_logits(x[rows - 1:], w, one)
+    assert torch.equal(one[0], out[rows - 1])
