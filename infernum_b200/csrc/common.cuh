@@ -38,6 +38,9 @@
 #define IB_SITE_GROUPED_PRODUCER 12  // gemm_grouped: TMA producer
 #define IB_SITE_GROUPED_MMA 13       // gemm_grouped: MMA issuer
 #define IB_SITE_GROUPED_EPILOGUE 14  // gemm_grouped: epilogue
+#define IB_SITE_EXPANDED_PRODUCER 15 // attention_expanded: TMA producer
+#define IB_SITE_EXPANDED_MMA 16      // attention_expanded: MMA issuer
+#define IB_SITE_EXPANDED_SOFTMAX 17  // attention_expanded: softmax warps
 #define IB_TIMEOUT_AT(site) (IB_FLAG_WAIT_TIMEOUT | (1u << (8 + (site))))
 
 #define IB_EXPORT extern "C" __attribute__((visibility("default")))

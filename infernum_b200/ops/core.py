@@ -35,7 +35,9 @@ TIMEOUT_SITES = ["product for few tokens: producer", "product for few tokens: MM
                  "prompt attention: producer", "prompt attention: MMA issuer", "prompt attention: softmax",
                  "prompt attention: shared memory window misplaced", "decode attention: producer",
                  "decode attention: computing warps",
-                 "experts' product: producer", "experts' product: MMA issuer", "experts' product: epilogue"]
+                 "experts' product: producer", "experts' product: MMA issuer", "experts' product: epilogue",
+                 "attention on made keys: producer", "attention on made keys: MMA issuer",
+                 "attention on made keys: softmax"]
 
 
 def describe_flags(flags: int) -> str:

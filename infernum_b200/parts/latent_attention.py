@@ -19,8 +19,10 @@ and layer, whatever the number of heads.  The keys and values are never made:
 taken into latent space once (a product per head with ``W_uk,h^T``), attention
 runs for all heads over the one cached vector per token, whose first
 ``kv_rank`` elements are also its value, and the weighted sum of latents goes
-through ``W_uv,h`` afterwards.  A step's result therefore does not depend on
-where a prompt was cut: cached and new tokens are read the same way.
+through ``W_uv,h`` afterwards.  Steps of many rows an entry (prompts) make the
+heads' keys and values of the cached vectors they see instead, for that step, and attend
+over those (``ops/attention_expanded.py``).  A step's result does not depend on
+where a prompt was cut beyond rounding: cached and new tokens are read the same way.
 
 A layer with ``kv_shared`` has no ``W_dkv``: it is scheduled with ``cache_of``
 and reads the latents another layer cached, with its own ``W_uk``, ``W_uv``,
@@ -59,6 +61,7 @@ import torch
 from ..errors import ConfigError
 from ..ops import core
 from ..ops import attention as attn_ops
+from ..ops import attention_expanded as expanded_ops
 from .base import MIXERS, Mixer, PagedCacheSpec, Runtime, WeightSpec
 from .linear import Linear, batched_matmul_nt
 from .rope import rotary_inv_freq, rotary_magnitude
@@ -148,13 +151,28 @@ class LatentAttention(Mixer):
         # per head: W_uk,h^T [kv_rank, dim] takes a query into latent space, W_uv,h [vdim, kv_rank] a
         # weighted sum of latents to the head's output
         self.uk_t = weights[n["uk"]].view(H, self.dim, self.kv_rank).transpose(1, 2).contiguous()
-        self.uv = weights[n["uv"]].view(H, self.vdim, self.kv_rank).contiguous()
+        # prompts: every head's key and value rows as they are, for the product that makes keys and values
+        self.w_kv = None
+        uv = weights[n["uv"]]
+        if expanded_ops.supported(self.dim, self.rot_dim, self.vdim) and self.kv_rank % 8 == 0 and self.scale > 0 \
+                and {t.dtype for t in (mats[0], weights[n["uk"]], uv)} == {torch.bfloat16}:
+            self.w_kv = Linear(torch.cat([weights[n["uk"]].view(H * self.dim, self.kv_rank),
+                                          uv.view(H * self.vdim, self.kv_rank)], dim=0), self.rt)
+            uv = self.w_kv.weight[H * self.dim:]
+        self.uv = uv.view(H, self.vdim, self.kv_rank).contiguous()
 
     def weight_bytes(self) -> int:
         return self.down.nbytes + (self.uq.nbytes if self.uq is not None else 0) + self.o.nbytes \
             + (self.uk_t.numel() + self.uv.numel()) * self.uk_t.element_size()
 
     # ---- the step -----------------------------------------------------------
+    def keys_to_make(self, q: torch.Tensor, gate: Optional[torch.Tensor], pool: torch.Tensor, ctx) -> int:
+        """Cached vectors whose keys and values a step of these rows makes; 0: it runs over the latents."""
+        if self.w_kv is None or q.dtype != torch.bfloat16 or self.rt.options.get("attention", "auto") == "plain" \
+                or self.rt.options.get("latent_plan") or q.stride(0) % 8 or q.data_ptr() % 16 or pool.data_ptr() % 16:
+            return 0
+        return expanded_ops.plan(ctx, q.shape[0], self.window, 2 * self.num_heads * (self.dim + self.vdim))
+
     def forward(self, x: torch.Tensor, ctx, cache) -> torch.Tensor:
         H, W, N = self.num_heads, self.width, x.shape[0]
         writes = cache.owner and not self.kv_shared
@@ -179,6 +197,15 @@ class LatentAttention(Mixer):
                 core.latent_prepare(lat[:, hq:], 0, self.kv_rank, self.rot_dim, self.rotary_dim, None, self.kv_norm,
                                     self.eps, self.inv_freq, ctx.positions, ctx.row_entry, tables, None, pool,
                                     self.rt.err, adjacent=self.adjacent, magnitude=self.magnitude)
+        keys = self.keys_to_make(q, gate, pool, ctx)
+        if keys:
+            qr = torch.empty((N, H, self.rot_dim), dtype=x.dtype, device=x.device)
+            core.latent_q_rotate(q, H, self.dim, self.rot_dim, self.rotary_dim, self.inv_freq, ctx.positions, qr, 0,
+                                 adjacent=self.adjacent, magnitude=self.magnitude)
+            o = torch.empty((N, H * self.vdim), dtype=x.dtype, device=x.device)
+            expanded_ops.run(q, qr, pool, self.w_kv, o, self.kv_rank, self.dim, self.vdim, keys, ctx, tables, self.scale,
+                             self.window, self.rt, sink=self.sink, gate=gate)
+            return self.o(o)
         # queries in latent space and the sums of latents are kept head by head ([H, N, .]):
         # the per-head products then read and write plain matrices
         q_abs = torch.empty((H, N, W), dtype=x.dtype, device=x.device)

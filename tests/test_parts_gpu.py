@@ -359,3 +359,52 @@ def test_router_logits_of_rows_of_eights(rows, experts, hidden, dx, dw):
     assert bool(((out.double() - ref).abs() <= size * 2 ** -24 * max(4.0, hidden ** 0.5)).all())
     core.router_logits(x[rows - 1:], w, one)
     assert torch.equal(one[0], out[rows - 1])
+
+
+@pytest.mark.parametrize("heads, window, sink, gate, q_rank", [(4, 0, False, False, 64), (3, 100, True, True, 0),
+                                                               (8, 300, True, False, 64)])
+@pytest.mark.parametrize("past, new, page", [([0], [64], 16), ([0], [129], 4), ([0, 77, 300], [200, 65, 128], 16),
+                                             ([513, 0], [300, 31], 32), ([128], [256], 128)])
+def test_latent_attention_over_made_keys_against_the_plain_kernel(heads, window, sink, gate, q_rank, past, new, page):
+    """Prompts of many rows make every head's keys and values; the plain kernel attends over the latents in 32-bit.  Both
+    round a handful of intermediate rows to bfloat16, other ones: bfloat16's tolerance of these tests.  Every page
+    and slot without a token is NaN."""
+    from types import SimpleNamespace
+
+    from infernum_b200.cache import CacheManager
+    from infernum_b200.ops import attention_expanded
+    from infernum_b200.parts.base import PartSpec, build_part
+
+    hidden, outs, made = 96, [], []
+    for options in ({}, {"attention": "plain"}):
+        rt = runtime(torch.bfloat16, **options)
+        part = build_part("mixer", PartSpec("latent_attention", dict(
+            hidden_size=hidden, num_heads=heads, dim=128, rot_dim=64, vdim=128, q_rank=q_rank, kv_rank=64, scale=0.08,
+            window=window, eps=1e-5, theta=10000.0, sink="sink" if sink else None, gate="g" if gate else None)), rt)
+        gen = torch.Generator(device=DEV).manual_seed(heads + page)
+        part.bind({n: (torch.randn(s.shape, generator=gen, device=DEV) * (1.0 if "norm" in n or n == "sink" else 0.15)).to(
+            torch.bfloat16) for n, s in part.weight_specs().items()})
+        need = SimpleNamespace(position=0, paged=part.cache_spec(), state=None, cache_of=None)
+        cache = CacheManager([need], page_size=page, num_pages=sum(-(-(p + n) // page) for p, n in zip(past, new)) + 3,
+                             max_requests=len(past), dtype=torch.bfloat16, device=DEV)
+        held = []
+        for e, p in enumerate(past):
+            rc = cache.admit(e)
+            cache.extend(rc, p)
+            cache.commit(rc, p)
+            held.append(rc)
+        ctx = step_ctx(cache, list(zip(held, new)))
+        pool = cache.layer_caches[0].k_pool
+        pool.fill_(float("nan"))
+        for rc, p in zip(held, past):
+            for i, pg in enumerate(rc.tables[0]):
+                n = min(page, p - i * page)
+                if pg >= 0 and n > 0:
+                    pool[pg, 0, :n] = torch.randn(n, 128, generator=gen, device=DEV).to(torch.bfloat16)
+        x = torch.randn(sum(new), hidden, generator=gen, device=DEV).to(torch.bfloat16)
+        made.append(attention_expanded.plan(ctx, sum(new), window, 1))
+        outs.append(part.forward(x, ctx, cache.layer_caches[0]))
+        assert int(rt.error_word().item()) == 0
+    wide = sum(new) >= 64 * len(new)
+    assert (made[0] > 0) == wide
+    assert outs[0].isfinite().all() and rel_err(outs[0], outs[1]) < TOL[torch.bfloat16]
