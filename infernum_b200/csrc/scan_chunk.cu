@@ -1,0 +1,421 @@
+// Recurrent scans of prompts in chunks of 64 tokens (state rows IB_ROWS, fixed when this file is compiled), 32-bit.
+//
+// scan.cu walks a request's tokens one after another, which leaves an SM eight warps that wait for one another.  Written
+// for a chunk whose state at its begin is S0, a_t the decays, A_t their product up to token t and D[t][s] of those after s
+// up to t, a state space layer is
+//
+//   y_t = A_t S0^T C_t + sum_{s<=t} D[t][s] (C_t.B_s) dt_s x_s + d x_t,      S <- A_L S0 + sum_s D[L][s] dt_s B_s x_s^T
+//
+// - matrix products of a chunk that need no other chunk, but for S0, which a short pass over the chunks hands on:
+//
+//   ssd_chunk_state   every chunk at once: sum_s D[L][s] dt_s B_s x_s^T per head, and C_t.B_s per group
+//   ssd_chunk_pass    every state element walks its entry's chunks: S0 of each chunk, the state after the last
+//   ssd_chunk_out     every chunk at once: y
+//
+// Decays are multiplied, never divided (a decay may be 0), and a token's result is made from what comes before it only:
+// what a later token brings is left out of the sum, not multiplied by zero.  A chunk's tokens are counted from the entry's
+// first row of the step: a prompt cut elsewhere rounds otherwise.
+// Bound by the multiply-adds (as many as token by token).
+#include "common.cuh"
+
+using namespace ib;
+
+#ifndef IB_ROWS
+#error "compile with -DIB_ROWS=<rows of the state matrix>"
+#endif
+
+namespace {
+
+constexpr int ROWS = IB_ROWS;
+static_assert(ROWS == 64 || ROWS == 128, "this file is built for states of 64 and 128 rows");
+constexpr int L = 64;              // tokens of a chunk
+constexpr int PT = 64;             // columns of the state a CTA takes
+constexpr int PITCH = ROWS + 4;    // of rows read four elements at a time by neighbouring lanes
+
+struct Chunk {
+    int e, index, row, n;   // its entry, its place in it, its first row, its tokens
+};
+// Chunk `idx` of the step: the entries' chunks follow one another.  n = 0: there is none.
+__device__ __forceinline__ Chunk find_chunk(const int* cu_rows, int n_entries, int idx) {
+    for (int e = 0; e < n_entries; ++e) {
+        const int first = cu_rows[e], n = cu_rows[e + 1] - first, c = n > 0 ? (n + L - 1) / L : 0;
+        if (idx < c) return {e, idx, first + idx * L, min(L, n - idx * L)};
+        idx -= c;
+    }
+    return {0, 0, 0, 0};
+}
+
+struct SsdParams {
+    const float* x;        // [heads][rows][P]
+    const float2* bc;      // [groups][rows][ROWS]: B, C
+    const float2* dd;      // [heads][rows]: dt, decay
+    const float* d_skip;
+    const int* cu_rows;
+    const int* slot_ids;
+    float* state;          // slot s, head h: state + s * state_stride + h * P * ROWS, [P][ROWS]
+    long long state_stride;
+    float* carry;          // [heads][chunks][P][ROWS]: a chunk's own share of the state, then the state before it
+    float* decay;          // [heads][chunks]: the product of the chunk's decays
+    float* cb;             // [groups][chunks][L][L]: C_t.B_s
+    float* out;            // [rows][heads * P]
+    int n_rows, n_entries, chunks, heads, groups, P;
+};
+
+__device__ __forceinline__ float2 pfma(float a, float2 b, float2 c) {
+    const float2 aa = make_float2(a, a);
+    float2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;"
+        : "=l"(reinterpret_cast<unsigned long long&>(d))
+        : "l"(reinterpret_cast<const unsigned long long&>(aa)), "l"(reinterpret_cast<const unsigned long long&>(b)),
+          "l"(reinterpret_cast<const unsigned long long&>(c)));
+    return d;
+}
+
+// dst[t][i] = the first (which = 0) or second of the pairs of L tokens, zeros behind token n; rows `pitch` apart.
+template <int THREADS>
+__device__ __forceinline__ void load_half(float* dst, int pitch, const float2* src, int n, int which) {
+    for (int i = threadIdx.x; i < L * (ROWS / 4); i += THREADS) {
+        const int t = i / (ROWS / 4), c = i % (ROWS / 4) * 4;
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (t < n) {
+            const float4 a = __ldcg(reinterpret_cast<const float4*>(src + (size_t)t * ROWS + c));
+            const float4 b = __ldcg(reinterpret_cast<const float4*>(src + (size_t)t * ROWS + c) + 1);
+            v = which ? make_float4(a.y, a.w, b.y, b.w) : make_float4(a.x, a.z, b.x, b.z);
+        }
+        *reinterpret_cast<float4*>(dst + t * pitch + c) = v;
+    }
+}
+
+// acc[i][j] += sum_k a[i * 4 rows on][k] b[j * 8 rows on][k] over ROWS: both operands by rows of k, `pitch` apart
+__device__ __forceinline__ void dot_tile(const float* a, const float* b, int pitch, float (&acc)[4][8]) {
+#pragma unroll 2
+    for (int k = 0; k < ROWS; k += 4) {
+        float4 u[4], v[8];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) u[i] = *reinterpret_cast<const float4*>(a + i * 4 * pitch + k);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[j] = *reinterpret_cast<const float4*>(b + j * 8 * pitch + k);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                acc[i][j] = fmaf(u[i].x, v[j].x, acc[i][j]);
+                acc[i][j] = fmaf(u[i].y, v[j].y, acc[i][j]);
+                acc[i][j] = fmaf(u[i].z, v[j].z, acc[i][j]);
+                acc[i][j] = fmaf(u[i].w, v[j].w, acc[i][j]);
+            }
+    }
+}
+
+constexpr int STATE_BYTES = 2 * L * PITCH * (int)sizeof(float);   // (C and B of the C.B product; B and x need less)
+static_assert(L * ROWS + L * PT <= 2 * L * PITCH, "B and x fit where C and B do");
+
+// blockIdx.y < heads * (P / PT): a head's columns of the chunk's share of the state; behind them, a group's C.B.
+__global__ void __launch_bounds__(128) ssd_chunk_state_kernel(const SsdParams p) {
+    pdl_wait();
+    extern __shared__ __align__(16) float smem[];
+    __shared__ float w[L];
+    const Chunk at = find_chunk(p.cu_rows, p.n_entries, blockIdx.x);
+    if (at.n == 0) return;
+    const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32, ly = lane / 8, lx = lane % 8;
+    const int slices = p.P / PT;
+    const int y = blockIdx.y;
+    if (y >= p.heads * slices) {
+        const int g = y - p.heads * slices;
+        const float2* src = p.bc + ((size_t)g * p.n_rows + at.row) * ROWS;
+        float* cs = smem;
+        float* bs = smem + L * PITCH;
+        load_half<128>(bs, PITCH, src, at.n, 0);
+        load_half<128>(cs, PITCH, src, at.n, 1);
+        __syncthreads();
+        float acc[4][8] = {};
+        dot_tile(cs + (warp * 16 + ly) * PITCH, bs + lx * PITCH, PITCH, acc);
+        float* out = p.cb + ((size_t)g * p.chunks + blockIdx.x) * L * L;
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 8; ++j) out[(warp * 16 + i * 4 + ly) * L + lx + j * 8] = acc[i][j];
+        return;
+    }
+    const int head = y / slices, p0 = y % slices * PT;
+    const int grp = head / (p.heads / p.groups);
+    const float2* dd = p.dd + (size_t)head * p.n_rows + at.row;
+    if (warp == 0) {   // w_s = dt_s times the decays after s: products from the chunk's end on, two tokens a lane
+        const float2 d0 = 2 * lane < at.n ? __ldcg(dd + 2 * lane) : make_float2(0.f, 1.f);
+        const float2 d1 = 2 * lane + 1 < at.n ? __ldcg(dd + 2 * lane + 1) : make_float2(0.f, 1.f);
+        float after = d0.y * d1.y;   // of this lane's tokens, then of all from this lane on
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const float v = __shfl_down_sync(0xffffffffu, after, o);
+            if (lane + o < 32) after *= v;
+        }
+        float rest = __shfl_down_sync(0xffffffffu, after, 1);
+        if (lane == 31) rest = 1.f;
+        w[2 * lane + 1] = d1.x * rest;
+        w[2 * lane] = d0.x * (d1.y * rest);
+        if (lane == 0 && p0 == 0) p.decay[(size_t)head * p.chunks + blockIdx.x] = after;
+    }
+    float* bs = smem;                // [L][ROWS]
+    float* xs = smem + L * ROWS;     // [L][PT]
+    load_half<128>(bs, ROWS, p.bc + ((size_t)grp * p.n_rows + at.row) * ROWS, at.n, 0);
+    __syncthreads();
+    const float* x = p.x + ((size_t)head * p.n_rows + at.row) * p.P + p0;
+    for (int i = tid; i < L * (PT / 4); i += 128) {
+        const int t = i / (PT / 4), c = i % (PT / 4) * 4;
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (t < at.n) {
+            v = __ldcg(reinterpret_cast<const float4*>(x + (size_t)t * p.P + c));
+            v.x *= w[t]; v.y *= w[t]; v.z *= w[t]; v.w *= w[t];
+        }
+        *reinterpret_cast<float4*>(xs + t * PT + c) = v;
+    }
+    __syncthreads();
+    // a thread: rows warp * 16 + ly * 4 .. + 3 (and, of 128, those 64 further on), columns lx * 4 .. + 3 and 32 further on
+    constexpr int RB = ROWS / 64;
+    float2 acc[RB][4][4] = {};
+#pragma unroll 4
+    for (int s = 0; s < L; ++s) {
+        float4 b[RB];
+#pragma unroll
+        for (int r = 0; r < RB; ++r) b[r] = *reinterpret_cast<const float4*>(bs + s * ROWS + r * 64 + warp * 16 + ly * 4);
+        const float4 v0 = *reinterpret_cast<const float4*>(xs + s * PT + lx * 4);
+        const float4 v1 = *reinterpret_cast<const float4*>(xs + s * PT + 32 + lx * 4);
+        const float2 v[4] = {make_float2(v0.x, v0.y), make_float2(v0.z, v0.w), make_float2(v1.x, v1.y), make_float2(v1.z, v1.w)};
+#pragma unroll
+        for (int r = 0; r < RB; ++r)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                acc[r][0][j] = pfma(b[r].x, v[j], acc[r][0][j]);
+                acc[r][1][j] = pfma(b[r].y, v[j], acc[r][1][j]);
+                acc[r][2][j] = pfma(b[r].z, v[j], acc[r][2][j]);
+                acc[r][3][j] = pfma(b[r].w, v[j], acc[r][3][j]);
+            }
+    }
+    float* out = p.carry + (((size_t)head * p.chunks + blockIdx.x) * p.P + p0) * ROWS;
+#pragma unroll
+    for (int r = 0; r < RB; ++r)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int col = (j / 2) * 32 + lx * 4 + (j % 2) * 2;
+            float* o = out + (size_t)col * ROWS + r * 64 + warp * 16 + ly * 4;
+            *reinterpret_cast<float4*>(o) = make_float4(acc[r][0][j].x, acc[r][1][j].x, acc[r][2][j].x, acc[r][3][j].x);
+            *reinterpret_cast<float4*>(o + ROWS) = make_float4(acc[r][0][j].y, acc[r][1][j].y, acc[r][2][j].y, acc[r][3][j].y);
+        }
+}
+
+// Four state elements a thread: the state before each of the entry's chunks takes the place of the chunk's own share.
+__global__ void __launch_bounds__(128) ssd_chunk_pass_kernel(const SsdParams p) {
+    pdl_trigger();
+    pdl_wait();
+    const int head = blockIdx.y, e = blockIdx.z;
+    const int i = (blockIdx.x * 128 + threadIdx.x) * 4;
+    const int n = p.cu_rows[e + 1] - p.cu_rows[e];
+    if (n <= 0 || i >= p.P * ROWS) return;
+    int first = 0;   // the entry's first chunk
+    for (int q = 0; q < e; ++q) {
+        const int m = p.cu_rows[q + 1] - p.cu_rows[q];
+        if (m > 0) first += (m + L - 1) / L;
+    }
+    const int count = (n + L - 1) / L;
+    float4* st = reinterpret_cast<float4*>(p.state + (long long)p.slot_ids[e] * p.state_stride + (size_t)head * p.P * ROWS + i);
+    float* c = p.carry + ((size_t)head * p.chunks + first) * p.P * ROWS + i;
+    const float* d = p.decay + (size_t)head * p.chunks + first;
+    const size_t step = (size_t)p.P * ROWS;
+    float4 S = __ldcg(st);
+    constexpr int AHEAD = 8;
+    for (int k0 = 0; k0 < count; k0 += AHEAD) {
+        float4 u[AHEAD];
+        float a[AHEAD];
+#pragma unroll
+        for (int k = 0; k < AHEAD; ++k)
+            if (k0 + k < count) {
+                u[k] = __ldcg(reinterpret_cast<const float4*>(c + (k0 + k) * step));
+                a[k] = __ldcg(d + k0 + k);
+            }
+#pragma unroll
+        for (int k = 0; k < AHEAD; ++k)
+            if (k0 + k < count) {
+                __stcg(reinterpret_cast<float4*>(c + (k0 + k) * step), S);
+                S.x = fmaf(a[k], S.x, u[k].x);
+                S.y = fmaf(a[k], S.y, u[k].y);
+                S.z = fmaf(a[k], S.z, u[k].z);
+                S.w = fmaf(a[k], S.w, u[k].w);
+            }
+    }
+    *st = S;
+}
+
+constexpr int MP = L + 4;   // pitch of the chunk's own weights
+constexpr int OUT_BYTES = (2 * L * PITCH + L * PT + L * MP) * (int)sizeof(float);
+
+__global__ void __launch_bounds__(128) ssd_chunk_out_kernel(const SsdParams p) {
+    pdl_trigger();
+    pdl_wait();
+    extern __shared__ __align__(16) float smem[];
+    float* cs = smem;                  // [L][PITCH] C
+    float* ss = cs + L * PITCH;        // [PT][PITCH] the state before the chunk, column c at row c % 4 * 8 + c / 4 % 8 + c / 32 * 32
+    float* xs = ss + PT * PITCH;       // [L][PT]
+    float* ms = xs + L * PT;           // [L][MP] D[t][s] (C_t.B_s) dt_s
+    __shared__ float dt[L], da[L], upto[L];
+    const Chunk at = find_chunk(p.cu_rows, p.n_entries, blockIdx.x);
+    if (at.n == 0) return;
+    const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32, ly = lane / 8, lx = lane % 8;
+    const int head = blockIdx.y, p0 = blockIdx.z * PT;
+    const int grp = head / (p.heads / p.groups);
+    if (tid < L) {
+        const float2 d = tid < at.n ? __ldcg(p.dd + (size_t)head * p.n_rows + at.row + tid) : make_float2(0.f, 1.f);
+        dt[tid] = d.x;
+        da[tid] = d.y;
+    }
+    load_half<128>(cs, PITCH, p.bc + ((size_t)grp * p.n_rows + at.row) * ROWS, at.n, 1);
+    const float* st = p.carry + (((size_t)head * p.chunks + blockIdx.x) * p.P + p0) * ROWS;
+    for (int i = tid; i < PT * (ROWS / 4); i += 128) {
+        const int c = i / (ROWS / 4), r = i % (ROWS / 4) * 4;
+        *reinterpret_cast<float4*>(ss + (c % 4 * 8 + c / 4 % 8 + c / 32 * 32) * PITCH + r) =
+            __ldcg(reinterpret_cast<const float4*>(st + (size_t)c * ROWS + r));
+    }
+    const float* x = p.x + ((size_t)head * p.n_rows + at.row) * p.P + p0;
+    for (int i = tid; i < L * (PT / 4); i += 128) {
+        const int t = i / (PT / 4), c = i % (PT / 4) * 4;
+        *reinterpret_cast<float4*>(xs + t * PT + c) =
+            t < at.n ? __ldcg(reinterpret_cast<const float4*>(x + (size_t)t * p.P + c)) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    __syncthreads();
+    {   // a thread walks half of a column s of the weights downwards
+        const int s = tid % L, half = tid / L;
+        const float* cb = p.cb + ((size_t)grp * p.chunks + blockIdx.x) * L * L + s;
+        const int t1 = half ? L : L / 2, t0 = max(s, half ? L / 2 : 0);
+        const float ds = dt[s];
+        float d = 1.f;   // D[t][s]
+        for (int t = s + 1; t <= t0 && t < L; ++t) d *= da[t];
+#pragma unroll 4
+        for (int t = t0; t < t1; ++t) {
+            ms[t * MP + s] = d * __ldcg(cb + t * L) * ds;
+            d *= t + 1 < L ? da[t + 1] : 1.f;
+        }
+        if (warp == 0) {   // A_t: two tokens a lane
+            const float d0 = da[2 * lane], d1 = da[2 * lane + 1];
+            float before = d0 * d1;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const float v = __shfl_up_sync(0xffffffffu, before, o);
+                if (lane >= o) before *= v;
+            }
+            float prior = __shfl_up_sync(0xffffffffu, before, 1);
+            if (lane == 0) prior = 1.f;
+            upto[2 * lane] = prior * d0;
+            upto[2 * lane + 1] = prior * d0 * d1;
+        }
+    }
+    __syncthreads();
+    // a thread: tokens warp * 16 + i * 4 + ly, columns (j / 4) * 32 + lx * 4 + j % 4 (row j * 8 + lx of `ss`)
+    float acc[4][8] = {};
+    dot_tile(cs + (warp * 16 + ly) * PITCH, ss + lx * PITCH, PITCH, acc);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const float a = upto[warp * 16 + i * 4 + ly];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) acc[i][j] *= a;
+    }
+    const float* mw = ms + (warp * 16 + ly) * MP;
+    const float* xw = xs + lx * 4;
+#pragma unroll 2
+    for (int s = 0; s < warp * 16; s += 4) {
+        float4 m[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) m[i] = *reinterpret_cast<const float4*>(mw + i * 4 * MP + s);
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                const float4 v = *reinterpret_cast<const float4*>(xw + (s + u) * PT + c * 32);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const float q = u == 0 ? m[i].x : u == 1 ? m[i].y : u == 2 ? m[i].z : m[i].w;
+                    acc[i][4 * c] = fmaf(q, v.x, acc[i][4 * c]);
+                    acc[i][4 * c + 1] = fmaf(q, v.y, acc[i][4 * c + 1]);
+                    acc[i][4 * c + 2] = fmaf(q, v.z, acc[i][4 * c + 2]);
+                    acc[i][4 * c + 3] = fmaf(q, v.w, acc[i][4 * c + 3]);
+                }
+            }
+    }
+#pragma unroll 2
+    for (int s = warp * 16; s < warp * 16 + 16; ++s) {   // the warp's own tokens: each takes those up to itself
+        float4 v[2];
+#pragma unroll
+        for (int c = 0; c < 2; ++c) v[c] = *reinterpret_cast<const float4*>(xw + s * PT + c * 32);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            if (s > warp * 16 + i * 4 + ly) continue;
+            const float q = mw[i * 4 * MP + s];
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                acc[i][4 * c] = fmaf(q, v[c].x, acc[i][4 * c]);
+                acc[i][4 * c + 1] = fmaf(q, v[c].y, acc[i][4 * c + 1]);
+                acc[i][4 * c + 2] = fmaf(q, v[c].z, acc[i][4 * c + 2]);
+                acc[i][4 * c + 3] = fmaf(q, v[c].w, acc[i][4 * c + 3]);
+            }
+        }
+    }
+    const float skip = p.d_skip[head];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int t = warp * 16 + i * 4 + ly;
+        if (t >= at.n) continue;
+        float* o = p.out + (size_t)(at.row + t) * p.heads * p.P + (size_t)head * p.P + p0 + lx * 4;
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+            const float4 v = *reinterpret_cast<const float4*>(xw + t * PT + c * 32);
+            *reinterpret_cast<float4*>(o + c * 32) =
+                make_float4(fmaf(skip, v.x, acc[i][4 * c]), fmaf(skip, v.y, acc[i][4 * c + 1]),
+                            fmaf(skip, v.z, acc[i][4 * c + 2]), fmaf(skip, v.w, acc[i][4 * c + 3]));
+        }
+    }
+}
+
+}  // namespace
+
+IB_EXPORT int ib_scan_chunk_rows() { return ROWS; }
+
+// Floats of scratch a step of n_rows rows in n_entries entries takes.
+IB_EXPORT long long ib_ssd_chunk_scratch(int n_rows, int n_entries, int heads, int groups, int P) {
+    const long long chunks = n_rows / L + n_entries;
+    return chunks * ((long long)heads * P * ROWS + (long long)groups * L * L + heads + 4);
+}
+
+// As ib_ssd_scan (scan.cu); P a multiple of 64, x, bc, state, scratch and out 16-byte aligned, state_stride a multiple of 4.
+IB_EXPORT int ib_ssd_chunk(const float* x, const void* bc, const void* dd, int n_rows, const float* d_skip, float* state,
+                           long long state_stride, const int* cu_rows, const int* slot_ids, float* out, int n_entries,
+                           int heads, int groups, int P, float* scratch, void* stream) {
+    if (n_entries <= 0 || n_rows <= 0) return IB_OK;
+    if (!x || !bc || !dd || !d_skip || !state || !cu_rows || !slot_ids || !out || !scratch || heads <= 0 || groups <= 0 ||
+        heads % groups || P <= 0)
+        return IB_ERR_BAD_ARG;
+    if (P % PT || state_stride % 4 || ((uintptr_t)dd & 7) ||
+        (((uintptr_t)x | (uintptr_t)bc | (uintptr_t)state | (uintptr_t)scratch | (uintptr_t)out) & 15))
+        return IB_ERR_UNSUPPORTED;
+    const int chunks = n_rows / L + n_entries;
+    if ((long long)heads * (P / PT) + groups > 65535 || n_entries > 65535) return IB_ERR_TOO_LARGE;
+    SsdParams p{x, (const float2*)bc, (const float2*)dd, d_skip, cu_rows, slot_ids, state, state_stride, scratch, nullptr,
+                nullptr, out, n_rows, n_entries, chunks, heads, groups, P};
+    p.cb = scratch + (size_t)chunks * heads * P * ROWS;
+    p.decay = p.cb + (size_t)chunks * groups * L * L;
+    static bool attr_done = false;
+    if (!attr_done) {
+        cudaError_t e = cudaFuncSetAttribute(ssd_chunk_state_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, STATE_BYTES);
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(ssd_chunk_out_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, OUT_BYTES);
+        if (e != cudaSuccess) return (int)e;
+        attr_done = true;
+    }
+    cudaStream_t s = (cudaStream_t)stream;
+    cudaError_t le = launch_kernel_in_order(ssd_chunk_state_kernel, dim3(chunks, heads * (P / PT) + groups), dim3(128),
+                                            (size_t)STATE_BYTES, s, p);
+    if (le == cudaSuccess)
+        le = launch_kernel(ssd_chunk_pass_kernel, dim3((P * ROWS / 4 + 127) / 128, heads, n_entries), dim3(128), 0, s, p);
+    if (le == cudaSuccess)
+        le = launch_kernel(ssd_chunk_out_kernel, dim3(chunks, heads, P / PT), dim3(128), (size_t)OUT_BYTES, s, p);
+    if (le != cudaSuccess) return (int)le;
+    IB_LAUNCH_CHECK();
+    return IB_OK;
+}

@@ -45,6 +45,37 @@ def lib_for(rows: int) -> ctypes.CDLL:
     return lib
 
 
+_chunk_libs: Dict[int, ctypes.CDLL] = {}
+CHUNK_ROWS = (64, 128)
+CHUNK_MIN_ROWS, CHUNK_MIN_MEAN = 96, 32
+
+
+def chunk_lib_for(rows: int) -> ctypes.CDLL:
+    """The scans of prompts in chunks (``scan_chunk.cu``)."""
+    lib = _chunk_libs.get(rows)
+    if lib is None:
+        lib = load_module(f"scan_chunk_r{rows}", ["scan_chunk.cu"], [f"-DIB_ROWS={rows}"])
+        lib.ib_ssd_chunk_scratch.argtypes = [_c_int, _c_int, _c_int, _c_int, _c_int]
+        lib.ib_ssd_chunk_scratch.restype = _c_ll
+        lib.ib_ssd_chunk.argtypes = [_c_void_p, _c_void_p, _c_void_p, _c_int, _c_void_p, _c_void_p, _c_ll, _c_void_p,
+                                     _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_void_p, _c_void_p]
+        for fn in (lib.ib_ssd_chunk, lib.ib_scan_chunk_rows):
+            fn.restype = _c_int
+        if lib.ib_scan_chunk_rows() != rows:
+            raise KernelError(f"scan module for {rows} state rows was built for another number")
+        _chunk_libs[rows] = lib
+    return lib
+
+
+def in_chunks(ctx, n_rows: int, rows: int, cols: int, state_ptr: int, state_stride: int) -> bool:
+    """Whether a step's scan runs in chunks of 64 tokens: where a request brings a prompt (below some hundred tokens the
+    walk token by token is over before three launches are), and not for its sake alone beside many decoded tokens, each
+    of which would be a chunk."""
+    most = getattr(ctx, "max_rows_per_entry", n_rows)
+    return (rows in CHUNK_ROWS and cols % 64 == 0 and state_ptr % 16 == 0 and state_stride % 4 == 0
+            and most >= CHUNK_MIN_ROWS and n_rows >= CHUNK_MIN_MEAN * ctx.n_entries)
+
+
 def choose_col_slices(n_entries: int, heads: int, cols: int, split: int, sm_count: int) -> int:
     """Into how many CTAs the columns of a head's state are cut.  The warps of a
     scan are as many as its columns times the lanes of a column, whatever the
@@ -200,6 +231,14 @@ def ssd_scan(xbc: torch.Tensor, dt: torch.Tensor, dt_bias: torch.Tensor, a_log: 
         taps,
         core.stream_ptr(xbc)), "ssd_prepare")
     ptr, stride = _state_ptr(state, state_offset)
+    if in_chunks(ctx, N, state_rows, vdim, ptr, stride) and out.data_ptr() % 16 == 0:
+        clib = chunk_lib_for(state_rows)
+        scratch = torch.empty(clib.ib_ssd_chunk_scratch(N, ctx.n_entries, heads, groups, vdim), dtype=torch.float32,
+                              device=xbc.device)
+        core.check(clib.ib_ssd_chunk(x32.data_ptr(), bc.data_ptr(), dd.data_ptr(), N, d_skip.data_ptr(), ptr, stride,
+                                     ctx.cu_rows.data_ptr(), ctx.slot_ids.data_ptr(), out.data_ptr(), ctx.n_entries, heads,
+                                     groups, vdim, scratch.data_ptr(), core.stream_ptr(xbc)), "ssd_chunk")
+        return
     sm = rt.options.get("sm_count") or SM_COUNT_FALLBACK
     slices = choose_col_slices(ctx.n_entries, heads, vdim, lib.ib_scan_split(), sm)
     core.check(lib.ib_ssd_scan(x32.data_ptr(), bc.data_ptr(), dd.data_ptr(), N, d_skip.data_ptr(), ptr, stride,

@@ -408,3 +408,52 @@ def test_latent_attention_over_made_keys_against_the_plain_kernel(heads, window,
     wide = sum(new) >= 64 * len(new)
     assert (made[0] > 0) == wide
     assert outs[0].isfinite().all() and rel_err(outs[0], outs[1]) < TOL[torch.bfloat16]
+
+
+@pytest.mark.parametrize("rule, heads, groups, rows, cols", [("ssd", 4, 2, 128, 64), ("ssd", 3, 1, 64, 128)])
+@pytest.mark.parametrize("lens", [[96], [128, 1, 63], [131, 64, 200], [0, 300], [65, 100, 193, 40]])
+def test_scans_in_chunks_against_one_token_at_a_time(rule, heads, groups, rows, cols, lens):
+    """The kernels for prompts against the token-by-token one, which a state whose rows are an odd number of floats apart
+    asks for: the same 32-bit sums in another order, over states of some hundred decaying tokens.  A token's result does
+    not see what comes after it, not even a NaN."""
+    from types import SimpleNamespace
+
+    from infernum_b200.ops import scan
+
+    rt, N, E = runtime(torch.float32), sum(lens), len(lens)
+    g = torch.Generator(device=DEV).manual_seed(N + rows)
+    rnd = lambda *s: torch.randn(*s, generator=g, device=DEV)  # noqa: E731
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)  # noqa: E731
+    cu = [sum(lens[:i]) for i in range(E + 1)]
+    ctx = SimpleNamespace(n_entries=E, n_rows=N, max_rows_per_entry=max(lens), cu_rows=i32(cu), slot_ids=i32(list(range(E))),
+                          row_entry=i32([e for e, n in enumerate(lens) for _ in range(n)]))
+    size, inner = heads * rows * cols, heads * cols
+    start = rnd(E, size)
+    width = 2 * groups * rows + inner + 2 * heads
+    x, a_log, dt_bias, skip = rnd(N, width), rnd(heads) * 0.5, rnd(heads) - 1.0, rnd(heads)
+
+    def walk(x, stride):
+        state = torch.full((E + 1, stride), 7.0, device=DEV)
+        state[:E, :size] = start
+        out = torch.empty(N, inner, device=DEV)
+        if rule == "ssd":
+            scan.ssd_scan(x[:, : inner + 2 * groups * rows], x[:, width - heads:], dt_bias, a_log, skip, state, 0, ctx, out,
+                          heads, groups, rows, cols, rt)
+        else:
+            scan.delta_scan(x, 0, width - 2 * heads, width - heads, None, a_log, dt_bias, state, 0, size, ctx, out, heads,
+                            groups, rows, cols, rt)
+        return out, state
+
+    assert scan.in_chunks(ctx, N, rows, cols, 0, size + 8) and not scan.in_chunks(ctx, N, rows, cols, 0, size + 9)
+    out, state = walk(x, size + 8)
+    ref, ref_state = walk(x, size + 9)
+    assert rel_err(out, ref) < 1e-5 and rel_err(state[:E, :size], ref_state[:E, :size]) < 1e-5
+    assert bool((state[:, size:] == 7.0).all()) and bool((state[E] == 7.0).all())
+    last = next(e for e in range(E) if lens[e] >= 96)
+    at = cu[last] + lens[last] - 2  # the token before the entry's last
+    bad = x.clone()
+    bad[at] = float("nan")
+    got, _ = walk(bad, size + 8)
+    keep = torch.ones(N, dtype=torch.bool, device=DEV)
+    keep[at: at + 2] = False
+    assert torch.equal(got[keep], out[keep]) and bool(got[at].isnan().all())
