@@ -26,6 +26,25 @@ using namespace ib;
 
 __device__ __forceinline__ float silu_f(float g) { return g / (1.f + expf(-g)); }
 
+// Four neighbouring values, past the L1 (a kernel begun under its predecessor's tail may meet an older line there).
+__device__ __forceinline__ float4 load4(const float* p) { return __ldcg(reinterpret_cast<const float4*>(p)); }
+__device__ __forceinline__ float4 load4(const bf16* p) {
+    const uint2 r = __ldcg(reinterpret_cast<const uint2*>(p));
+    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&r);
+    const float2 a = __bfloat1622float2(h[0]), b = __bfloat1622float2(h[1]);
+    return make_float4(a.x, a.y, b.x, b.y);
+}
+__device__ __forceinline__ void store4(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
+__device__ __forceinline__ void store4(bf16* p, float4 v) {
+    __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
+    uint2 r;
+    r.x = *reinterpret_cast<unsigned*>(&lo);
+    r.y = *reinterpret_cast<unsigned*>(&hi);
+    *reinterpret_cast<uint2*>(p) = r;
+}
+template <typename T>
+static bool fours(const T* p, int stride) { return stride % 4 == 0 && (uintptr_t)p % (4 * sizeof(T)) == 0; }
+
 // ---------------------------------------------------------------------------
 template <typename T>
 __global__ void token_shift_kernel(const T* __restrict__ x, const float* __restrict__ mu, float* __restrict__ state,
@@ -198,6 +217,129 @@ IB_EXPORT int ib_ssd_prepare(const void* x, int x_stride, int act_dtype, const f
     } else {
         return IB_ERR_UNSUPPORTED;
     }
+    if (le != cudaSuccess) return (int)le;
+    IB_LAUNCH_CHECK();
+    return IB_OK;
+}
+
+// The same for prompts, whose scan goes in chunks (scan_chunk.cu): B and C of a token one after the other, bc [groups]
+// [rows][2][state].  A thread has four channels and walks ROWS rows of them with the last inputs in registers, so an
+// input is read once instead of once a tap: 2,048 rows of 2,304 channels 48 us -> 29 us.
+constexpr int SSD_ROWS = 16, SSD_TAPS = 4;
+template <typename T>
+__global__ void __launch_bounds__(128)
+ssd_prepare_rows_kernel(const T* __restrict__ x, int x_stride, const float* __restrict__ w, const float* __restrict__ b,
+                        const float* __restrict__ state, long long state_stride, const int* __restrict__ row_entry,
+                        const int* __restrict__ cu_rows, const int* __restrict__ slot_ids, const T* __restrict__ dt_raw,
+                        int dt_stride, const float* __restrict__ dt_bias, const float* __restrict__ a_log,
+                        float* __restrict__ xo, float* __restrict__ bc, float2* __restrict__ dd, int inner, int gn, int heads,
+                        int n_rows, int P, int state_rows) {
+    pdl_trigger();
+    pdl_wait();
+    const int r0 = blockIdx.x * SSD_ROWS, r1 = min(n_rows, r0 + SSD_ROWS);
+    const int C = inner + 2 * gn;
+    if (blockIdx.y == gridDim.y - 1) {   // the gates of the heads
+        for (int i = threadIdx.x; i < heads * (r1 - r0); i += blockDim.x) {
+            const int h = i % heads, row = r0 + i / heads;
+            const float raw = to_f32(dt_raw[(size_t)row * dt_stride + h]) + dt_bias[h];
+            const float dt = raw > 20.f ? raw : log1pf(expf(raw));
+            dd[(size_t)h * n_rows + row] = make_float2(dt, expf(-expf(a_log[h]) * dt));
+        }
+        return;
+    }
+    const int c = (blockIdx.y * 128 + threadIdx.x) * 4;
+    if (c >= C) return;
+    float4 in[SSD_ROWS];
+#pragma unroll
+    for (int i = 0; i < SSD_ROWS; ++i)
+        if (r0 + i < r1) in[i] = load4(x + (size_t)(r0 + i) * x_stride + c);
+    float wt[4][SSD_TAPS];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const float4 v = *reinterpret_cast<const float4*>(w + (size_t)(c + q) * SSD_TAPS);
+        wt[q][0] = v.x; wt[q][1] = v.y; wt[q][2] = v.z; wt[q][3] = v.w;
+    }
+    const float4 bias = b ? *reinterpret_cast<const float4*>(b + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 past[SSD_TAPS - 1];
+#pragma unroll
+    for (int i = 0; i < SSD_ROWS; ++i) {
+        const int row = r0 + i;
+        if (row >= r1) break;
+        const int e = row_entry[row], first = cu_rows[e];
+        if (i == 0 || row == first) {   // (the inputs before an entry's first row are in its state)
+            const float* st = state + (long long)slot_ids[e] * state_stride;
+#pragma unroll
+            for (int j = 0; j < SSD_TAPS - 1; ++j) {
+                const int src = row - (SSD_TAPS - 1) + j;
+                past[j] = src >= first ? load4(x + (size_t)src * x_stride + c)
+                                       : load4(st + (size_t)(SSD_TAPS - 1 - (first - src)) * C + c);
+            }
+        }
+        float4 v = bias;
+#pragma unroll
+        for (int j = 0; j < SSD_TAPS; ++j) {
+            const float4 a = j < SSD_TAPS - 1 ? past[j < SSD_TAPS - 1 ? j : 0] : in[i];
+            v.x = fmaf(wt[0][j], a.x, v.x);
+            v.y = fmaf(wt[1][j], a.y, v.y);
+            v.z = fmaf(wt[2][j], a.z, v.z);
+            v.w = fmaf(wt[3][j], a.w, v.w);
+        }
+#pragma unroll
+        for (int j = 0; j + 1 < SSD_TAPS - 1; ++j) past[j] = past[j + 1];
+        past[SSD_TAPS - 2] = in[i];
+        v = make_float4(silu_f(v.x), silu_f(v.y), silu_f(v.z), silu_f(v.w));
+        float* dst;
+        if (c < inner) {
+            dst = xo + ((size_t)(c / P) * n_rows + row) * P + c % P;
+        } else {
+            const int k = c < inner + gn ? c - inner : c - inner - gn;
+            dst = bc + (((size_t)(k / state_rows) * n_rows + row) * 2 + (c < inner + gn ? 0 : 1)) * state_rows + k % state_rows;
+        }
+        store4(dst, v);
+    }
+}
+
+// 1 where ib_ssd_prepare_rows takes these operands.
+template <typename T>
+static bool ssd_rows_suit(const T* x, int x_stride, const float* w, const float* b, const float* state,
+                          long long state_stride, int inner, int gn, int heads, int state_rows, int taps) {
+    return w && taps == SSD_TAPS && fours(x, x_stride) && inner % 4 == 0 && gn % 4 == 0 && state_rows % 4 == 0 &&
+           inner / heads % 4 == 0 && ((uintptr_t)w & 15) == 0 && ((uintptr_t)b & 15) == 0 && ((uintptr_t)state & 15) == 0 &&
+           state_stride % 4 == 0;
+}
+
+IB_EXPORT int ib_ssd_prepare_rows(const void* x, int x_stride, int act_dtype, const float* w, const float* b,
+                                  float* state, long long state_stride, const int* row_entry, const int* cu_rows,
+                                  const int* slot_ids, const void* dt_raw, int dt_stride, const float* dt_bias,
+                                  const float* a_log, float* xo, void* bc, void* dd, int n_rows, int n_entries,
+                                  int inner, int gn, int heads, int state_rows, int taps, void* stream) {
+    if (n_rows <= 0) return IB_OK;
+    if (!x || !dt_raw || !dt_bias || !a_log || !xo || !bc || !dd || inner <= 0 || gn <= 0 || heads <= 0 || inner % heads ||
+        state_rows <= 0 || gn % state_rows || !w || !state || !row_entry || !cu_rows || !slot_ids || n_entries <= 0)
+        return IB_ERR_BAD_ARG;
+    const int C = inner + 2 * gn;
+    const dim3 grid((n_rows + SSD_ROWS - 1) / SSD_ROWS, (C / 4 + 127) / 128 + 1);
+    const int gy = min(64, (C + 127) / 128);
+    cudaStream_t s = (cudaStream_t)stream;
+    cudaError_t le;
+#define IB_PREP(T)                                                                                                        \
+    if (!ssd_rows_suit<T>((const T*)x, x_stride, w, b, state, state_stride, inner, gn, heads, state_rows, taps) ||        \
+        (((uintptr_t)xo | (uintptr_t)bc) & 15))                                                                           \
+        return IB_ERR_UNSUPPORTED;                                                                                        \
+    le = launch_kernel(ssd_prepare_rows_kernel<T>, grid, dim3(128), 0, s, (const T*)x, x_stride, w, b, (const float*)state, \
+                       state_stride, row_entry, cu_rows, slot_ids, (const T*)dt_raw, dt_stride, dt_bias, a_log, xo,       \
+                       (float*)bc, (float2*)dd, inner, gn, heads, n_rows, inner / heads, state_rows);                     \
+    if (le == cudaSuccess)                                                                                                \
+        le = launch_kernel(conv_state_kernel<T>, dim3(n_entries, gy), dim3(128), 0, s, (const T*)x, x_stride, state,      \
+                           state_stride, cu_rows, slot_ids, C, taps)
+    if (act_dtype == 0) {
+        IB_PREP(float);
+    } else if (act_dtype == 1) {
+        IB_PREP(bf16);
+    } else {
+        return IB_ERR_UNSUPPORTED;
+    }
+#undef IB_PREP
     if (le != cudaSuccess) return (int)le;
     IB_LAUNCH_CHECK();
     return IB_OK;
@@ -380,6 +522,43 @@ __global__ void head_norm_gate_kernel(const float* __restrict__ o, const T* __re
     }
 }
 
+// The same for heads of K = 4 LANES values, LANES neighbouring lanes a head, four values a lane, read once.
+template <typename T, int LANES>
+__global__ void head_norm_gate_vec4_kernel(const float* __restrict__ o, const T* __restrict__ g, int g_stride,
+                                           const float* __restrict__ w, T* __restrict__ out, int n_rows, int heads, float eps) {
+    pdl_trigger();
+    pdl_wait();
+    constexpr int K = 4 * LANES;
+    const long long item = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / LANES;
+    const bool live = item < (long long)n_rows * heads;
+    const long long at = live ? item : 0;
+    const int row = (int)(at / heads), head = (int)(at % heads), i = threadIdx.x % LANES * 4;
+    float4 v = load4(o + (size_t)at * K + i);
+    float ss = v.x * v.x + v.y * v.y + (v.z * v.z + v.w * v.w);
+#pragma unroll
+    for (int q = LANES / 2; q > 0; q >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, q);
+    if (!live) return;
+    const float inv = 1.f / sqrtf(ss / (float)K + eps);
+    const float4 ww = *reinterpret_cast<const float4*>(w + (size_t)head * K + i);
+    v = make_float4(v.x * inv * ww.x, v.y * inv * ww.y, v.z * inv * ww.z, v.w * inv * ww.w);
+    if (g) {
+        const float4 gg = load4(g + (size_t)row * g_stride + (size_t)head * K + i);
+        v = make_float4(v.x * silu_f(gg.x), v.y * silu_f(gg.y), v.z * silu_f(gg.z), v.w * silu_f(gg.w));
+    }
+    store4(out + (size_t)at * K + i, v);
+}
+
+template <typename T>
+static bool launch_head_norm_vec4(const float* o, const T* g, int g_stride, const float* w, T* out, int n_rows, int heads,
+                                  int K, float eps, cudaStream_t s, cudaError_t* le) {
+    if ((K != 64 && K != 128) || !fours(o, 4) || !fours(w, 4) || !fours(out, 4) || (g && !fours(g, g_stride))) return false;
+    const long long threads = (long long)n_rows * heads * (K / 4);
+    const dim3 grid((unsigned)((threads + 255) / 256));
+    *le = K == 64 ? launch_kernel(head_norm_gate_vec4_kernel<T, 16>, grid, dim3(256), 0, s, o, g, g_stride, w, out, n_rows, heads, eps)
+                  : launch_kernel(head_norm_gate_vec4_kernel<T, 32>, grid, dim3(256), 0, s, o, g, g_stride, w, out, n_rows, heads, eps);
+    return true;
+}
+
 IB_EXPORT int ib_head_norm_gate(const float* o, const void* g, int g_stride, int act_dtype, const float* w, void* out,
                                 int n_rows, int heads, int K, float eps, void* stream) {
     if (n_rows <= 0) return IB_OK;
@@ -388,7 +567,11 @@ IB_EXPORT int ib_head_norm_gate(const float* o, const void* g, int g_stride, int
     const long long items = (long long)n_rows * heads;
     const unsigned grid = (unsigned)((items + 3) / 4);
     cudaError_t le;
-    if (act_dtype == 0)
+    if (act_dtype == 0 && launch_head_norm_vec4<float>(o, (const float*)g, g_stride, w, (float*)out, n_rows, heads, K, eps, s, &le))
+        ;
+    else if (act_dtype == 1 && launch_head_norm_vec4<bf16>(o, (const bf16*)g, g_stride, w, (bf16*)out, n_rows, heads, K, eps, s, &le))
+        ;
+    else if (act_dtype == 0)
         le = launch_kernel(head_norm_gate_kernel<float>, dim3(grid), dim3(128), 0, s, o, (const float*)g, g_stride, w,
                            (float*)out, n_rows, heads, K, eps);
     else if (act_dtype == 1)
@@ -425,6 +608,47 @@ __global__ void gated_group_norm_kernel(const float* __restrict__ y, const T* __
     }
 }
 
+// The same for groups of 4 NV values a thread, kept in registers between the sum and the store.
+template <typename T, int NV>
+__global__ void gated_group_norm_vec4_kernel(const float* __restrict__ y, const T* __restrict__ z, int z_stride,
+                                             const float* __restrict__ w, T* __restrict__ out, int inner, int group, float eps) {
+    pdl_trigger();
+    pdl_wait();
+    __shared__ float scratch[33];
+    const int row = blockIdx.x, g0 = blockIdx.y * group;
+    float4 v[NV];
+    float ss = 0.f;
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+        const int i = g0 + (k * blockDim.x + threadIdx.x) * 4;
+        const float4 a = load4(y + (size_t)row * inner + i), g = load4(z + (size_t)row * z_stride + i);
+        v[k] = make_float4(a.x * silu_f(g.x), a.y * silu_f(g.y), a.z * silu_f(g.z), a.w * silu_f(g.w));
+        ss += v[k].x * v[k].x + v[k].y * v[k].y + (v[k].z * v[k].z + v[k].w * v[k].w);
+    }
+    ss = block_sum(ss, scratch);
+    const float inv = 1.f / sqrtf(ss / (float)group + eps);
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+        const int i = g0 + (k * blockDim.x + threadIdx.x) * 4;
+        const float4 ww = *reinterpret_cast<const float4*>(w + i);
+        store4(out + (size_t)row * inner + i,
+               make_float4(v[k].x * inv * ww.x, v[k].y * inv * ww.y, v[k].z * inv * ww.z, v[k].w * inv * ww.w));
+    }
+}
+
+template <typename T>
+static bool launch_group_norm_vec4(const float* y, const T* z, int z_stride, const float* w, T* out, int n_rows, int inner,
+                                   int groups, int group, float eps, cudaStream_t s, cudaError_t* le) {
+    const int nv = group <= 2048 ? 1 : 2, threads = group / (4 * nv);
+    if (group % (128 * nv) || threads > 512 || !fours(y, inner) || !fours(z, z_stride) || !fours(w, 4) || !fours(out, inner))
+        return false;
+    *le = nv == 1 ? launch_kernel(gated_group_norm_vec4_kernel<T, 1>, dim3(n_rows, groups), dim3(threads), 0, s, y, z, z_stride, w,
+                                  out, inner, group, eps)
+                  : launch_kernel(gated_group_norm_vec4_kernel<T, 2>, dim3(n_rows, groups), dim3(threads), 0, s, y, z, z_stride, w,
+                                  out, inner, group, eps);
+    return true;
+}
+
 IB_EXPORT int ib_gated_group_norm(const float* y, const void* z, int z_stride, int act_dtype, const float* w,
                                   void* out, int n_rows, int inner, int groups, float eps, void* stream) {
     if (n_rows <= 0) return IB_OK;
@@ -433,7 +657,11 @@ IB_EXPORT int ib_gated_group_norm(const float* y, const void* z, int z_stride, i
     const int group = inner / groups;
     const int threads = group >= 2048 ? 512 : (group >= 512 ? 256 : 128);
     cudaError_t le;
-    if (act_dtype == 0)
+    if (act_dtype == 0 && launch_group_norm_vec4<float>(y, (const float*)z, z_stride, w, (float*)out, n_rows, inner, groups, group, eps, s, &le))
+        ;
+    else if (act_dtype == 1 && launch_group_norm_vec4<bf16>(y, (const bf16*)z, z_stride, w, (bf16*)out, n_rows, inner, groups, group, eps, s, &le))
+        ;
+    else if (act_dtype == 0)
         le = launch_kernel(gated_group_norm_kernel<float>, dim3(n_rows, groups), dim3(threads), 0, s, y,
                            (const float*)z, z_stride, w, (float*)out, inner, group, eps);
     else if (act_dtype == 1)

@@ -15,7 +15,8 @@
 // Decays are multiplied, never divided (a decay may be 0), and a token's result is made from what comes before it only:
 // what a later token brings is left out of the sum, not multiplied by zero.  A chunk's tokens are counted from the entry's
 // first row of the step: a prompt cut elsewhere rounds otherwise.
-// Bound by the multiply-adds (as many as token by token).
+// Bound by the multiply-adds (as many as token by token).  2,048 tokens, 32 heads of 128 x 64: 414 us by scan.cu, 36 + 28 +
+// 67 us here.
 #include "common.cuh"
 
 using namespace ib;
@@ -47,7 +48,7 @@ __device__ __forceinline__ Chunk find_chunk(const int* cu_rows, int n_entries, i
 
 struct SsdParams {
     const float* x;        // [heads][rows][P]
-    const float2* bc;      // [groups][rows][ROWS]: B, C
+    const float* bc;       // [groups][rows][2][ROWS]: B, then C
     const float2* dd;      // [heads][rows]: dt, decay
     const float* d_skip;
     const int* cu_rows;
@@ -71,18 +72,21 @@ __device__ __forceinline__ float2 pfma(float a, float2 b, float2 c) {
     return d;
 }
 
-// dst[t][i] = the first (which = 0) or second of the pairs of L tokens, zeros behind token n; rows `pitch` apart.
-template <int THREADS>
-__device__ __forceinline__ void load_half(float* dst, int pitch, const float2* src, int n, int which) {
-    for (int i = threadIdx.x; i < L * (ROWS / 4); i += THREADS) {
-        const int t = i / (ROWS / 4), c = i % (ROWS / 4) * 4;
-        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (t < n) {
-            const float4 a = __ldcg(reinterpret_cast<const float4*>(src + (size_t)t * ROWS + c));
-            const float4 b = __ldcg(reinterpret_cast<const float4*>(src + (size_t)t * ROWS + c) + 1);
-            v = which ? make_float4(a.y, a.w, b.y, b.w) : make_float4(a.x, a.z, b.x, b.z);
-        }
-        *reinterpret_cast<float4*>(dst + t * pitch + c) = v;
+__device__ __forceinline__ void cp_async16(float* smem, const float* gmem, bool real) {   // zeros where not real
+    const unsigned d = (unsigned)__cvta_generic_to_shared(smem);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(gmem), "r"(real ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_async_land() {   // every thread's copies, for all
+    asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;\n" ::: "memory");
+    __syncthreads();
+}
+// L rows of WIDTH floats, `stride` apart, to rows `pitch` apart; zeros behind row n.
+template <int WIDTH>
+__device__ __forceinline__ void fetch_rows(float* dst, int pitch, const float* src, size_t stride, int n) {
+#pragma unroll 4
+    for (int i = threadIdx.x; i < L * (WIDTH / 4); i += 128) {
+        const int t = i / (WIDTH / 4), c = i % (WIDTH / 4) * 4;
+        cp_async16(dst + t * pitch + c, src + (t < n ? t : 0) * stride + c, t < n);
     }
 }
 
@@ -122,12 +126,12 @@ __global__ void __launch_bounds__(128) ssd_chunk_state_kernel(const SsdParams p)
     const int y = blockIdx.y;
     if (y >= p.heads * slices) {
         const int g = y - p.heads * slices;
-        const float2* src = p.bc + ((size_t)g * p.n_rows + at.row) * ROWS;
+        const float* src = p.bc + ((size_t)g * p.n_rows + at.row) * 2 * ROWS;
         float* cs = smem;
         float* bs = smem + L * PITCH;
-        load_half<128>(bs, PITCH, src, at.n, 0);
-        load_half<128>(cs, PITCH, src, at.n, 1);
-        __syncthreads();
+        fetch_rows<ROWS>(bs, PITCH, src, 2 * ROWS, at.n);
+        fetch_rows<ROWS>(cs, PITCH, src + ROWS, 2 * ROWS, at.n);
+        cp_async_land();
         float acc[4][8] = {};
         dot_tile(cs + (warp * 16 + ly) * PITCH, bs + lx * PITCH, PITCH, acc);
         float* out = p.cb + ((size_t)g * p.chunks + blockIdx.x) * L * L;
@@ -140,6 +144,10 @@ __global__ void __launch_bounds__(128) ssd_chunk_state_kernel(const SsdParams p)
     const int head = y / slices, p0 = y % slices * PT;
     const int grp = head / (p.heads / p.groups);
     const float2* dd = p.dd + (size_t)head * p.n_rows + at.row;
+    float* bs = smem;                // [L][ROWS]
+    float* xs = smem + L * ROWS;     // [L][PT]
+    fetch_rows<ROWS>(bs, ROWS, p.bc + ((size_t)grp * p.n_rows + at.row) * 2 * ROWS, 2 * ROWS, at.n);
+    fetch_rows<PT>(xs, PT, p.x + ((size_t)head * p.n_rows + at.row) * p.P + p0, p.P, at.n);
     if (warp == 0) {   // w_s = dt_s times the decays after s: products from the chunk's end on, two tokens a lane
         const float2 d0 = 2 * lane < at.n ? __ldcg(dd + 2 * lane) : make_float2(0.f, 1.f);
         const float2 d1 = 2 * lane + 1 < at.n ? __ldcg(dd + 2 * lane + 1) : make_float2(0.f, 1.f);
@@ -155,19 +163,13 @@ __global__ void __launch_bounds__(128) ssd_chunk_state_kernel(const SsdParams p)
         w[2 * lane] = d0.x * (d1.y * rest);
         if (lane == 0 && p0 == 0) p.decay[(size_t)head * p.chunks + blockIdx.x] = after;
     }
-    float* bs = smem;                // [L][ROWS]
-    float* xs = smem + L * ROWS;     // [L][PT]
-    load_half<128>(bs, ROWS, p.bc + ((size_t)grp * p.n_rows + at.row) * ROWS, at.n, 0);
-    __syncthreads();
-    const float* x = p.x + ((size_t)head * p.n_rows + at.row) * p.P + p0;
-    for (int i = tid; i < L * (PT / 4); i += 128) {
-        const int t = i / (PT / 4), c = i % (PT / 4) * 4;
-        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (t < at.n) {
-            v = __ldcg(reinterpret_cast<const float4*>(x + (size_t)t * p.P + c));
-            v.x *= w[t]; v.y *= w[t]; v.z *= w[t]; v.w *= w[t];
-        }
-        *reinterpret_cast<float4*>(xs + t * PT + c) = v;
+    cp_async_land();
+#pragma unroll
+    for (int k = 0; k < L * (PT / 4) / 128; ++k) {
+        const int i = tid + k * 128;
+        float4 v = reinterpret_cast<float4*>(xs)[i];
+        const float f = w[i / (PT / 4)];
+        reinterpret_cast<float4*>(xs)[i] = make_float4(v.x * f, v.y * f, v.z * f, v.w * f);
     }
     __syncthreads();
     // a thread: rows warp * 16 + ly * 4 .. + 3 (and, of 128, those 64 further on), columns lx * 4 .. + 3 and 32 further on
@@ -267,30 +269,25 @@ __global__ void __launch_bounds__(128) ssd_chunk_out_kernel(const SsdParams p) {
         dt[tid] = d.x;
         da[tid] = d.y;
     }
-    load_half<128>(cs, PITCH, p.bc + ((size_t)grp * p.n_rows + at.row) * ROWS, at.n, 1);
+    fetch_rows<ROWS>(cs, PITCH, p.bc + (((size_t)grp * p.n_rows + at.row) * 2 + 1) * ROWS, 2 * ROWS, at.n);
     const float* st = p.carry + (((size_t)head * p.chunks + blockIdx.x) * p.P + p0) * ROWS;
+#pragma unroll 4
     for (int i = tid; i < PT * (ROWS / 4); i += 128) {
         const int c = i / (ROWS / 4), r = i % (ROWS / 4) * 4;
-        *reinterpret_cast<float4*>(ss + (c % 4 * 8 + c / 4 % 8 + c / 32 * 32) * PITCH + r) =
-            __ldcg(reinterpret_cast<const float4*>(st + (size_t)c * ROWS + r));
+        cp_async16(ss + (c % 4 * 8 + c / 4 % 8 + c / 32 * 32) * PITCH + r, st + (size_t)c * ROWS + r, true);
     }
-    const float* x = p.x + ((size_t)head * p.n_rows + at.row) * p.P + p0;
-    for (int i = tid; i < L * (PT / 4); i += 128) {
-        const int t = i / (PT / 4), c = i % (PT / 4) * 4;
-        *reinterpret_cast<float4*>(xs + t * PT + c) =
-            t < at.n ? __ldcg(reinterpret_cast<const float4*>(x + (size_t)t * p.P + c)) : make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-    __syncthreads();
+    fetch_rows<PT>(xs, PT, p.x + ((size_t)head * p.n_rows + at.row) * p.P + p0, p.P, at.n);
+    fetch_rows<L>(ms, MP, p.cb + ((size_t)grp * p.chunks + blockIdx.x) * L * L, L, L);
+    cp_async_land();
     {   // a thread walks half of a column s of the weights downwards
         const int s = tid % L, half = tid / L;
-        const float* cb = p.cb + ((size_t)grp * p.chunks + blockIdx.x) * L * L + s;
         const int t1 = half ? L : L / 2, t0 = max(s, half ? L / 2 : 0);
         const float ds = dt[s];
         float d = 1.f;   // D[t][s]
         for (int t = s + 1; t <= t0 && t < L; ++t) d *= da[t];
-#pragma unroll 4
+#pragma unroll 8
         for (int t = t0; t < t1; ++t) {
-            ms[t * MP + s] = d * __ldcg(cb + t * L) * ds;
+            ms[t * MP + s] *= d * ds;
             d *= t + 1 < L ? da[t + 1] : 1.f;
         }
         if (warp == 0) {   // A_t: two tokens a lane
@@ -383,7 +380,7 @@ IB_EXPORT long long ib_ssd_chunk_scratch(int n_rows, int n_entries, int heads, i
     return chunks * ((long long)heads * P * ROWS + (long long)groups * L * L + heads + 4);
 }
 
-// As ib_ssd_scan (scan.cu); P a multiple of 64, x, bc, state, scratch and out 16-byte aligned, state_stride a multiple of 4.
+// As ib_ssd_scan (scan.cu), bc float32 [groups][rows][2][ROWS] (B, then C); P a multiple of 64, x, bc, state, scratch and out 16-byte aligned, state_stride a multiple of 4.
 IB_EXPORT int ib_ssd_chunk(const float* x, const void* bc, const void* dd, int n_rows, const float* d_skip, float* state,
                            long long state_stride, const int* cu_rows, const int* slot_ids, float* out, int n_entries,
                            int heads, int groups, int P, float* scratch, void* stream) {
@@ -396,7 +393,7 @@ IB_EXPORT int ib_ssd_chunk(const float* x, const void* bc, const void* dd, int n
         return IB_ERR_UNSUPPORTED;
     const int chunks = n_rows / L + n_entries;
     if ((long long)heads * (P / PT) + groups > 65535 || n_entries > 65535) return IB_ERR_TOO_LARGE;
-    SsdParams p{x, (const float2*)bc, (const float2*)dd, d_skip, cu_rows, slot_ids, state, state_stride, scratch, nullptr,
+    SsdParams p{x, (const float*)bc, (const float2*)dd, d_skip, cu_rows, slot_ids, state, state_stride, scratch, nullptr,
                 nullptr, out, n_rows, n_entries, chunks, heads, groups, P};
     p.cb = scratch + (size_t)chunks * heads * P * ROWS;
     p.decay = p.cb + (size_t)chunks * groups * L * L;

@@ -156,10 +156,12 @@ def core_lib() -> ctypes.CDLL:
         lib.ib_qk_norm_append.argtypes = [_c_void_p, _c_int, _c_int, _c_void_p, _c_void_p, _c_float, _c_void_p, _c_void_p,
                                           _c_void_p, _c_int, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int,
                                           _c_int, _c_int, _c_void_p, _c_void_p]
+        lib.ib_ssd_prepare_rows.restype = _c_int
         lib.ib_ssd_prepare.argtypes = [_c_void_p, _c_int, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_ll, _c_void_p,
                                        _c_void_p, _c_void_p, _c_void_p, _c_int, _c_void_p, _c_void_p, _c_void_p,
                                        _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int,
                                        _c_void_p]
+        lib.ib_ssd_prepare_rows.argtypes = lib.ib_ssd_prepare.argtypes
         lib.ib_wkv_prepare.argtypes = [_c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_void_p, _c_void_p, _c_void_p,
                                        _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_void_p]
         lib.ib_ssd_prepare.restype = _c_int

@@ -223,15 +223,20 @@ def ssd_scan(xbc: torch.Tensor, dt: torch.Tensor, dt_bias: torch.Tensor, a_log: 
                 b is not None and (b.dtype != torch.float32 or b.numel() != inner + 2 * gn or not b.is_contiguous())):
             raise KernelError("ssd_scan: the convolution's weight [C, taps] and bias [C] must be contiguous float32")
         conv_ptr, conv_stride = _state_ptr(state, conv_offset)
-    core.check(core.core_lib().ib_ssd_prepare(
+    ptr, stride = _state_ptr(state, state_offset)
+    # (prompts in chunks read B and C one after the other, which the pass for rows of fours with four taps writes)
+    chunked = in_chunks(ctx, N, state_rows, vdim, ptr, stride) and out.data_ptr() % 16 == 0 and taps == 4 \
+        and conv_ptr % 16 == 0 and xbc.stride(0) % 4 == 0 and xbc.data_ptr() % (4 * xbc.element_size()) == 0 \
+        and w.data_ptr() % 16 == 0 and (b is None or b.data_ptr() % 16 == 0)
+    prepare = core.core_lib().ib_ssd_prepare_rows if chunked else core.core_lib().ib_ssd_prepare
+    core.check(prepare(
         xbc.data_ptr(), xbc.stride(0), core.dtype_code(xbc.dtype), w.data_ptr() if w is not None else None,
         b.data_ptr() if b is not None else None, conv_ptr, conv_stride, ctx.row_entry.data_ptr(),
         ctx.cu_rows.data_ptr(), ctx.slot_ids.data_ptr(), dt.data_ptr(), dt.stride(0), dt_bias.data_ptr(),
         a_log.data_ptr(), x32.data_ptr(), bc.data_ptr(), dd.data_ptr(), N, ctx.n_entries, inner, gn, heads, state_rows,
         taps,
         core.stream_ptr(xbc)), "ssd_prepare")
-    ptr, stride = _state_ptr(state, state_offset)
-    if in_chunks(ctx, N, state_rows, vdim, ptr, stride) and out.data_ptr() % 16 == 0:
+    if chunked:
         clib = chunk_lib_for(state_rows)
         scratch = torch.empty(clib.ib_ssd_chunk_scratch(N, ctx.n_entries, heads, groups, vdim), dtype=torch.float32,
                               device=xbc.device)

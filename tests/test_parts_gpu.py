@@ -429,8 +429,10 @@ def test_scans_in_chunks_against_one_token_at_a_time(rule, heads, groups, rows, 
                           row_entry=i32([e for e, n in enumerate(lens) for _ in range(n)]))
     size, inner = heads * rows * cols, heads * cols
     start = rnd(E, size)
-    width = 2 * groups * rows + inner + 2 * heads
+    width = 2 * groups * rows + inner + 4 * heads  # (rows of fours)
     x, a_log, dt_bias, skip = rnd(N, width), rnd(heads) * 0.5, rnd(heads) - 1.0, rnd(heads)
+    channels = width - 4 * heads
+    conv, tail = (rnd(channels, 4) * 0.5, rnd(channels), size), size + 3 * channels  # (the last inputs behind the matrices)
 
     def walk(x, stride):
         state = torch.full((E + 1, stride), 7.0, device=DEV)
@@ -438,22 +440,23 @@ def test_scans_in_chunks_against_one_token_at_a_time(rule, heads, groups, rows, 
         out = torch.empty(N, inner, device=DEV)
         if rule == "ssd":
             scan.ssd_scan(x[:, : inner + 2 * groups * rows], x[:, width - heads:], dt_bias, a_log, skip, state, 0, ctx, out,
-                          heads, groups, rows, cols, rt)
+                          heads, groups, rows, cols, rt, conv=conv)
         else:
-            scan.delta_scan(x, 0, width - 2 * heads, width - heads, None, a_log, dt_bias, state, 0, size, ctx, out, heads,
+            scan.delta_scan(x, 0, width - 2 * heads, width - heads, conv[0], a_log, dt_bias, state, 0, size, ctx, out, heads,
                             groups, rows, cols, rt)
         return out, state
 
-    assert scan.in_chunks(ctx, N, rows, cols, 0, size + 8) and not scan.in_chunks(ctx, N, rows, cols, 0, size + 9)
-    out, state = walk(x, size + 8)
-    ref, ref_state = walk(x, size + 9)
+    assert scan.in_chunks(ctx, N, rows, cols, 0, tail + 8) and not scan.in_chunks(ctx, N, rows, cols, 0, tail + 9)
+    out, state = walk(x, tail + 8)
+    ref, ref_state = walk(x, tail + 9)
     assert rel_err(out, ref) < 1e-5 and rel_err(state[:E, :size], ref_state[:E, :size]) < 1e-5
-    assert bool((state[:, size:] == 7.0).all()) and bool((state[E] == 7.0).all())
+    assert torch.equal(state[:, size: tail], ref_state[:, size: tail])
+    assert bool((state[:, tail:] == 7.0).all()) and bool((state[E] == 7.0).all())
     last = next(e for e in range(E) if lens[e] >= 96)
     at = cu[last] + lens[last] - 2  # the token before the entry's last
     bad = x.clone()
     bad[at] = float("nan")
-    got, _ = walk(bad, size + 8)
+    got, _ = walk(bad, tail + 8)
     keep = torch.ones(N, dtype=torch.bool, device=DEV)
     keep[at: at + 2] = False
     assert torch.equal(got[keep], out[keep]) and bool(got[at].isnan().all())
