@@ -807,8 +807,8 @@ IB_EXPORT int ib_pointwise(void* a, const void* b, int b_stride, int act_dtype, 
 // last taps - 1 inputs kept in the state; taps 0: no convolution), then SiLU.
 // Per key head: q <- q / sqrt(sum q^2 + 1e-6) * dk^-1/2, k <- k / sqrt(sum k^2 + 1e-6).
 // Per value head: beta = sigmoid(b), g = exp(-exp(A_log) softplus(a + dt_bias)).
-// Written in 32-bit the way the scan fetches: (k, q) pairs [G][rows][dk], values
-// [H][rows][dv], and (beta, g, k . q, 0) [H][rows].
+// Written in 32-bit the way the scan fetches: (k, q) pairs [G][rows][dk] (`apart`:
+// k, then q, [G][rows][2][dk], for the scan in chunks), values [H][rows][dv], and (beta, g, k . q, 0) [H][rows].
 // One CTA per row; the row's channels meet in shared memory.
 template <typename T>
 __global__ void delta_prepare_kernel(const T* __restrict__ x, int x_stride, int c_off, int b_off, int a_off,
@@ -817,7 +817,7 @@ __global__ void delta_prepare_kernel(const T* __restrict__ x, int x_stride, int 
                                      const int* __restrict__ cu_rows, const int* __restrict__ slot_ids,
                                      const float* __restrict__ a_log, const float* __restrict__ dt_bias,
                                      float2* __restrict__ kq, float* __restrict__ vo, float4* __restrict__ dd,
-                                     int n_rows, int G, int H, int dk, int dv) {
+                                     int n_rows, int G, int H, int dk, int dv, int apart) {
     pdl_trigger();
     pdl_wait();
     extern __shared__ float ch[];  // [C] channels, then [G] k . q
@@ -864,7 +864,12 @@ __global__ void delta_prepare_kernel(const T* __restrict__ x, int x_stride, int 
         float2* dst = kq + ((size_t)g * n_rows + row) * dk;
         for (int i = lane; i < dk; i += 32) {
             const float kn = k[i] * ik, qn = q[i] * iq;
-            dst[i] = make_float2(kn, qn);
+            if (apart) {   // (for the scan in chunks: k, then q)
+                reinterpret_cast<float*>(dst)[i] = kn;
+                reinterpret_cast<float*>(dst)[dk + i] = qn;
+            } else {
+                dst[i] = make_float2(kn, qn);
+            }
             qk = fmaf(kn, qn, qk);
         }
         qk = warp_sum(qk);
@@ -887,7 +892,7 @@ IB_EXPORT int ib_delta_prepare(const void* x, int x_stride, int act_dtype, int c
                                const float* w, int taps, float* state, long long state_stride, const int* row_entry,
                                const int* cu_rows, const int* slot_ids, const float* a_log, const float* dt_bias,
                                void* kq, float* vo, void* dd, int n_rows, int n_entries, int G, int H, int dk, int dv,
-                               void* stream) {
+                               int apart, void* stream) {
     if (n_rows <= 0) return IB_OK;
     if (!x || !a_log || !dt_bias || !kq || !vo || !dd || G <= 0 || H <= 0 || H % G || dk <= 0 || dv <= 0 || taps < 0 ||
         taps > IB_MAX_TAPS || ((uintptr_t)kq & 7) || ((uintptr_t)dd & 15))
@@ -906,7 +911,7 @@ IB_EXPORT int ib_delta_prepare(const void* x, int x_stride, int act_dtype, int c
             cudaFuncSetAttribute(delta_prepare_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         le = launch_kernel(delta_prepare_kernel<float>, dim3(n_rows), dim3(threads), smem, s, (const float*)x, x_stride,
                            c_off, b_off, a_off, w, taps, (const float*)state, state_stride, row_entry, cu_rows,
-                           slot_ids, a_log, dt_bias, (float2*)kq, vo, (float4*)dd, n_rows, G, H, dk, dv);
+                           slot_ids, a_log, dt_bias, (float2*)kq, vo, (float4*)dd, n_rows, G, H, dk, dv, apart);
         if (le == cudaSuccess && taps > 1)
             le = launch_kernel(conv_state_kernel<float>, dim3(n_entries, gy), dim3(128), 0, s, (const float*)x + c_off,
                                x_stride, state, state_stride, cu_rows, slot_ids, C, taps);
@@ -915,7 +920,7 @@ IB_EXPORT int ib_delta_prepare(const void* x, int x_stride, int act_dtype, int c
             cudaFuncSetAttribute(delta_prepare_kernel<bf16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         le = launch_kernel(delta_prepare_kernel<bf16>, dim3(n_rows), dim3(threads), smem, s, (const bf16*)x, x_stride,
                            c_off, b_off, a_off, w, taps, (const float*)state, state_stride, row_entry, cu_rows,
-                           slot_ids, a_log, dt_bias, (float2*)kq, vo, (float4*)dd, n_rows, G, H, dk, dv);
+                           slot_ids, a_log, dt_bias, (float2*)kq, vo, (float4*)dd, n_rows, G, H, dk, dv, apart);
         if (le == cudaSuccess && taps > 1)
             le = launch_kernel(conv_state_kernel<bf16>, dim3(n_entries, gy), dim3(128), 0, s, (const bf16*)x + c_off,
                                x_stride, state, state_stride, cu_rows, slot_ids, C, taps);

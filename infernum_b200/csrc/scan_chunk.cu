@@ -10,7 +10,7 @@
 //
 //   ssd_chunk_state   every chunk at once: sum_s D[L][s] dt_s B_s x_s^T per head, and C_t.B_s per group
 //   ssd_chunk_pass    every state element walks its entry's chunks: S0 of each chunk, the state after the last
-//   ssd_chunk_out     every chunk at once: y
+//   chunk_out         every chunk at once: y
 //
 // Decays are multiplied, never divided (a decay may be 0), and a token's result is made from what comes before it only:
 // what a later token brings is left out of the sum, not multiplied by zero.  A chunk's tokens are counted from the entry's
@@ -49,7 +49,7 @@ __device__ __forceinline__ Chunk find_chunk(const int* cu_rows, int n_entries, i
 struct SsdParams {
     const float* x;        // [heads][rows][P]
     const float* bc;       // [groups][rows][2][ROWS]: B, then C
-    const float2* dd;      // [heads][rows]: dt, decay
+    const float* dd;       // ssd: float2 [heads][rows] (dt, decay); delta: float4 (beta, decay, unused, unused)
     const float* d_skip;
     const int* cu_rows;
     const int* slot_ids;
@@ -143,7 +143,7 @@ __global__ void __launch_bounds__(128) ssd_chunk_state_kernel(const SsdParams p)
     }
     const int head = y / slices, p0 = y % slices * PT;
     const int grp = head / (p.heads / p.groups);
-    const float2* dd = p.dd + (size_t)head * p.n_rows + at.row;
+    const float2* dd = reinterpret_cast<const float2*>(p.dd) + (size_t)head * p.n_rows + at.row;
     float* bs = smem;                // [L][ROWS]
     float* xs = smem + L * ROWS;     // [L][PT]
     fetch_rows<ROWS>(bs, ROWS, p.bc + ((size_t)grp * p.n_rows + at.row) * 2 * ROWS, 2 * ROWS, at.n);
@@ -250,7 +250,9 @@ __global__ void __launch_bounds__(128) ssd_chunk_pass_kernel(const SsdParams p) 
 constexpr int MP = L + 4;   // pitch of the chunk's own weights
 constexpr int OUT_BYTES = (2 * L * PITCH + L * PT + L * MP) * (int)sizeof(float);
 
-__global__ void __launch_bounds__(128) ssd_chunk_out_kernel(const SsdParams p) {
+// DELTA: the same with k for B, q for C and the rule's u for dt x, without a share of x of its own.
+template <bool DELTA>
+__global__ void __launch_bounds__(128) chunk_out_kernel(const SsdParams p) {
     pdl_trigger();
     pdl_wait();
     extern __shared__ __align__(16) float smem[];
@@ -265,9 +267,9 @@ __global__ void __launch_bounds__(128) ssd_chunk_out_kernel(const SsdParams p) {
     const int head = blockIdx.y, p0 = blockIdx.z * PT;
     const int grp = head / (p.heads / p.groups);
     if (tid < L) {
-        const float2 d = tid < at.n ? __ldcg(p.dd + (size_t)head * p.n_rows + at.row + tid) : make_float2(0.f, 1.f);
-        dt[tid] = d.x;
-        da[tid] = d.y;
+        const float* d = p.dd + ((size_t)head * p.n_rows + at.row + tid) * (DELTA ? 4 : 2);
+        dt[tid] = DELTA ? 1.f : tid < at.n ? __ldcg(d) : 0.f;
+        da[tid] = tid < at.n ? __ldcg(d + 1) : 1.f;
     }
     fetch_rows<ROWS>(cs, PITCH, p.bc + (((size_t)grp * p.n_rows + at.row) * 2 + 1) * ROWS, 2 * ROWS, at.n);
     const float* st = p.carry + (((size_t)head * p.chunks + blockIdx.x) * p.P + p0) * ROWS;
@@ -354,7 +356,7 @@ __global__ void __launch_bounds__(128) ssd_chunk_out_kernel(const SsdParams p) {
             }
         }
     }
-    const float skip = p.d_skip[head];
+    const float skip = DELTA ? 0.f : p.d_skip[head];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         const int t = warp * 16 + i * 4 + ly;
@@ -362,12 +364,292 @@ __global__ void __launch_bounds__(128) ssd_chunk_out_kernel(const SsdParams p) {
         float* o = p.out + (size_t)(at.row + t) * p.heads * p.P + (size_t)head * p.P + p0 + lx * 4;
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
-            const float4 v = *reinterpret_cast<const float4*>(xw + t * PT + c * 32);
+            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (!DELTA) v = *reinterpret_cast<const float4*>(xw + t * PT + c * 32);
             *reinterpret_cast<float4*>(o + c * 32) =
                 make_float4(fmaf(skip, v.x, acc[i][4 * c]), fmaf(skip, v.y, acc[i][4 * c + 1]),
                             fmaf(skip, v.z, acc[i][4 * c + 2]), fmaf(skip, v.w, acc[i][4 * c + 3]));
         }
     }
+}
+
+// ---- the gated delta rule ---------------------------------------------------------------------------------------
+//   u_t = beta_t (v_t - A_t k_t.S0 - sum_{s<t} D[t][s] (k_t.k_s) u_s),   o_t = A_t q_t.S0 + sum_{s<=t} D[t][s] (q_t.k_s) u_s,
+//   S <- A_L S0 + sum_s D[L][s] k_s u_s^T:
+// with M[t][s] = beta_t D[t][s] (k_t.k_s) below the diagonal, (I + M) u = beta v - (beta A k) S0, so that
+//   delta_chunk_dots    every chunk at once: k_t.k_s and q_t.k_s per key head
+//   delta_chunk_solve   every chunk at once: U = (I + M)^-1 beta v and W = (I + M)^-1 beta A k, forward substitution
+//                       in blocks of sixteen tokens, a thread two columns
+//   delta_chunk_walk    an entry's chunks in turn: u = U - W S0 and the state after, 32 columns a CTA
+//   chunk_out           every chunk at once: o
+// The walk is the only part that waits for the chunk before: 32 columns a CTA, so that there are four for a head of 128,
+// and the next chunk's operands come while one is worked on.  Two entries of 750 tokens, 16 heads of 128 x 128 on eight key
+// heads: 376 us by scan.cu, 20 + 32 + 113 + 51 us here.
+struct DeltaParams {
+    SsdParams o;           // what chunk_out reads: x is `u`, bc the k and q, cb the q_t.k_s, carry the states before the chunks
+    const float* v;        // [heads][rows][P]
+    float* u;              // [heads][rows][P]: U, then u
+    float* w;              // [heads][rows][ROWS]
+    float* kk;             // [groups][chunks][L][L]: k_t.k_s
+};
+
+__global__ void __launch_bounds__(128) delta_chunk_dots_kernel(const DeltaParams p) {
+    pdl_wait();
+    extern __shared__ __align__(16) float smem[];
+    const Chunk at = find_chunk(p.o.cu_rows, p.o.n_entries, blockIdx.x);
+    if (at.n == 0) return;
+    const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32, ly = lane / 8, lx = lane % 8, g = blockIdx.y;
+    const float* src = p.o.bc + ((size_t)g * p.o.n_rows + at.row) * 2 * ROWS;
+    float* ks = smem;
+    float* qs = smem + L * PITCH;
+    fetch_rows<ROWS>(ks, PITCH, src, 2 * ROWS, at.n);
+    fetch_rows<ROWS>(qs, PITCH, src + ROWS, 2 * ROWS, at.n);
+    cp_async_land();
+    const size_t out = ((size_t)g * p.o.chunks + blockIdx.x) * L * L;
+#pragma unroll 1
+    for (int which = 0; which < 2; ++which) {
+        float acc[4][8] = {};
+        dot_tile((which ? qs : ks) + (warp * 16 + ly) * PITCH, ks + lx * PITCH, PITCH, acc);
+        float* dst = (which ? p.o.cb : p.kk) + out;
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 8; ++j) dst[(warp * 16 + i * 4 + ly) * L + lx + j * 8] = acc[i][j];
+    }
+}
+
+constexpr int SOLVE_COLS = 256, SB = 16;   // columns of a CTA, tokens of a block
+constexpr int SOLVE_BYTES = (L * SOLVE_COLS + 2 * L * MP) * (int)sizeof(float);
+
+__global__ void __launch_bounds__(128) delta_chunk_solve_kernel(const DeltaParams p) {
+    pdl_trigger();
+    pdl_wait();
+    extern __shared__ __align__(16) float smem[];
+    float* X = smem;                      // [L][SOLVE_COLS]: k | v, then W | U
+    float* kks = X + L * SOLVE_COLS;      // [L][MP]
+    float* mt = kks + L * MP;             // [L][MP]: M transposed, mt[s][t]
+    __shared__ float beta[L], da[L], upto[L];
+    const Chunk at = find_chunk(p.o.cu_rows, p.o.n_entries, blockIdx.x);
+    if (at.n == 0) return;
+    const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
+    const int head = blockIdx.y, P = p.o.P, col0 = blockIdx.z * SOLVE_COLS;
+    const int cols = min(SOLVE_COLS, ROWS + P - col0);
+    const int g = head / (p.o.heads / p.o.groups);
+    const float* ksrc = p.o.bc + ((size_t)g * p.o.n_rows + at.row) * 2 * ROWS;
+    const float* vsrc = p.v + ((size_t)head * p.o.n_rows + at.row) * P;
+#pragma unroll 4
+    for (int i = tid; i < L * (SOLVE_COLS / 4); i += 128) {
+        const int t = i / (SOLVE_COLS / 4), c = i % (SOLVE_COLS / 4) * 4, col = col0 + c;
+        if (c < cols)
+            cp_async16(X + t * SOLVE_COLS + c, t >= at.n ? ksrc : col < ROWS ? ksrc + (size_t)t * 2 * ROWS + col
+                                                                             : vsrc + (size_t)t * P + col - ROWS, t < at.n);
+    }
+    fetch_rows<L>(kks, MP, p.kk + ((size_t)g * p.o.chunks + blockIdx.x) * L * L, L, L);
+    if (tid < L) {
+        const float4 d = tid < at.n ? __ldcg(reinterpret_cast<const float4*>(p.o.dd) + (size_t)head * p.o.n_rows + at.row + tid)
+                                    : make_float4(0.f, 1.f, 0.f, 0.f);
+        beta[tid] = d.x;
+        da[tid] = d.y;
+    }
+    cp_async_land();
+    {
+        const int s = tid % L, half = tid / L;
+        const int t1 = half ? L : L / 2, t0 = max(s, half ? L / 2 : 0);
+        float d = 1.f;   // D[t][s]
+        for (int t = s + 1; t <= t0 && t < L; ++t) d *= da[t];
+#pragma unroll 8
+        for (int t = t0; t < t1; ++t) {
+            mt[s * MP + t] = beta[t] * d * kks[t * MP + s];
+            d *= t + 1 < L ? da[t + 1] : 1.f;
+        }
+        if (warp == 0) {   // A_t: two tokens a lane
+            const float d0 = da[2 * lane], d1 = da[2 * lane + 1];
+            float before = d0 * d1;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const float v = __shfl_up_sync(0xffffffffu, before, o);
+                if (lane >= o) before *= v;
+            }
+            float prior = __shfl_up_sync(0xffffffffu, before, 1);
+            if (lane == 0) prior = 1.f;
+            upto[2 * lane] = prior * d0;
+            upto[2 * lane + 1] = prior * d0 * d1;
+        }
+    }
+    __syncthreads();
+    if (2 * tid >= cols) return;
+    const bool is_k = col0 + 2 * tid < ROWS;
+    float* xc = X + 2 * tid;   // (a thread reads and writes its own two columns only)
+#pragma unroll 1
+    for (int b = 0; b < L / SB; ++b) {
+        float2 r[SB];
+#pragma unroll
+        for (int i = 0; i < SB; ++i) {
+            const int t = b * SB + i;
+            const float f = is_k ? beta[t] * upto[t] : beta[t];
+            const float2 v = *reinterpret_cast<const float2*>(xc + t * SOLVE_COLS);
+            r[i] = make_float2(v.x * f, v.y * f);
+        }
+#pragma unroll 2
+        for (int s = 0; s < b * SB; ++s) {
+            const float2 x = *reinterpret_cast<const float2*>(xc + s * SOLVE_COLS);
+#pragma unroll
+            for (int q = 0; q < SB / 4; ++q) {
+                const float4 m = *reinterpret_cast<const float4*>(mt + s * MP + b * SB + 4 * q);
+                r[4 * q] = pfma(-m.x, x, r[4 * q]);
+                r[4 * q + 1] = pfma(-m.y, x, r[4 * q + 1]);
+                r[4 * q + 2] = pfma(-m.z, x, r[4 * q + 2]);
+                r[4 * q + 3] = pfma(-m.w, x, r[4 * q + 3]);
+            }
+        }
+#pragma unroll
+        for (int s = 0; s < SB; ++s) {
+#pragma unroll
+            for (int i = s + 1; i < SB; ++i) r[i] = pfma(-mt[(b * SB + s) * MP + b * SB + i], r[s], r[i]);
+            *reinterpret_cast<float2*>(xc + (b * SB + s) * SOLVE_COLS) = r[s];
+        }
+    }
+    const int col = col0 + 2 * tid;
+    float* dst = is_k ? p.w + ((size_t)head * p.o.n_rows + at.row) * ROWS + col
+                      : p.u + ((size_t)head * p.o.n_rows + at.row) * P + col - ROWS;
+    const size_t step = is_k ? ROWS : P;
+    for (int t = 0; t < at.n; ++t)
+        *reinterpret_cast<float2*>(dst + t * step) = *reinterpret_cast<const float2*>(xc + t * SOLVE_COLS);
+}
+
+constexpr int WC = 32, UP = WC + 4;   // columns of a CTA that walks, pitch of its u
+constexpr int WALK_STAGE = L * PITCH + L * ROWS + L * UP + L * 4;   // floats: W, k, U, gates
+constexpr int WALK_BYTES = (2 * WALK_STAGE + WC * PITCH + L * UP) * (int)sizeof(float);
+
+__global__ void __launch_bounds__(256) delta_chunk_walk_kernel(const DeltaParams p) {
+    pdl_trigger();
+    pdl_wait();
+    extern __shared__ __align__(16) float smem[];
+    float* ss = smem + 2 * WALK_STAGE;    // [WC][PITCH] the state, by columns
+    float* us = ss + WC * PITCH;          // [L][UP] D[L][t] u_t
+    const int e = blockIdx.x, head = blockIdx.y, P = p.o.P, p0 = blockIdx.z * WC;
+    const int first = p.o.cu_rows[e], n = p.o.cu_rows[e + 1] - first;
+    if (n <= 0) return;
+    int chunk = 0;   // the entry's first
+    for (int q = 0; q < e; ++q) {
+        const int m = p.o.cu_rows[q + 1] - p.o.cu_rows[q];
+        if (m > 0) chunk += (m + L - 1) / L;
+    }
+    const int count = (n + L - 1) / L;
+    const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32, ly = lane / 8, lx = lane % 8;
+    const int g = head / (p.o.heads / p.o.groups);
+    auto fetch = [&](int c) {
+        float* st = smem + (c & 1) * WALK_STAGE;
+        const size_t row = first + c * L;
+        const int m = min(L, n - c * L);
+        const float* w = p.w + ((size_t)head * p.o.n_rows + row) * ROWS;
+        const float* k = p.o.bc + ((size_t)g * p.o.n_rows + row) * 2 * ROWS;
+        const float* u = p.u + ((size_t)head * p.o.n_rows + row) * P + p0;
+        const float* d = p.o.dd + ((size_t)head * p.o.n_rows + row) * 4;
+#pragma unroll 4
+        for (int i = tid; i < L * (ROWS / 4); i += 256) {
+            const int t = i / (ROWS / 4), c4 = i % (ROWS / 4) * 4, from = t < m ? t : 0;
+            cp_async16(st + t * PITCH + c4, w + (size_t)from * ROWS + c4, t < m);
+            cp_async16(st + L * PITCH + t * ROWS + c4, k + (size_t)from * 2 * ROWS + c4, t < m);
+        }
+#pragma unroll
+        for (int i = tid; i < L * (WC / 4); i += 256) {
+            const int t = i / (WC / 4), c4 = i % (WC / 4) * 4, from = t < m ? t : 0;
+            cp_async16(st + L * PITCH + L * ROWS + t * UP + c4, u + (size_t)from * P + c4, t < m);
+        }
+        if (tid < L) cp_async16(st + L * PITCH + L * ROWS + L * UP + tid * 4, d + (tid < m ? tid : 0) * 4, tid < m);
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+    };
+    // a thread's part of the state: rows r4 .. + 3 of columns pg * CPT .. + CPT - 1
+    constexpr int RG = ROWS / 4, CPT = WC * RG / 256;   // lanes a column, columns a thread
+    const int r4 = tid % RG * 4, pg = tid / RG;
+    float* state = p.o.state + (long long)p.o.slot_ids[e] * p.o.state_stride + ((size_t)head * P + p0 + pg * CPT) * ROWS + r4;
+    float4 S[CPT];
+#pragma unroll
+    for (int j = 0; j < CPT; ++j) {
+        S[j] = __ldcg(reinterpret_cast<const float4*>(state + (size_t)j * ROWS));
+        *reinterpret_cast<float4*>(ss + (pg * CPT + j) * PITCH + r4) = S[j];
+    }
+    fetch(0);
+    for (int c = 0; c < count; ++c) {
+        asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+        __syncthreads();   // the stage has come; the state is in shared memory; the other stage is read
+        if (c + 1 < count) fetch(c + 1);
+        const float* st = smem + (c & 1) * WALK_STAGE;
+        const float* kc = st + L * PITCH;
+        const float* uc = kc + L * ROWS;
+        const float* dc = uc + L * UP;
+        const int m = min(L, n - c * L);
+        // D[L][t] of two tokens a lane, in every warp; the chunk's decay in lane 0
+        const float g0 = 2 * lane < m ? dc[2 * lane * 4 + 1] : 1.f, g1 = 2 * lane + 1 < m ? dc[(2 * lane + 1) * 4 + 1] : 1.f;
+        float after = g0 * g1;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const float v = __shfl_down_sync(0xffffffffu, after, o);
+            if (lane + o < 32) after *= v;
+        }
+        float rest = __shfl_down_sync(0xffffffffu, after, 1);
+        if (lane == 31) rest = 1.f;
+        const float w1 = rest, w0 = g1 * rest, all = __shfl_sync(0xffffffffu, after, 0);
+        // the state before the chunk, for the results
+        float* carry = p.o.carry + (((size_t)head * p.o.chunks + chunk + c) * P + p0 + pg * CPT) * ROWS + r4;
+#pragma unroll
+        for (int j = 0; j < CPT; ++j) __stcg(reinterpret_cast<float4*>(carry + (size_t)j * ROWS), S[j]);
+        // u = U - W S0: a thread tokens warp * 8 + ly and 4 further on, columns lx + 8 j
+        float acc[2][4] = {};
+        const float* wt = st + (warp * 8 + ly) * PITCH;
+        const float* sp = ss + lx * PITCH;
+#pragma unroll 4
+        for (int k = 0; k < ROWS; k += 4) {
+            float4 a[2], b[4];
+#pragma unroll
+            for (int i = 0; i < 2; ++i) a[i] = *reinterpret_cast<const float4*>(wt + i * 4 * PITCH + k);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) b[j] = *reinterpret_cast<const float4*>(sp + j * 8 * PITCH + k);
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    acc[i][j] = fmaf(a[i].x, b[j].x, acc[i][j]);
+                    acc[i][j] = fmaf(a[i].y, b[j].y, acc[i][j]);
+                    acc[i][j] = fmaf(a[i].z, b[j].z, acc[i][j]);
+                    acc[i][j] = fmaf(a[i].w, b[j].w, acc[i][j]);
+                }
+        }
+        float* ug = p.u + ((size_t)head * p.o.n_rows + first + c * L) * P + p0;
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const int t = warp * 8 + i * 4 + ly;
+            const float even = __shfl_sync(0xffffffffu, w0, t / 2), odd = __shfl_sync(0xffffffffu, w1, t / 2);
+            const float f = t & 1 ? odd : even;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const float v = uc[t * UP + lx + 8 * j] - acc[i][j];
+                if (t < m) __stcg(ug + (size_t)t * P + lx + 8 * j, v);
+                us[t * UP + lx + 8 * j] = t < m ? f * v : 0.f;
+            }
+        }
+        __syncthreads();
+        // S <- A_L S0 + sum_t k_t (D[L][t] u_t)^T
+#pragma unroll
+        for (int j = 0; j < CPT; ++j) S[j] = make_float4(S[j].x * all, S[j].y * all, S[j].z * all, S[j].w * all);
+#pragma unroll 8
+        for (int t = 0; t < L; ++t) {
+            const float4 k = *reinterpret_cast<const float4*>(kc + t * ROWS + r4);
+#pragma unroll
+            for (int j = 0; j < CPT; ++j) {
+                const float v = us[t * UP + pg * CPT + j];
+                S[j].x = fmaf(k.x, v, S[j].x);
+                S[j].y = fmaf(k.y, v, S[j].y);
+                S[j].z = fmaf(k.z, v, S[j].z);
+                S[j].w = fmaf(k.w, v, S[j].w);
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < CPT; ++j) *reinterpret_cast<float4*>(ss + (pg * CPT + j) * PITCH + r4) = S[j];
+    }
+#pragma unroll
+    for (int j = 0; j < CPT; ++j) *reinterpret_cast<float4*>(state + (size_t)j * ROWS) = S[j];
 }
 
 }  // namespace
@@ -393,7 +675,7 @@ IB_EXPORT int ib_ssd_chunk(const float* x, const void* bc, const void* dd, int n
         return IB_ERR_UNSUPPORTED;
     const int chunks = n_rows / L + n_entries;
     if ((long long)heads * (P / PT) + groups > 65535 || n_entries > 65535) return IB_ERR_TOO_LARGE;
-    SsdParams p{x, (const float*)bc, (const float2*)dd, d_skip, cu_rows, slot_ids, state, state_stride, scratch, nullptr,
+    SsdParams p{x, (const float*)bc, (const float*)dd, d_skip, cu_rows, slot_ids, state, state_stride, scratch, nullptr,
                 nullptr, out, n_rows, n_entries, chunks, heads, groups, P};
     p.cb = scratch + (size_t)chunks * heads * P * ROWS;
     p.decay = p.cb + (size_t)chunks * groups * L * L;
@@ -401,7 +683,7 @@ IB_EXPORT int ib_ssd_chunk(const float* x, const void* bc, const void* dd, int n
     if (!attr_done) {
         cudaError_t e = cudaFuncSetAttribute(ssd_chunk_state_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, STATE_BYTES);
         if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(ssd_chunk_out_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, OUT_BYTES);
+            e = cudaFuncSetAttribute(chunk_out_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, OUT_BYTES);
         if (e != cudaSuccess) return (int)e;
         attr_done = true;
     }
@@ -411,7 +693,61 @@ IB_EXPORT int ib_ssd_chunk(const float* x, const void* bc, const void* dd, int n
     if (le == cudaSuccess)
         le = launch_kernel(ssd_chunk_pass_kernel, dim3((P * ROWS / 4 + 127) / 128, heads, n_entries), dim3(128), 0, s, p);
     if (le == cudaSuccess)
-        le = launch_kernel(ssd_chunk_out_kernel, dim3(chunks, heads, P / PT), dim3(128), (size_t)OUT_BYTES, s, p);
+        le = launch_kernel(chunk_out_kernel<false>, dim3(chunks, heads, P / PT), dim3(128), (size_t)OUT_BYTES, s, p);
+    if (le != cudaSuccess) return (int)le;
+    IB_LAUNCH_CHECK();
+    return IB_OK;
+}
+
+IB_EXPORT long long ib_delta_chunk_scratch(int n_rows, int n_entries, int heads, int groups, int P) {
+    const long long chunks = n_rows / L + n_entries;
+    return chunks * ((long long)heads * P * ROWS + 2LL * groups * L * L) + (long long)heads * n_rows * (P + ROWS);
+}
+
+// As ib_delta_scan (scan.cu), kq float32 [groups][rows][2][ROWS] (k, then q); P a multiple of 64, alignments as above, dd
+// 16-byte aligned.
+IB_EXPORT int ib_delta_chunk(const float* v, const void* kq, const void* dd, int n_rows, float* state,
+                             long long state_stride, const int* cu_rows, const int* slot_ids, float* out, int n_entries,
+                             int heads, int groups, int P, float* scratch, void* stream) {
+    if (n_entries <= 0 || n_rows <= 0) return IB_OK;
+    if (!v || !kq || !dd || !state || !cu_rows || !slot_ids || !out || !scratch || heads <= 0 || groups <= 0 ||
+        heads % groups || P <= 0)
+        return IB_ERR_BAD_ARG;
+    if (P % PT || state_stride % 4 || (((uintptr_t)v | (uintptr_t)kq | (uintptr_t)dd | (uintptr_t)state | (uintptr_t)scratch |
+                                        (uintptr_t)out) & 15))
+        return IB_ERR_UNSUPPORTED;
+    const int chunks = n_rows / L + n_entries;
+    if (heads > 65535 || n_entries > 65535 || P / WC > 65535) return IB_ERR_TOO_LARGE;
+    DeltaParams p;
+    p.o = SsdParams{nullptr, (const float*)kq, (const float*)dd, nullptr, cu_rows, slot_ids, state, state_stride, scratch,
+                    nullptr, nullptr, out, n_rows, n_entries, chunks, heads, groups, P};
+    p.o.cb = scratch + (size_t)chunks * heads * P * ROWS;
+    p.kk = p.o.cb + (size_t)chunks * groups * L * L;
+    p.u = p.kk + (size_t)chunks * groups * L * L;
+    p.w = p.u + (size_t)heads * n_rows * P;
+    p.o.x = p.u;
+    p.v = v;
+    static bool attr_done = false;
+    if (!attr_done) {
+        cudaError_t e = cudaFuncSetAttribute(delta_chunk_dots_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, STATE_BYTES);
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(delta_chunk_solve_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SOLVE_BYTES);
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(delta_chunk_walk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, WALK_BYTES);
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(chunk_out_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, OUT_BYTES);
+        if (e != cudaSuccess) return (int)e;
+        attr_done = true;
+    }
+    cudaStream_t s = (cudaStream_t)stream;
+    cudaError_t le = launch_kernel_in_order(delta_chunk_dots_kernel, dim3(chunks, groups), dim3(128), (size_t)STATE_BYTES, s, p);
+    if (le == cudaSuccess)
+        le = launch_kernel(delta_chunk_solve_kernel, dim3(chunks, heads, (ROWS + P + SOLVE_COLS - 1) / SOLVE_COLS), dim3(128),
+                           (size_t)SOLVE_BYTES, s, p);
+    if (le == cudaSuccess)
+        le = launch_kernel(delta_chunk_walk_kernel, dim3(n_entries, heads, P / WC), dim3(256), (size_t)WALK_BYTES, s, p);
+    if (le == cudaSuccess)
+        le = launch_kernel(chunk_out_kernel<true>, dim3(chunks, heads, P / PT), dim3(128), (size_t)OUT_BYTES, s, p.o);
     if (le != cudaSuccess) return (int)le;
     IB_LAUNCH_CHECK();
     return IB_OK;

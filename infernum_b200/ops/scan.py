@@ -59,7 +59,11 @@ def chunk_lib_for(rows: int) -> ctypes.CDLL:
         lib.ib_ssd_chunk_scratch.restype = _c_ll
         lib.ib_ssd_chunk.argtypes = [_c_void_p, _c_void_p, _c_void_p, _c_int, _c_void_p, _c_void_p, _c_ll, _c_void_p,
                                      _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_void_p, _c_void_p]
-        for fn in (lib.ib_ssd_chunk, lib.ib_scan_chunk_rows):
+        lib.ib_delta_chunk_scratch.argtypes = lib.ib_ssd_chunk_scratch.argtypes
+        lib.ib_delta_chunk_scratch.restype = _c_ll
+        lib.ib_delta_chunk.argtypes = [_c_void_p, _c_void_p, _c_void_p, _c_int, _c_void_p, _c_ll, _c_void_p, _c_void_p,
+                                       _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_void_p, _c_void_p]
+        for fn in (lib.ib_ssd_chunk, lib.ib_delta_chunk, lib.ib_scan_chunk_rows):
             fn.restype = _c_int
         if lib.ib_scan_chunk_rows() != rows:
             raise KernelError(f"scan module for {rows} state rows was built for another number")
@@ -69,7 +73,7 @@ def chunk_lib_for(rows: int) -> ctypes.CDLL:
 
 def in_chunks(ctx, n_rows: int, rows: int, cols: int, state_ptr: int, state_stride: int) -> bool:
     """Whether a step's scan runs in chunks of 64 tokens: where a request brings a prompt (below some hundred tokens the
-    walk token by token is over before three launches are), and not for its sake alone beside many decoded tokens, each
+    walk token by token is over before three or four launches are), and not for its sake alone beside many decoded tokens, each
     of which would be a chunk."""
     most = getattr(ctx, "max_rows_per_entry", n_rows)
     return (rows in CHUNK_ROWS and cols % 64 == 0 and state_ptr % 16 == 0 and state_stride % 4 == 0
@@ -287,13 +291,22 @@ def delta_scan(proj: torch.Tensor, c_off: int, b_off: int, a_off: int, conv_w: O
     v32 = torch.empty((heads, N, vdim), dtype=torch.float32, device=dev)
     dd = torch.empty((heads, N, 4), dtype=torch.float32, device=dev)
     conv_ptr, conv_stride = _state_ptr(state, conv_offset)
+    ptr, stride = _state_ptr(state, state_offset)
+    chunked = in_chunks(ctx, N, dim, vdim, ptr, stride) and out.data_ptr() % 16 == 0
     core.check(core.core_lib().ib_delta_prepare(
         proj.data_ptr(), proj.stride(0), core.dtype_code(proj.dtype), int(c_off), int(b_off), int(a_off),
         conv_w.data_ptr() if conv_w is not None else None, taps, conv_ptr, conv_stride, ctx.row_entry.data_ptr(),
         ctx.cu_rows.data_ptr(), ctx.slot_ids.data_ptr(), a_log.data_ptr(), dt_bias.data_ptr(), kq.data_ptr(),
-        v32.data_ptr(), dd.data_ptr(), N, ctx.n_entries, kv_heads, heads, dim, vdim, core.stream_ptr(proj)),
+        v32.data_ptr(), dd.data_ptr(), N, ctx.n_entries, kv_heads, heads, dim, vdim, int(chunked), core.stream_ptr(proj)),
         "delta_prepare")
-    ptr, stride = _state_ptr(state, state_offset)
+    if chunked:
+        clib = chunk_lib_for(dim)
+        scratch = torch.empty(clib.ib_delta_chunk_scratch(N, ctx.n_entries, heads, kv_heads, vdim), dtype=torch.float32,
+                              device=dev)
+        core.check(clib.ib_delta_chunk(v32.data_ptr(), kq.data_ptr(), dd.data_ptr(), N, ptr, stride, ctx.cu_rows.data_ptr(),
+                                       ctx.slot_ids.data_ptr(), out.data_ptr(), ctx.n_entries, heads, kv_heads, vdim,
+                                       scratch.data_ptr(), core.stream_ptr(proj)), "delta_chunk")
+        return
     sm = rt.options.get("sm_count") or SM_COUNT_FALLBACK
     slices = choose_col_slices(ctx.n_entries, heads, vdim, lib.ib_scan_split(), sm)
     core.check(lib.ib_delta_scan(v32.data_ptr(), kq.data_ptr(), dd.data_ptr(), N, ptr, stride, ctx.cu_rows.data_ptr(),

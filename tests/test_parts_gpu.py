@@ -410,7 +410,9 @@ def test_latent_attention_over_made_keys_against_the_plain_kernel(heads, window,
     assert outs[0].isfinite().all() and rel_err(outs[0], outs[1]) < TOL[torch.bfloat16]
 
 
-@pytest.mark.parametrize("rule, heads, groups, rows, cols", [("ssd", 4, 2, 128, 64), ("ssd", 3, 1, 64, 128)])
+@pytest.mark.parametrize("rule, heads, groups, rows, cols", [("ssd", 4, 2, 128, 64), ("ssd", 3, 1, 64, 128),
+                                                             ("delta", 4, 2, 128, 128), ("delta", 3, 3, 64, 64),
+                                                             ("delta", 2, 1, 128, 192)])
 @pytest.mark.parametrize("lens", [[96], [128, 1, 63], [131, 64, 200], [0, 300], [65, 100, 193, 40]])
 def test_scans_in_chunks_against_one_token_at_a_time(rule, heads, groups, rows, cols, lens):
     """The kernels for prompts against the token-by-token one, which a state whose rows are an odd number of floats apart
