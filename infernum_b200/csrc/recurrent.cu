@@ -222,10 +222,62 @@ IB_EXPORT int ib_ssd_prepare(const void* x, int x_stride, int act_dtype, const f
     return IB_OK;
 }
 
+// A thread's four channels of a causal convolution over rows r0 .. r1 - 1 and SiLU, emit(row, four values): the last inputs
+// stay in registers, so an input is read once instead of once a tap.
+constexpr int CONV_ROWS = 8, CONV_TAPS = 4;
+template <typename T, typename F>
+__device__ __forceinline__ void conv_silu_rows(const T* __restrict__ x, int x_stride, const float* __restrict__ w, float4 bias,
+                                               const float* __restrict__ state, long long state_stride,
+                                               const int* __restrict__ row_entry, const int* __restrict__ cu_rows,
+                                               const int* __restrict__ slot_ids, int C, int c, int r0, int r1, F emit) {
+    float4 in[CONV_ROWS];
+#pragma unroll
+    for (int i = 0; i < CONV_ROWS; ++i)
+        if (r0 + i < r1) in[i] = load4(x + (size_t)(r0 + i) * x_stride + c);
+    float wt[4][CONV_TAPS];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const float4 v = *reinterpret_cast<const float4*>(w + (size_t)(c + q) * CONV_TAPS);
+        wt[q][0] = v.x; wt[q][1] = v.y; wt[q][2] = v.z; wt[q][3] = v.w;
+    }
+    int e = row_entry[r0], first = cu_rows[e], next = cu_rows[e + 1];
+    float4 past[CONV_TAPS - 1];
+#pragma unroll
+    for (int i = 0; i < CONV_ROWS; ++i) {
+        const int row = r0 + i;
+        if (row >= r1) break;
+        if (row >= next) {
+            e = row_entry[row];
+            first = cu_rows[e];
+            next = cu_rows[e + 1];
+        }
+        if (i == 0 || row == first) {   // (the inputs before an entry's first row are in its state)
+            const float* st = state + (long long)slot_ids[e] * state_stride;
+#pragma unroll
+            for (int j = 0; j < CONV_TAPS - 1; ++j) {
+                const int src = row - (CONV_TAPS - 1) + j;
+                past[j] = src >= first ? load4(x + (size_t)src * x_stride + c)
+                                       : load4(st + (size_t)(CONV_TAPS - 1 - (first - src)) * C + c);
+            }
+        }
+        float4 v = bias;
+#pragma unroll
+        for (int j = 0; j < CONV_TAPS; ++j) {
+            const float4 a = j < CONV_TAPS - 1 ? past[j < CONV_TAPS - 1 ? j : 0] : in[i];
+            v.x = fmaf(wt[0][j], a.x, v.x);
+            v.y = fmaf(wt[1][j], a.y, v.y);
+            v.z = fmaf(wt[2][j], a.z, v.z);
+            v.w = fmaf(wt[3][j], a.w, v.w);
+        }
+#pragma unroll
+        for (int j = 0; j + 1 < CONV_TAPS - 1; ++j) past[j] = past[j + 1];
+        past[CONV_TAPS - 2] = in[i];
+        emit(row, make_float4(silu_f(v.x), silu_f(v.y), silu_f(v.z), silu_f(v.w)));
+    }
+}
+
 // The same for prompts, whose scan goes in chunks (scan_chunk.cu): B and C of a token one after the other, bc [groups]
-// [rows][2][state].  A thread has four channels and walks ROWS rows of them with the last inputs in registers, so an
-// input is read once instead of once a tap: 2,048 rows of 2,304 channels 48 us -> 29 us.
-constexpr int SSD_ROWS = 16, SSD_TAPS = 4;
+// [rows][2][state].  2,048 rows of 2,304 channels 48 us -> 29 us.
 template <typename T>
 __global__ void __launch_bounds__(128)
 ssd_prepare_rows_kernel(const T* __restrict__ x, int x_stride, const float* __restrict__ w, const float* __restrict__ b,
@@ -236,7 +288,7 @@ ssd_prepare_rows_kernel(const T* __restrict__ x, int x_stride, const float* __re
                         int n_rows, int P, int state_rows) {
     pdl_trigger();
     pdl_wait();
-    const int r0 = blockIdx.x * SSD_ROWS, r1 = min(n_rows, r0 + SSD_ROWS);
+    const int r0 = blockIdx.x * CONV_ROWS, r1 = min(n_rows, r0 + CONV_ROWS);
     const int C = inner + 2 * gn;
     if (blockIdx.y == gridDim.y - 1) {   // the gates of the heads
         for (int i = threadIdx.x; i < heads * (r1 - r0); i += blockDim.x) {
@@ -249,45 +301,8 @@ ssd_prepare_rows_kernel(const T* __restrict__ x, int x_stride, const float* __re
     }
     const int c = (blockIdx.y * 128 + threadIdx.x) * 4;
     if (c >= C) return;
-    float4 in[SSD_ROWS];
-#pragma unroll
-    for (int i = 0; i < SSD_ROWS; ++i)
-        if (r0 + i < r1) in[i] = load4(x + (size_t)(r0 + i) * x_stride + c);
-    float wt[4][SSD_TAPS];
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        const float4 v = *reinterpret_cast<const float4*>(w + (size_t)(c + q) * SSD_TAPS);
-        wt[q][0] = v.x; wt[q][1] = v.y; wt[q][2] = v.z; wt[q][3] = v.w;
-    }
     const float4 bias = b ? *reinterpret_cast<const float4*>(b + c) : make_float4(0.f, 0.f, 0.f, 0.f);
-    float4 past[SSD_TAPS - 1];
-#pragma unroll
-    for (int i = 0; i < SSD_ROWS; ++i) {
-        const int row = r0 + i;
-        if (row >= r1) break;
-        const int e = row_entry[row], first = cu_rows[e];
-        if (i == 0 || row == first) {   // (the inputs before an entry's first row are in its state)
-            const float* st = state + (long long)slot_ids[e] * state_stride;
-#pragma unroll
-            for (int j = 0; j < SSD_TAPS - 1; ++j) {
-                const int src = row - (SSD_TAPS - 1) + j;
-                past[j] = src >= first ? load4(x + (size_t)src * x_stride + c)
-                                       : load4(st + (size_t)(SSD_TAPS - 1 - (first - src)) * C + c);
-            }
-        }
-        float4 v = bias;
-#pragma unroll
-        for (int j = 0; j < SSD_TAPS; ++j) {
-            const float4 a = j < SSD_TAPS - 1 ? past[j < SSD_TAPS - 1 ? j : 0] : in[i];
-            v.x = fmaf(wt[0][j], a.x, v.x);
-            v.y = fmaf(wt[1][j], a.y, v.y);
-            v.z = fmaf(wt[2][j], a.z, v.z);
-            v.w = fmaf(wt[3][j], a.w, v.w);
-        }
-#pragma unroll
-        for (int j = 0; j + 1 < SSD_TAPS - 1; ++j) past[j] = past[j + 1];
-        past[SSD_TAPS - 2] = in[i];
-        v = make_float4(silu_f(v.x), silu_f(v.y), silu_f(v.z), silu_f(v.w));
+    conv_silu_rows(x, x_stride, w, bias, state, state_stride, row_entry, cu_rows, slot_ids, C, c, r0, r1, [&](int row, float4 v) {
         float* dst;
         if (c < inner) {
             dst = xo + ((size_t)(c / P) * n_rows + row) * P + c % P;
@@ -296,14 +311,14 @@ ssd_prepare_rows_kernel(const T* __restrict__ x, int x_stride, const float* __re
             dst = bc + (((size_t)(k / state_rows) * n_rows + row) * 2 + (c < inner + gn ? 0 : 1)) * state_rows + k % state_rows;
         }
         store4(dst, v);
-    }
+    });
 }
 
 // 1 where ib_ssd_prepare_rows takes these operands.
 template <typename T>
 static bool ssd_rows_suit(const T* x, int x_stride, const float* w, const float* b, const float* state,
                           long long state_stride, int inner, int gn, int heads, int state_rows, int taps) {
-    return w && taps == SSD_TAPS && fours(x, x_stride) && inner % 4 == 0 && gn % 4 == 0 && state_rows % 4 == 0 &&
+    return w && taps == CONV_TAPS && fours(x, x_stride) && inner % 4 == 0 && gn % 4 == 0 && state_rows % 4 == 0 &&
            inner / heads % 4 == 0 && ((uintptr_t)w & 15) == 0 && ((uintptr_t)b & 15) == 0 && ((uintptr_t)state & 15) == 0 &&
            state_stride % 4 == 0;
 }
@@ -318,7 +333,7 @@ IB_EXPORT int ib_ssd_prepare_rows(const void* x, int x_stride, int act_dtype, co
         state_rows <= 0 || gn % state_rows || !w || !state || !row_entry || !cu_rows || !slot_ids || n_entries <= 0)
         return IB_ERR_BAD_ARG;
     const int C = inner + 2 * gn;
-    const dim3 grid((n_rows + SSD_ROWS - 1) / SSD_ROWS, (C / 4 + 127) / 128 + 1);
+    const dim3 grid((n_rows + CONV_ROWS - 1) / CONV_ROWS, (C / 4 + 127) / 128 + 1);
     const int gy = min(64, (C + 127) / 128);
     cudaStream_t s = (cudaStream_t)stream;
     cudaError_t le;
@@ -888,6 +903,49 @@ __global__ void delta_prepare_kernel(const T* __restrict__ x, int x_stride, int 
     }
 }
 
+// The same for prompts, whose scan goes in chunks (scan_chunk.cu): k, then q, kq [G][rows][2][dk], and no k . q.  dk is 64
+// or 128, a half or a whole warp's channels.
+template <typename T>
+__global__ void __launch_bounds__(128)
+delta_prepare_rows_kernel(const T* __restrict__ x, int x_stride, int c_off, int b_off, int a_off, const float* __restrict__ w,
+                          const float* __restrict__ state, long long state_stride, const int* __restrict__ row_entry,
+                          const int* __restrict__ cu_rows, const int* __restrict__ slot_ids, const float* __restrict__ a_log,
+                          const float* __restrict__ dt_bias, float* __restrict__ kq, float* __restrict__ vo,
+                          float4* __restrict__ dd, int n_rows, int G, int H, int dk, int dv) {
+    pdl_trigger();
+    pdl_wait();
+    const int r0 = blockIdx.x * CONV_ROWS, r1 = min(n_rows, r0 + CONV_ROWS);
+    const int keys = G * dk, C = 2 * keys + H * dv;
+    if (blockIdx.y == gridDim.y - 1) {   // the gates of the heads
+        for (int i = threadIdx.x; i < H * (r1 - r0); i += blockDim.x) {
+            const int h = i % H, row = r0 + i / H;
+            const float b = to_f32(x[(size_t)row * x_stride + b_off + h]);
+            const float a = to_f32(x[(size_t)row * x_stride + a_off + h]) + dt_bias[h];
+            const float sp = a > 20.f ? a : log1pf(expf(a));
+            dd[(size_t)h * n_rows + row] = make_float4(1.f / (1.f + expf(-b)), expf(-expf(a_log[h]) * sp), 0.f, 0.f);
+        }
+        return;
+    }
+    const int c = (blockIdx.y * 128 + threadIdx.x) * 4;
+    if (c >= C) return;   // (whole warps have q and k, or none of their lanes has)
+    const float q_scale = (float)(1.0 / sqrt((double)dk));
+    conv_silu_rows(x + c_off, x_stride, w, make_float4(0.f, 0.f, 0.f, 0.f), state, state_stride, row_entry, cu_rows, slot_ids,
+                   C, c, r0, r1, [&](int row, float4 v) {
+        if (c >= 2 * keys) {
+            const int k = c - 2 * keys;
+            store4(vo + ((size_t)(k / dv) * n_rows + row) * dv + k % dv, v);
+            return;
+        }
+        float sum = fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, v.w * v.w)));
+        for (int o = dk / 8; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        const bool is_k = c >= keys;
+        const float f = (is_k ? 1.f : q_scale) / sqrtf(sum + 1e-6f);
+        const int k = is_k ? c - keys : c;
+        store4(kq + (((size_t)(k / dk) * n_rows + row) * 2 + (is_k ? 0 : 1)) * dk + k % dk,
+               make_float4(v.x * f, v.y * f, v.z * f, v.w * f));
+    });
+}
+
 IB_EXPORT int ib_delta_prepare(const void* x, int x_stride, int act_dtype, int c_off, int b_off, int a_off,
                                const float* w, int taps, float* state, long long state_stride, const int* row_entry,
                                const int* cu_rows, const int* slot_ids, const float* a_log, const float* dt_bias,
@@ -906,27 +964,32 @@ IB_EXPORT int ib_delta_prepare(const void* x, int x_stride, int act_dtype, int c
     const int threads = C >= 2048 ? 512 : 256;
     const int gy = min(64, (C + 127) / 128);
     cudaError_t le;
+#define IB_PREP(T)                                                                                                        \
+    const T* xt = (const T*)x;                                                                                            \
+    if (apart && taps == CONV_TAPS && (dk == 64 || dk == 128) && dv % 4 == 0 && fours(xt + c_off, x_stride) &&            \
+        state_stride % 4 == 0 && (((uintptr_t)w | (uintptr_t)state | (uintptr_t)kq | (uintptr_t)vo) & 15) == 0) {         \
+        const dim3 grid((n_rows + CONV_ROWS - 1) / CONV_ROWS, (C / 4 + 127) / 128 + 1);                                   \
+        le = launch_kernel(delta_prepare_rows_kernel<T>, grid, dim3(128), 0, s, xt, x_stride, c_off, b_off, a_off, w,     \
+                           (const float*)state, state_stride, row_entry, cu_rows, slot_ids, a_log, dt_bias, (float*)kq,   \
+                           vo, (float4*)dd, n_rows, G, H, dk, dv);                                                        \
+    } else {                                                                                                              \
+        if (smem > 48 * 1024)                                                                                             \
+            cudaFuncSetAttribute(delta_prepare_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);        \
+        le = launch_kernel(delta_prepare_kernel<T>, dim3(n_rows), dim3(threads), smem, s, xt, x_stride, c_off, b_off,     \
+                           a_off, w, taps, (const float*)state, state_stride, row_entry, cu_rows, slot_ids, a_log,        \
+                           dt_bias, (float2*)kq, vo, (float4*)dd, n_rows, G, H, dk, dv, apart);                           \
+    }                                                                                                                     \
+    if (le == cudaSuccess && taps > 1)                                                                                    \
+        le = launch_kernel(conv_state_kernel<T>, dim3(n_entries, gy), dim3(128), 0, s, xt + c_off, x_stride, state,       \
+                           state_stride, cu_rows, slot_ids, C, taps)
     if (act_dtype == 0) {
-        if (smem > 48 * 1024)
-            cudaFuncSetAttribute(delta_prepare_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        le = launch_kernel(delta_prepare_kernel<float>, dim3(n_rows), dim3(threads), smem, s, (const float*)x, x_stride,
-                           c_off, b_off, a_off, w, taps, (const float*)state, state_stride, row_entry, cu_rows,
-                           slot_ids, a_log, dt_bias, (float2*)kq, vo, (float4*)dd, n_rows, G, H, dk, dv, apart);
-        if (le == cudaSuccess && taps > 1)
-            le = launch_kernel(conv_state_kernel<float>, dim3(n_entries, gy), dim3(128), 0, s, (const float*)x + c_off,
-                               x_stride, state, state_stride, cu_rows, slot_ids, C, taps);
+        IB_PREP(float);
     } else if (act_dtype == 1) {
-        if (smem > 48 * 1024)
-            cudaFuncSetAttribute(delta_prepare_kernel<bf16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        le = launch_kernel(delta_prepare_kernel<bf16>, dim3(n_rows), dim3(threads), smem, s, (const bf16*)x, x_stride,
-                           c_off, b_off, a_off, w, taps, (const float*)state, state_stride, row_entry, cu_rows,
-                           slot_ids, a_log, dt_bias, (float2*)kq, vo, (float4*)dd, n_rows, G, H, dk, dv, apart);
-        if (le == cudaSuccess && taps > 1)
-            le = launch_kernel(conv_state_kernel<bf16>, dim3(n_entries, gy), dim3(128), 0, s, (const bf16*)x + c_off,
-                               x_stride, state, state_stride, cu_rows, slot_ids, C, taps);
+        IB_PREP(bf16);
     } else {
         return IB_ERR_UNSUPPORTED;
     }
+#undef IB_PREP
     if (le != cudaSuccess) return (int)le;
     IB_LAUNCH_CHECK();
     return IB_OK;

@@ -90,25 +90,38 @@ __device__ __forceinline__ void fetch_rows(float* dst, int pitch, const float* s
     }
 }
 
-// acc[i][j] += sum_k a[i * 4 rows on][k] b[j * 8 rows on][k] over ROWS: both operands by rows of k, `pitch` apart
-__device__ __forceinline__ void dot_tile(const float* a, const float* b, int pitch, float (&acc)[4][8]) {
+// Two products and sums at once: half the issue slots of fmaf, which leaves the loads between them room.
+__device__ __forceinline__ void pfma2(float2& c, float ax, float ay, float bx, float by) {
+    const float2 a = make_float2(ax, ay), b = make_float2(bx, by);
+    asm("fma.rn.f32x2 %0, %1, %2, %0;"
+        : "+l"(reinterpret_cast<unsigned long long&>(c))
+        : "l"(reinterpret_cast<const unsigned long long&>(a)), "l"(reinterpret_cast<const unsigned long long&>(b)));
+}
+
+// acc[i][j] = sum_k a[i * 4 rows on][k] b[j * 8 rows on][k] over ROWS: both operands by rows of k, `pitch` apart
+template <int M, int N>
+__device__ __forceinline__ void dot_tile(const float* a, const float* b, int pitch, float (&acc)[M][N]) {
+    float2 sum[M][N] = {};   // of the even and of the odd k
 #pragma unroll 2
     for (int k = 0; k < ROWS; k += 4) {
-        float4 u[4], v[8];
+        float4 u[M], v[N];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) u[i] = *reinterpret_cast<const float4*>(a + i * 4 * pitch + k);
+        for (int i = 0; i < M; ++i) u[i] = *reinterpret_cast<const float4*>(a + i * 4 * pitch + k);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) v[j] = *reinterpret_cast<const float4*>(b + j * 8 * pitch + k);
+        for (int j = 0; j < N; ++j) v[j] = *reinterpret_cast<const float4*>(b + j * 8 * pitch + k);
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
+        for (int i = 0; i < M; ++i)
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                acc[i][j] = fmaf(u[i].x, v[j].x, acc[i][j]);
-                acc[i][j] = fmaf(u[i].y, v[j].y, acc[i][j]);
-                acc[i][j] = fmaf(u[i].z, v[j].z, acc[i][j]);
-                acc[i][j] = fmaf(u[i].w, v[j].w, acc[i][j]);
-            }
+            for (int j = 0; j < N; ++j) pfma2(sum[i][j], u[i].x, u[i].y, v[j].x, v[j].y);
+#pragma unroll
+        for (int i = 0; i < M; ++i)
+#pragma unroll
+            for (int j = 0; j < N; ++j) pfma2(sum[i][j], u[i].z, u[i].w, v[j].z, v[j].w);
     }
+#pragma unroll
+    for (int i = 0; i < M; ++i)
+#pragma unroll
+        for (int j = 0; j < N; ++j) acc[i][j] = sum[i][j].x + sum[i][j].y;
 }
 
 constexpr int STATE_BYTES = 2 * L * PITCH * (int)sizeof(float);   // (C and B of the C.B product; B and x need less)
@@ -132,7 +145,7 @@ __global__ void __launch_bounds__(128) ssd_chunk_state_kernel(const SsdParams p)
         fetch_rows<ROWS>(bs, PITCH, src, 2 * ROWS, at.n);
         fetch_rows<ROWS>(cs, PITCH, src + ROWS, 2 * ROWS, at.n);
         cp_async_land();
-        float acc[4][8] = {};
+        float acc[4][8];
         dot_tile(cs + (warp * 16 + ly) * PITCH, bs + lx * PITCH, PITCH, acc);
         float* out = p.cb + ((size_t)g * p.chunks + blockIdx.x) * L * L;
 #pragma unroll
@@ -308,7 +321,7 @@ __global__ void __launch_bounds__(128) chunk_out_kernel(const SsdParams p) {
     }
     __syncthreads();
     // a thread: tokens warp * 16 + i * 4 + ly, columns (j / 4) * 32 + lx * 4 + j % 4 (row j * 8 + lx of `ss`)
-    float acc[4][8] = {};
+    float acc[4][8];
     dot_tile(cs + (warp * 16 + ly) * PITCH, ss + lx * PITCH, PITCH, acc);
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -402,20 +415,17 @@ __global__ void __launch_bounds__(128) delta_chunk_dots_kernel(const DeltaParams
     const float* src = p.o.bc + ((size_t)g * p.o.n_rows + at.row) * 2 * ROWS;
     float* ks = smem;
     float* qs = smem + L * PITCH;
+    const bool which = blockIdx.z == 1;   // q_t.k_s
     fetch_rows<ROWS>(ks, PITCH, src, 2 * ROWS, at.n);
-    fetch_rows<ROWS>(qs, PITCH, src + ROWS, 2 * ROWS, at.n);
+    if (which) fetch_rows<ROWS>(qs, PITCH, src + ROWS, 2 * ROWS, at.n);
     cp_async_land();
-    const size_t out = ((size_t)g * p.o.chunks + blockIdx.x) * L * L;
-#pragma unroll 1
-    for (int which = 0; which < 2; ++which) {
-        float acc[4][8] = {};
-        dot_tile((which ? qs : ks) + (warp * 16 + ly) * PITCH, ks + lx * PITCH, PITCH, acc);
-        float* dst = (which ? p.o.cb : p.kk) + out;
+    float acc[4][8];
+    dot_tile((which ? qs : ks) + (warp * 16 + ly) * PITCH, ks + lx * PITCH, PITCH, acc);
+    float* dst = (which ? p.o.cb : p.kk) + ((size_t)g * p.o.chunks + blockIdx.x) * L * L;
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < 4; ++i)
 #pragma unroll
-            for (int j = 0; j < 8; ++j) dst[(warp * 16 + i * 4 + ly) * L + lx + j * 8] = acc[i][j];
-    }
+        for (int j = 0; j < 8; ++j) dst[(warp * 16 + i * 4 + ly) * L + lx + j * 8] = acc[i][j];
 }
 
 constexpr int SOLVE_COLS = 256, SB = 16;   // columns of a CTA, tokens of a block
@@ -560,15 +570,16 @@ __global__ void __launch_bounds__(256) delta_chunk_walk_kernel(const DeltaParams
         if (tid < L) cp_async16(st + L * PITCH + L * ROWS + L * UP + tid * 4, d + (tid < m ? tid : 0) * 4, tid < m);
         asm volatile("cp.async.commit_group;\n" ::: "memory");
     };
-    // a thread's part of the state: rows r4 .. + 3 of columns pg * CPT .. + CPT - 1
-    constexpr int RG = ROWS / 4, CPT = WC * RG / 256;   // lanes a column, columns a thread
-    const int r4 = tid % RG * 4, pg = tid / RG;
-    float* state = p.o.state + (long long)p.o.slot_ids[e] * p.o.state_stride + ((size_t)head * P + p0 + pg * CPT) * ROWS + r4;
+    // a thread's part of the state: rows r4 .. + 3 of columns c0 .. + CPT - 1; a warp has 32 rows of 4 CPT columns, whose
+    // factors it reads in one access each
+    constexpr int CPT = WC * ROWS / 4 / 256;
+    const int r4 = warp % (ROWS / 32) * 32 + lane % 8 * 4, c0 = warp / (ROWS / 32) * 4 * CPT + lane / 8 * CPT;
+    float* state = p.o.state + (long long)p.o.slot_ids[e] * p.o.state_stride + ((size_t)head * P + p0 + c0) * ROWS + r4;
     float4 S[CPT];
 #pragma unroll
     for (int j = 0; j < CPT; ++j) {
         S[j] = __ldcg(reinterpret_cast<const float4*>(state + (size_t)j * ROWS));
-        *reinterpret_cast<float4*>(ss + (pg * CPT + j) * PITCH + r4) = S[j];
+        *reinterpret_cast<float4*>(ss + (c0 + j) * PITCH + r4) = S[j];
     }
     fetch(0);
     for (int c = 0; c < count; ++c) {
@@ -592,30 +603,12 @@ __global__ void __launch_bounds__(256) delta_chunk_walk_kernel(const DeltaParams
         if (lane == 31) rest = 1.f;
         const float w1 = rest, w0 = g1 * rest, all = __shfl_sync(0xffffffffu, after, 0);
         // the state before the chunk, for the results
-        float* carry = p.o.carry + (((size_t)head * p.o.chunks + chunk + c) * P + p0 + pg * CPT) * ROWS + r4;
+        float* carry = p.o.carry + (((size_t)head * p.o.chunks + chunk + c) * P + p0 + c0) * ROWS + r4;
 #pragma unroll
         for (int j = 0; j < CPT; ++j) __stcg(reinterpret_cast<float4*>(carry + (size_t)j * ROWS), S[j]);
         // u = U - W S0: a thread tokens warp * 8 + ly and 4 further on, columns lx + 8 j
-        float acc[2][4] = {};
-        const float* wt = st + (warp * 8 + ly) * PITCH;
-        const float* sp = ss + lx * PITCH;
-#pragma unroll 4
-        for (int k = 0; k < ROWS; k += 4) {
-            float4 a[2], b[4];
-#pragma unroll
-            for (int i = 0; i < 2; ++i) a[i] = *reinterpret_cast<const float4*>(wt + i * 4 * PITCH + k);
-#pragma unroll
-            for (int j = 0; j < 4; ++j) b[j] = *reinterpret_cast<const float4*>(sp + j * 8 * PITCH + k);
-#pragma unroll
-            for (int i = 0; i < 2; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    acc[i][j] = fmaf(a[i].x, b[j].x, acc[i][j]);
-                    acc[i][j] = fmaf(a[i].y, b[j].y, acc[i][j]);
-                    acc[i][j] = fmaf(a[i].z, b[j].z, acc[i][j]);
-                    acc[i][j] = fmaf(a[i].w, b[j].w, acc[i][j]);
-                }
-        }
+        float acc[2][4];
+        dot_tile(st + (warp * 8 + ly) * PITCH, ss + lx * PITCH, PITCH, acc);
         float* ug = p.u + ((size_t)head * p.o.n_rows + first + c * L) * P + p0;
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
@@ -636,17 +629,18 @@ __global__ void __launch_bounds__(256) delta_chunk_walk_kernel(const DeltaParams
 #pragma unroll 8
         for (int t = 0; t < L; ++t) {
             const float4 k = *reinterpret_cast<const float4*>(kc + t * ROWS + r4);
+            float v[CPT];
+            if (CPT == 4) *reinterpret_cast<float4*>(v) = *reinterpret_cast<const float4*>(us + t * UP + c0);
+            else *reinterpret_cast<float2*>(v) = *reinterpret_cast<const float2*>(us + t * UP + c0);
 #pragma unroll
             for (int j = 0; j < CPT; ++j) {
-                const float v = us[t * UP + pg * CPT + j];
-                S[j].x = fmaf(k.x, v, S[j].x);
-                S[j].y = fmaf(k.y, v, S[j].y);
-                S[j].z = fmaf(k.z, v, S[j].z);
-                S[j].w = fmaf(k.w, v, S[j].w);
+                float2* Sj = reinterpret_cast<float2*>(&S[j]);
+                Sj[0] = pfma(v[j], make_float2(k.x, k.y), Sj[0]);
+                Sj[1] = pfma(v[j], make_float2(k.z, k.w), Sj[1]);
             }
         }
 #pragma unroll
-        for (int j = 0; j < CPT; ++j) *reinterpret_cast<float4*>(ss + (pg * CPT + j) * PITCH + r4) = S[j];
+        for (int j = 0; j < CPT; ++j) *reinterpret_cast<float4*>(ss + (c0 + j) * PITCH + r4) = S[j];
     }
 #pragma unroll
     for (int j = 0; j < CPT; ++j) *reinterpret_cast<float4*>(state + (size_t)j * ROWS) = S[j];
@@ -740,7 +734,7 @@ IB_EXPORT int ib_delta_chunk(const float* v, const void* kq, const void* dd, int
         attr_done = true;
     }
     cudaStream_t s = (cudaStream_t)stream;
-    cudaError_t le = launch_kernel_in_order(delta_chunk_dots_kernel, dim3(chunks, groups), dim3(128), (size_t)STATE_BYTES, s, p);
+    cudaError_t le = launch_kernel_in_order(delta_chunk_dots_kernel, dim3(chunks, groups, 2), dim3(128), (size_t)STATE_BYTES, s, p);
     if (le == cudaSuccess)
         le = launch_kernel(delta_chunk_solve_kernel, dim3(chunks, heads, (ROWS + P + SOLVE_COLS - 1) / SOLVE_COLS), dim3(128),
                            (size_t)SOLVE_BYTES, s, p);
