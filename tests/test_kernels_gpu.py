@@ -42,6 +42,50 @@ def test_embed(dtype):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("H,shift", [(8, 0), (1032, 0), (4096, 0), (4096, 1)])
+def test_embed_in_eights(dtype, H, shift):
+    """Rows of eights, and a table that begins off a 16-byte boundary, which goes by single elements: the same values."""
+    c = core()
+    flat = torch.randn(9 * H + shift).to(dtype).to(DEV)
+    table = flat[shift:].view(9, H)
+    ids = torch.tensor([8, 0, 4, 9, -1], dtype=torch.int32, device=DEV)
+    out = torch.empty(5, H, device=DEV)
+    err = c.new_error_word(DEV)
+    c.embed(ids, table, out, err, 1.5)
+    assert torch.equal(out[:3], table[[8, 0, 4]].float() * 1.5) and err.item() == c.FLAG_BAD_TOKEN
+    assert not out[3:].any()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("q_rank,kv_rank,rot_dim,rotary", [(1536, 512, 64, 64), (0, 32, 8, 4), (132, 128, 20, 20)])
+def test_latent_prepare_in_fours(dtype, q_rank, kv_rank, rot_dim, rotary):
+    """Against rows an odd number of elements apart, which go by single elements: sums in another order, so a result may
+    round to its neighbour (2^-8 of it in bf16; some 2^-24 of the norm, three roundings, in float32)."""
+    c = core()
+    g = torch.Generator(device=DEV).manual_seed(kv_rank)
+    rnd = lambda *s: torch.randn(*s, generator=g, device=DEV).to(dtype)  # noqa: E731
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)  # noqa: E731
+    N, width = 5, q_rank + kv_rank + rot_dim
+    x, wq, wkv = rnd(N, width), rnd(q_rank), rnd(kv_rank)
+    freq = torch.rand(rotary // 2, generator=g, device=DEV)
+    got = []
+    for stride in (width + 4, width + 5):
+        rows = torch.zeros(N, stride, dtype=dtype, device=DEV)
+        rows[:, :width] = x
+        cq = torch.zeros(N, q_rank, dtype=dtype, device=DEV)
+        pool = torch.zeros(3, 1, 4, kv_rank + rot_dim, dtype=dtype, device=DEV)
+        err = c.new_error_word(DEV)
+        c.latent_prepare(rows[:, :width], q_rank, kv_rank, rot_dim, rotary, wq if q_rank else None, wkv, 1e-5, freq,
+                         i32([0, 5, 2, 7, 9]), i32([0, 0, 1, 1, 1]), i32([[2, 0], [1, -1]]), cq if q_rank else None, pool, err,
+                         adjacent=rotary < rot_dim, magnitude=1.25)
+        assert err.item() == c.FLAG_BAD_PAGE  # (positions 7 and 9 of the second request have no page)
+        got.append((cq.double(), pool.double()))
+    bound = 2.0 ** -8 if dtype == torch.bfloat16 else 1e-6
+    for a, b in zip(*got):
+        assert bool(((a - b).abs() <= bound * b.abs() + 1e-9).all())
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("H", [50, 64, 333, 4096, 9000])
 def test_add_rmsnorm(dtype, H):
     c = core()
