@@ -189,9 +189,18 @@ struct GemmParams {
     float act_limit, act_alpha;  // of the clamped activation
     int swiglu;           // gate_times' code: W rows are 64 gates then their 64 ups per tile; out is [T, N/2]
     int alone;            // act_alone's code, for products without a gate
+    // with the gated epilogue:
+    int limit_col;        // from this output column on the limit is act_limit2 (4 | limit_col)
+    float act_limit2;
+    const float* scale;   // optional [T, n_scales]: out[t, c] *= scale[t, c / cols_per_scale] (4 | cols_per_scale)
+    int n_scales, cols_per_scale;
 };
 
-template <int BN>
+// GATED is a kernel of its own: what the gates need, inlined beside the plain epilogue, costs every launch its fetch from
+// the instruction cache (2 us of a product's 8 to 12 with one token).  The tile goes through shared memory and four warps
+// walk over it in a loop of a few instructions, eight values a thread and round: 64 tokens of 28,672 x 4,096 weights
+// 52.6 -> 44.4 us against two warps with every value's gate unrolled.
+template <int BN, bool GATED>
 __global__ void __launch_bounds__(NUM_THREADS, 2)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w,
                     const __grid_constant__ CUtensorMap map_x, const GemmParams p) {
@@ -317,43 +326,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w,
         tc_fence_after();
         const unsigned taddr = tmem_base + ((unsigned)(quad * 32) << 16);
         const int t0 = t_tile * BN;
-        if (p.swiglu) {
-            // Rows 0..63 of the tile are gates, rows 64..127 their ups (splits == 1).
-            // The up lanes park their values in shared memory (the stages are free:
-            // every MMA has completed), the gate lanes fetch them and store
-            // silu(gate) * up.  out is [T, N / 2], column n_tile * 64 + row.
-            float* xch = reinterpret_cast<float*>(smem);  // [BN][64]
-            if (row >= 64 && ok && n_kblocks > 0) {
-#pragma unroll
-                for (int c = 0; c < BN; c += 16) {
-                    unsigned v[16];
-                    tmem_ld16(taddr + c, v);
-                    tmem_ld_wait();
-#pragma unroll
-                    for (int j = 0; j < 16; ++j) xch[(c + j) * 64 + (row - 64)] = __uint_as_float(v[j]);
-                }
-            }
-            epilogue_bar_sync();
-            const int col = n_tile * 64 + row;
-            if (row < 64 && ok && n_kblocks > 0 && col < p.N / 2) {
-#pragma unroll
-                for (int c = 0; c < BN; c += 16) {
-                    unsigned v[16];
-                    tmem_ld16(taddr + c, v);
-                    tmem_ld_wait();
-#pragma unroll
-                    for (int j = 0; j < 16; ++j) {
-                        const int t = t0 + c + j;
-                        if (t < p.T) {
-                            const float g = __uint_as_float(v[j]);
-                            const float u = xch[(c + j) * 64 + row];
-                            ((bf16*)p.out)[(size_t)t * p.ldo + col] =
-                                __float2bfloat16_rn(gate_times(g, u, p.swiglu, p.act_limit, p.act_alpha));
-                        }
-                    }
-                }
-            }
-        } else if (p.splits == 1) {
+        if (!GATED && p.splits == 1) {
             if (ok && n_kblocks > 0) {
 #pragma unroll
                 for (int c = 0; c < BN; c += 16) {
@@ -372,7 +345,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w,
                 }
             }
         } else {
-            // my slice's partial tile into my own shared memory: [col][row].
+            // my slice's partial tile (with gates, the tile) into my own shared memory: [col][row].
             // The pipeline stages are free by now (every MMA has completed).
             float* red = reinterpret_cast<float*>(smem);
 #pragma unroll
@@ -392,7 +365,64 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w,
         tc_fence_before();
     }
     __syncwarp();  // the elected lanes are back with their warps before the aligned barriers
-    if (p.splits > 1) {
+    if (GATED) {
+        // Rows 0..63 of the tile are gates, rows 64..127 their ups; out is [T, N / 2], column n_tile * 64 + row.  Sixteen
+        // lanes a token: four gates and their ups a lane, two tokens a warp.
+        if (p.splits > 1) cluster_sync_all();  // every slice's partial tile is in place
+        if (warp >= 2) {
+            if (p.splits == 1) epilogue_bar_sync();
+            const int t0 = t_tile * BN;
+            const float* red = reinterpret_cast<const float*>(smem);
+            const int cols_per = (BN + p.splits - 1) / p.splits;
+            const int c_begin = p.splits > 1 ? (int)cluster_ctarank() * cols_per : 0;
+            const int c_end = min(min(BN, c_begin + cols_per), p.T - t0);
+            const int r4 = (lane & 15) * 4, col = n_tile * 64 + r4;
+            const bool vec_ok = p.ldo % 4 == 0 && ((uintptr_t)p.out & 7) == 0;
+            const float limit = col < p.limit_col ? p.act_limit : p.act_limit2;
+#pragma unroll 1
+            for (int c = c_begin + 2 * (warp & 3) + (lane >> 4); c < c_end; c += 8) {
+                const float* at = red + c * BM + r4;
+                float4 g = make_float4(0.f, 0.f, 0.f, 0.f), u = g;
+                if (p.splits == 1) {
+                    g = *reinterpret_cast<const float4*>(at);
+                    u = *reinterpret_cast<const float4*>(at + 64);
+                } else {
+                    float4 part[2][8];
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) {
+                        part[0][k] = part[1][k] = make_float4(0.f, 0.f, 0.f, 0.f);
+                        if (k < p.splits) {
+                            part[0][k] = ld_peer_smem4(at, (unsigned)k);
+                            part[1][k] = ld_peer_smem4(at + 64, (unsigned)k);
+                        }
+                    }
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) {  // in slice order
+                        g.x += part[0][k].x; g.y += part[0][k].y; g.z += part[0][k].z; g.w += part[0][k].w;
+                        u.x += part[1][k].x; u.y += part[1][k].y; u.z += part[1][k].z; u.w += part[1][k].w;
+                    }
+                }
+                const int t = t0 + c;
+                const float sc = p.scale ? __ldcg(p.scale + (size_t)t * p.n_scales + col / p.cols_per_scale) : 1.f;
+                float v[4] = {g.x, g.y, g.z, g.w};
+                const float w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+                for (int k = 0; k < 4; ++k) v[k] = gate_times(v[k], w[k], p.swiglu, limit, p.act_alpha) * sc;
+                bf16* dst = (bf16*)p.out + (size_t)t * p.ldo + col;
+                if (vec_ok) {
+                    __nv_bfloat162 lo = __floats2bfloat162_rn(v[0], v[1]), hi = __floats2bfloat162_rn(v[2], v[3]);
+                    uint2 packed;
+                    packed.x = *reinterpret_cast<unsigned*>(&lo);
+                    packed.y = *reinterpret_cast<unsigned*>(&hi);
+                    *reinterpret_cast<uint2*>(dst) = packed;
+                } else {
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) dst[k] = __float2bfloat16_rn(v[k]);
+                }
+            }
+        }
+        if (p.splits > 1) cluster_sync_all();  // nobody leaves while a peer may still read its tile
+    } else if (p.splits > 1) {
         cluster_sync_all();  // every slice's partial tile is in place
         if (warp >= 2) {
             const int quad = warp & 3;
@@ -515,15 +545,14 @@ static int make_map(CUtensorMap* map, const void* base, long long rows, long lon
     return r == CUDA_SUCCESS ? IB_OK : IB_ERR_BAD_ARG;
 }
 
-template <int BN>
+template <int BN, bool GATED>
 static int launch(const CUtensorMap& mw, const CUtensorMap& mx, const GemmParams& p, int t_tiles,
                   int n_tiles, cudaStream_t s) {
     constexpr int smem = num_stages(BN) * stage_bytes(BN) + 1024;
     static_assert(BN * BM * 4 <= num_stages(BN) * stage_bytes(BN), "partial tile must fit the stages");
-    if (p.swiglu && BN > 64) return IB_ERR_UNSUPPORTED;  // the exchange buffer is sized for small token tiles
     static bool attr_done = false;
     if (!attr_done) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_kernel<BN>,
+        cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_kernel<BN, GATED>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (e != cudaSuccess) return (int)e;
         attr_done = true;
@@ -542,7 +571,7 @@ static int launch(const CUtensorMap& mw, const CUtensorMap& mx, const GemmParams
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = pdl_flag() ? 2 : 1;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_tcgen05_kernel<BN>, mw, mx, p);
+    cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_tcgen05_kernel<BN, GATED>, mw, mx, p);
     if (e != cudaSuccess) return (int)e;
     IB_LAUNCH_CHECK();
     return IB_OK;
@@ -563,15 +592,20 @@ IB_EXPORT int ib_gemm_tc_token_tile(int T) {
 // ldx, ldw, ldo: row strides in elements.  `splits` (1..8) cuts K over the
 // CTAs of a cluster.  swiglu > 0 (gate_times' code; act_limit and act_alpha are those of code 3): W holds, per
 // 128 rows, 64 gate rows followed by their 64 up rows; out is [T, N / 2] bf16 with
-// out[t, 64 b + r] = gate_times(x . W[128 b + r], x . W[128 b + 64 + r]); K is not split.
+// out[t, 64 b + r] = gate_times(x . W[128 b + r], x . W[128 b + 64 + r]); with `scale` (float32
+// [T, (N/2) / cols_per_scale]; cols_per_scale a multiple of 16 that divides N/2) times scale[t, column / cols_per_scale];
+// from output column `limit_col` on (a multiple of 16; N for none) the clamped activation's limit is act_limit2.
 // swiglu < 0: no gates; -swiglu is act_alone's code, applied to every value of the product.
 IB_EXPORT int ib_gemm_tc(const void* x, int ldx, const void* w, int ldw, void* out, int ldo,
                          int out_f32, int T, int N, int K, int splits, int swiglu, unsigned* err,
-                         void* stream, float act_limit, float act_alpha) {
+                         void* stream, float act_limit, float act_alpha, const float* scale,
+                         int cols_per_scale, int limit_col, float act_limit2) {
     const int alone = swiglu < 0 ? -swiglu : 0;
     if (alone) swiglu = 0;
-    if (alone > 1) return IB_ERR_BAD_ARG;
+    if (alone > 1 || limit_col < 0 || limit_col % 16) return IB_ERR_BAD_ARG;
     if (T <= 0 || N <= 0) return IB_OK;
+    if (scale && (swiglu <= 0 || cols_per_scale <= 0 || cols_per_scale % 16 || (N / 2) % cols_per_scale))
+        return IB_ERR_BAD_ARG;
     if (!x || !w || !out || !err || K <= 0) return IB_ERR_BAD_ARG;
     // TMA: 16-byte aligned bases and row strides
     if (((uintptr_t)x & 15) || ((uintptr_t)w & 15) || (ldx % 8) || (ldw % 8) || ldx < K || ldw < K ||
@@ -583,7 +617,6 @@ IB_EXPORT int ib_gemm_tc(const void* x, int ldx, const void* w, int ldw, void* o
     const int kblocks = (K + BK - 1) / BK;
     int sp = splits < 1 ? 1 : (splits > 8 ? 8 : splits);  // a cluster holds at most 8 CTAs
     if (sp > kblocks) sp = kblocks;
-    if (swiglu) sp = 1;
     if (n_tiles > 65535) return IB_ERR_TOO_LARGE;
     GemmParams p;
     p.out = out;
@@ -599,17 +632,30 @@ IB_EXPORT int ib_gemm_tc(const void* x, int ldx, const void* w, int ldw, void* o
     p.alone = alone;
     p.act_limit = act_limit;
     p.act_alpha = act_alpha;
+    p.limit_col = limit_col;
+    p.act_limit2 = act_limit2;
+    p.scale = scale;
+    p.cols_per_scale = scale ? cols_per_scale : 1;
+    p.n_scales = scale ? (N / 2) / cols_per_scale : 0;
     CUtensorMap mw, mx;
     int rc = make_map(&mw, w, N, K, ldw, BM);
     if (rc != IB_OK) return rc;
     rc = make_map(&mx, x, T, K, ldx, bn);
     if (rc != IB_OK) return rc;
     cudaStream_t s = (cudaStream_t)stream;
+    if (swiglu) {
+        switch (bn) {
+            case 16: return launch<16, true>(mw, mx, p, t_tiles, n_tiles, s);
+            case 32: return launch<32, true>(mw, mx, p, t_tiles, n_tiles, s);
+            case 64: return launch<64, true>(mw, mx, p, t_tiles, n_tiles, s);
+            default: return IB_ERR_UNSUPPORTED;  // (prompts run on pairs of SMs)
+        }
+    }
     switch (bn) {
-        case 16: return launch<16>(mw, mx, p, t_tiles, n_tiles, s);
-        case 32: return launch<32>(mw, mx, p, t_tiles, n_tiles, s);
-        case 64: return launch<64>(mw, mx, p, t_tiles, n_tiles, s);
-        case 128: return launch<128>(mw, mx, p, t_tiles, n_tiles, s);
-        default: return launch<256>(mw, mx, p, t_tiles, n_tiles, s);
+        case 16: return launch<16, false>(mw, mx, p, t_tiles, n_tiles, s);
+        case 32: return launch<32, false>(mw, mx, p, t_tiles, n_tiles, s);
+        case 64: return launch<64, false>(mw, mx, p, t_tiles, n_tiles, s);
+        case 128: return launch<128, false>(mw, mx, p, t_tiles, n_tiles, s);
+        default: return launch<256, false>(mw, mx, p, t_tiles, n_tiles, s);
     }
 }

@@ -64,7 +64,8 @@ def lib() -> ctypes.CDLL:
     if _lib is None:
         l = load_module("gemm_tc", ["gemm_tcgen05.cu"])
         l.ib_gemm_tc.argtypes = [_c_void_p, _c_int, _c_void_p, _c_int, _c_void_p, _c_int, _c_int,
-                                 _c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p, _c_void_p, _c_float, _c_float]
+                                 _c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p, _c_void_p, _c_float, _c_float,
+                                 _c_void_p, _c_int, _c_int, _c_float]
         l.ib_gemm_tc.restype = _c_int
         l.ib_gemm_tc_token_tile.argtypes = [_c_int]
         l.ib_gemm_tc_token_tile.restype = _c_int
@@ -121,7 +122,9 @@ def choose_splits(T: int, N: int, K: int, sm_count: int) -> int:
     largest slice count is taken whose grid still fits one round with some room
     for the placement of whole clusters (measured on the 8B shapes: 48 tiles x 5
     and 32 tiles x 8 run in one round, 48 x 6 does not), each slice keeping at
-    least four blocks of 64 k."""
+    least four blocks of 64 k.  The gated products are cut by the same rule: 44 tiles
+    of K = 1,024 in one slice 6.0 us with one token and 10.2 with 64, in four 5.0 and
+    6.9; 128 tiles of K = 3,072 20.7 and 29.7, in two 19.7 and 24.9."""
     bn = lib().ib_gemm_tc_token_tile(T)
     tiles = -(-N // BM) * -(-T // bn)
     kblocks = -(-K // BK)
@@ -144,22 +147,36 @@ def eligible(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> bool:
 
 def gemm_tc(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, splits: Optional[int] = None,
             err: Optional[torch.Tensor] = None, swiglu: bool = False, act_limit: float = 0.0,
-            act_alpha: float = 0.0) -> None:
+            act_alpha: float = 0.0, scale: Optional[torch.Tensor] = None, cols_per_scale: int = 0,
+            limit_col: Optional[int] = None, act_limit2: float = 0.0) -> None:
     """Runs the tcgen05 kernel; raises KernelError if the operands do not fit it.
     ``swiglu``: ``w`` holds, per 128 rows, 64 gate rows then their 64 up rows, and
     ``out`` [T, N/2] receives silu(gate) * up (at most 64 tokens); a code of ``GATE_CODES`` names another
     activation (``act_limit`` and ``act_alpha`` are the clamped one's), a (negative) code of ``ALONE_CODES`` one
-    that is applied to every value of a product without a gate."""
+    that is applied to every value of a product without a gate.  ``scale`` and ``limit_col`` as in ``gemm_pair``."""
     core.require_cuda(x, w, out)
     T, K = x.shape
     N = w.shape[0]
+    if scale is not None:
+        _check_scale("gemm_tc", scale, cols_per_scale, swiglu, T, N)
     if splits is None:
         splits = choose_splits(T, N, K, POLICY["sm_count"])
     code = lib().ib_gemm_tc(x.data_ptr(), x.stride(0), w.data_ptr(), w.stride(0), out.data_ptr(),
                             out.stride(0), 1 if out.dtype == torch.float32 else 0, T, N, K, splits,
                             int(swiglu), (err if err is not None else _error_word(x.device)).data_ptr(),
-                            core.stream_ptr(x), float(act_limit), float(act_alpha))
+                            core.stream_ptr(x), float(act_limit), float(act_alpha),
+                            scale.data_ptr() if scale is not None else None, int(cols_per_scale),
+                            -(-N // 16) * 16 if limit_col is None else int(limit_col), float(act_limit2))
     core.check(code, "gemm_tc")
+
+
+def _check_scale(name: str, scale: torch.Tensor, cols_per_scale: int, swiglu, T: int, N: int) -> None:
+    if not swiglu or cols_per_scale <= 0 or cols_per_scale % 16 or (N // 2) % cols_per_scale:
+        raise KernelError(f"{name}: a scale goes with the gated epilogue and runs of a multiple of 16 columns")
+    if scale.dtype != torch.float32 or not scale.is_contiguous() \
+            or tuple(scale.shape) != (T, (N // 2) // cols_per_scale):
+        raise KernelError(f"{name}: scale must be contiguous float32 [{T}, {(N // 2) // cols_per_scale}]")
+    core.require_cuda(scale)
 
 
 @functools.lru_cache(maxsize=256)
@@ -226,12 +243,7 @@ def gemm_pair(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor,
     T, K = x.shape
     N = w.shape[0]
     if scale is not None:
-        if not swiglu or cols_per_scale <= 0 or cols_per_scale % 16 or (N // 2) % cols_per_scale:
-            raise KernelError("gemm_pair: a scale goes with the gated epilogue and runs of a multiple of 16 columns")
-        if scale.dtype != torch.float32 or not scale.is_contiguous() \
-                or tuple(scale.shape) != (T, (N // 2) // cols_per_scale):
-            raise KernelError(f"gemm_pair: scale must be contiguous float32 [{T}, {(N // 2) // cols_per_scale}]")
-        core.require_cuda(scale)
+        _check_scale("gemm_pair", scale, cols_per_scale, swiglu, T, N)
     bn_a, cols_a, bn_b = tiling or choose_pair_tiling(T, N, POLICY["sm_count"], int(swiglu) > 0)
     code = pair_lib().ib_gemm_pair_scaled(x.data_ptr(), x.stride(0), w.data_ptr(), w.stride(0), out.data_ptr(),
                                           out.stride(0), T, N, K, int(swiglu), bn_a, cols_a, bn_b,
@@ -316,8 +328,8 @@ def swiglu_route(x: torch.Tensor, w_interleaved: torch.Tensor, out: torch.Tensor
     """The gate/up product with SiLU(gate) * up applied in its epilogue, when
     the policy and the operands allow; ``out`` is [T, I].  Up to 64 tokens go to
     the kernel that streams the weights once (decode), prompts to the kernel on
-    pairs of SMs when their length suits its tiles (``pair_suits``).  With
-    ``scale`` or a second limit (see ``gemm_pair``) only the latter is offered."""
+    pairs of SMs when their length suits its tiles (``pair_suits``).  ``scale``
+    and the second limit: see ``gemm_pair``."""
     mode = POLICY["mode"]
     if mode in ("none", "cublas", "library") or activation not in GATE_CODES:
         return False
@@ -332,9 +344,8 @@ def swiglu_route(x: torch.Tensor, w_interleaved: torch.Tensor, out: torch.Tensor
     if limit_col is not None and limit_col % 16:
         return False
     if T <= min(POLICY["max_tokens"], 64):
-        if scale is not None or limit_col is not None:
-            return False
-        gemm_tc(x, w_interleaved, out, splits=1, swiglu=code, err=err, act_limit=act_limit, act_alpha=act_alpha)
+        gemm_tc(x, w_interleaved, out, swiglu=code, err=err, act_limit=act_limit, act_alpha=act_alpha, scale=scale,
+                cols_per_scale=cols_per_scale, limit_col=limit_col, act_limit2=act_limit2)
         return True
     if pair_suits(T, fused_activation=True):
         gemm_pair(x, w_interleaved, out, swiglu=code, err=err, scale=scale, cols_per_scale=cols_per_scale,

@@ -9,7 +9,7 @@ token, and the dense row ``gate[N, experts]`` that is 0 for experts not chosen),
 so a recorded step replays.  The experts' gate/up weights are kept as one
 stacked matrix ``[experts * 2 ff, hidden]`` and their down weights side by side
 as ``[hidden, experts * ff]``; one product gives every expert's gate and up
-values, the activation kernel multiplies each expert's run of ``ff`` outputs by
+values, the activation (in that product's epilogue where it can be) multiplies each expert's run of ``ff`` outputs by
 the token's weight for that expert (0 where it was not chosen), and the down
 product sums over all experts at once: ``sum_e Wd_e (w_e a_e)`` is one product
 with the concatenated vector.  What a token did not choose is multiplied by an exact 0.
@@ -248,7 +248,7 @@ class MixtureOfExperts(FeedForward):
         limit_col = self.experts * self.expert_size if self.shared_runs and self.shared["limit"] != self.limit else None
         limit2 = self.shared["limit"] if limit_col is not None else 0.0
         if self.block == 64 and x.dtype == torch.bfloat16 and self.gate_up.weight.dtype == torch.bfloat16:
-            # prompts: activation and the router's weights in the product's epilogue
+            # activation and the router's weights in the product's epilogue
             fused = gemm_tc.swiglu_route(x, self.gate_up.weight, act, self.gate_up.err, activation=self.activation,
                                          scale=gate, cols_per_scale=self.expert_size, act_limit=self.limit,
                                          act_alpha=self.alpha, limit_col=limit_col, act_limit2=limit2)

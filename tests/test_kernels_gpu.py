@@ -597,6 +597,40 @@ def test_gemm_tcgen05_with_swiglu_epilogue(T, I, K):
 
 
 
+@pytest.mark.parametrize("T, experts, ff, K", [(1, 4, 64, 1024), (8, 16, 32, 2048), (33, 3, 128, 520), (64, 8, 16, 1024)])
+@pytest.mark.parametrize("splits", [None, 1, 2, 8])
+@pytest.mark.parametrize("act", ["silu", "clamped_swish"])
+def test_gemm_tcgen05_gated_epilogue_of_slices_with_scales(T, experts, ff, K, splits, act):
+    """The gated epilogue behind slices of K, with a weight per token and run of columns and a second limit, against 64
+    bits: an output rounds to bfloat16 once (2^-8 of itself, half of that at most); the 32-bit sums of K terms stay far
+    below (K 2^-24 of the sum of their sizes)."""
+    from infernum_b200.ops import gemm_tc
+    I = experts * ff
+    g = torch.Generator().manual_seed(I + T)
+    x = torch.randn(T, K, generator=g).to(torch.bfloat16)
+    wg = (torch.randn(I, K, generator=g) * 0.05).to(torch.bfloat16)
+    wu = (torch.randn(I, K, generator=g) * 0.05).to(torch.bfloat16)
+    w = torch.stack([wg.view(I // 64, 64, K), wu.view(I // 64, 64, K)], dim=1).reshape(2 * I, K).contiguous().to(DEV)
+    scale = torch.rand(T, experts, generator=g) * 2.0
+    scale[torch.rand(T, experts, generator=g) < 0.4] = 0.0
+    wide = torch.full((T + 1, I + 8), 7.0, dtype=torch.bfloat16, device=DEV)
+    gemm_tc.gemm_tc(x.to(DEV), w, wide[:T, :I], splits=splits, swiglu=gemm_tc.GATE_CODES[act], act_limit=0.8, act_alpha=1.5,
+                    scale=scale.to(DEV), cols_per_scale=ff, limit_col=I // 2, act_limit2=0.3)
+    assert gemm_tc.error_flags(DEV) == 0
+    gate, up = x.double() @ wg.double().T, x.double() @ wu.double().T
+    if act == "silu":
+        want = gate / (1 + torch.exp(-gate)) * up
+    else:
+        limit = torch.where(torch.arange(I) < I // 2, 0.8, 0.3).double()
+        gate, up = torch.minimum(gate, limit), torch.maximum(torch.minimum(up, limit), -limit)
+        want = gate / (1 + torch.exp(-1.5 * gate)) * (up + 1)
+    want = want * scale.double().repeat_interleave(ff, dim=1)
+    got = wide[:T, :I].double().cpu()
+    assert bool(((got - want).abs() <= want.abs() * 2.0 ** -8 + 1e-4).all())
+    assert bool((got[scale.repeat_interleave(ff, dim=1) == 0] == 0).all())
+    assert bool((wide[T] == 7.0).all()) and bool((wide[:, I:] == 7.0).all())
+
+
 # --------------------------------------------------------------------------
 # the matrix product on pairs of SMs (prompts)
 # --------------------------------------------------------------------------
