@@ -21,7 +21,12 @@
 //   warps 2..9  epilogue (two warps per 32 TMEM lanes, half of the columns each):
 //               TMEM -> registers -> bf16 -> 32-byte pieces of a token's row of
 //               `out`; with `swiglu`, W holds per 128 rows 64 gate rows and their
-//               64 up rows, and silu(gate) * up is written to out[T, N/2]
+//               64 up rows, and silu(gate) * up is written to out[T, N/2] by
+//               sixteen warps (2..17), a quarter of the columns each: an
+//               exponential and a division per output, with eight warps and the
+//               activation chosen per value, took as long as the MMAs of a short K
+//               (1,019 tokens, 16,384 x 2,048 weights: 64 us against 48 for the
+//               plain product; 52 here)
 //
 // The weight rows are cut into columns of tiles in two regions: `cols_a` columns
 // of `bn_a` rows, then the rest in columns of `bn_b` rows.  The caller picks them
@@ -52,7 +57,8 @@ constexpr int STAGES = 6;
 constexpr int X_BYTES = BT * BK * 2;
 constexpr int STAGE_BYTES = X_BYTES + BNH * BK * 2;   // 32 KiB
 constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024;
-constexpr int NUM_THREADS = 320;   // producer, MMA and eight epilogue warps
+__host__ __device__ constexpr int epilogue_warps(bool swiglu) { return swiglu ? 16 : 8; }
+__host__ __device__ constexpr int num_threads(bool swiglu) { return 64 + 32 * epilogue_warps(swiglu); }   // producer, MMA, epilogue
 constexpr unsigned TMEM_COLS = 512;   // two accumulators of 256 columns
 constexpr unsigned PEER_BIT_MASK = 0xFEFFFFFFu;  // clears the CTA-rank bit of a shared::cluster address
 
@@ -141,6 +147,13 @@ __device__ __forceinline__ unsigned pack_bf16(float lo, float hi) {
     __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
     return *reinterpret_cast<unsigned*>(&v);
 }
+// Sixteen gates and their ups, the activation known when this is compiled.
+template <int ACT>
+__device__ __forceinline__ void gate_sixteen(const unsigned (&g)[16], const unsigned (&u)[16], float limit, float alpha, float sc,
+                                             float (&v)[16]) {
+#pragma unroll
+    for (int q = 0; q < 16; ++q) v[q] = gate_times(__uint_as_float(g[q]), __uint_as_float(u[q]), ACT, limit, alpha) * sc;
+}
 // Sixteen values of a token's row, bf16, at out[col .. col+16); `limit` ends the row.
 __device__ __forceinline__ void store16(bf16* row, int col, int limit, const float (&v)[16]) {
     if (col + 16 <= limit) {
@@ -211,7 +224,7 @@ __device__ __forceinline__ TilePlace locate(const Params& p, int tile) {
 }
 
 template <bool SWIGLU>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(num_threads(SWIGLU), 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
                  const __grid_constant__ CUtensorMap map_w2, const Params p) {
     extern __shared__ unsigned char smem_dyn[];
@@ -236,7 +249,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         }
         for (int b = 0; b < 2; ++b) {
             mbar_init(&acc_full[b], 1);
-            mbar_init(&acc_empty[b], 16);   // eight epilogue warps in each CTA
+            mbar_init(&acc_empty[b], 2 * epilogue_warps(SWIGLU));   // of both CTAs
         }
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
@@ -308,7 +321,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
     } else {
         // ---- epilogue: my 128 tokens x the tile's weight rows, half of them per warp ------------
         const int quad = warp & 3;
-        const int half = (warp - 2) >> 2;
+        const int half = (warp - 2) >> 2;   // of the columns; with gates, a quarter
         const int trow = quad * 32 + lane;   // token within my half = TMEM lane
         const int limit = SWIGLU ? p.N / 2 : p.N;
         bool ok = true;
@@ -328,23 +341,21 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
             if (SWIGLU) {
 #pragma unroll 1
                 for (int blk = 0; blk < bn / 128; ++blk) {
-#pragma unroll
-                    for (int c = half * 32; c < half * 32 + 32; c += 16) {
-                        unsigned g[16], u[16];
-                        tmem_ld16(taddr + blk * 128 + c, g);
-                        tmem_ld16(taddr + blk * 128 + 64 + c, u);
-                        tmem_ld_wait();
-                        float v[16];
-                        const int col = n0 / 2 + blk * 64 + c;
-                        // (sixteen columns share a scale; those past the row's end are not stored)
-                        const float sc = p.scale && live && col < limit
-                                             ? p.scale[(size_t)gt * p.n_scales + col / p.cols_per_scale] : 1.f;
-                        const float limit_here = col < p.limit_col ? p.act_limit : p.act_limit2;
-#pragma unroll
-                        for (int q = 0; q < 16; ++q)
-                            v[q] = gate_times(__uint_as_float(g[q]), __uint_as_float(u[q]), p.act, limit_here, p.act_alpha) * sc;
-                        if (live) store16(row, col, limit, v);
-                    }
+                    const int c = half * 16;
+                    unsigned g[16], u[16];
+                    tmem_ld16(taddr + blk * 128 + c, g);
+                    tmem_ld16(taddr + blk * 128 + 64 + c, u);
+                    tmem_ld_wait();
+                    float v[16];
+                    const int col = n0 / 2 + blk * 64 + c;
+                    // (sixteen columns share a scale; those past the row's end are not stored)
+                    const float sc = p.scale && live && col < limit
+                                         ? p.scale[(size_t)gt * p.n_scales + col / p.cols_per_scale] : 1.f;
+                    const float limit_here = col < p.limit_col ? p.act_limit : p.act_limit2;
+                    if (p.act == 2) gate_sixteen<2>(g, u, limit_here, p.act_alpha, sc, v);
+                    else if (p.act == 3) gate_sixteen<3>(g, u, limit_here, p.act_alpha, sc, v);
+                    else gate_sixteen<1>(g, u, limit_here, p.act_alpha, sc, v);
+                    if (live) store16(row, col, limit, v);
                 }
             } else {
                 const int split = ((bn >> 1) + 15) & ~15;
@@ -435,7 +446,7 @@ int launch_pair(const CUtensorMap& mx, const CUtensorMap& mw, const CUtensorMap&
     // idle lanes too, as they now do) or when the kernel let no successor begin
     // early, and stalled every time as it was.
     cudaError_t le = launch_kernel_in_order(gemm_pair_kernel<SWIGLU>, dim3((unsigned)(pairs * 2)),
-                                            dim3(NUM_THREADS), (size_t)SMEM_BYTES, stream, mx, mw, mw2, p);
+                                            dim3(num_threads(SWIGLU)), (size_t)SMEM_BYTES, stream, mx, mw, mw2, p);
     if (le != cudaSuccess) return (int)le;
     IB_LAUNCH_CHECK();
     return IB_OK;
