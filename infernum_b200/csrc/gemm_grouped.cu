@@ -170,6 +170,13 @@ struct TileWalk {
     }
 };
 
+// Eight gates and their ups, times sc, into sc; the activation is known when this is compiled.
+template <int ACT>
+__device__ __forceinline__ void gate_eight(const float (&g)[8], const float (&u)[8], float limit, float alpha, float (&sc)[8]) {
+#pragma unroll
+    for (int q = 0; q < 8; ++q) sc[q] = gate_times(g[q], u[q], ACT, limit, alpha) * sc[q];
+}
+
 template <bool GATED>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
 gemm_grouped_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
@@ -320,16 +327,22 @@ gemm_grouped_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
                     pair_sync(id);   // (two buffers: the one after next is written behind the next barrier)
                     const int col = row / 2 + (quad & 1) * 32 + lane;
                     bf16* out = (bf16*)p.out + col;
+                    float g[8], u[8], sc[8];
 #pragma unroll
                     for (int q = 0; q < 8; ++q) {
                         const int t = c + (up ? 8 + q : q);
                         const float mine = __uint_as_float(up ? v[8 + q] : v[q]), other = take[q * 32];
-                        if (t < at.count && row < p.N) {
-                            const size_t s = (size_t)(at.t0 + t);
-                            const float sc = p.scale ? __ldcg(p.scale + s * p.scale_stride) : 1.f;
-                            const float y = gate_times(up ? other : mine, up ? mine : other, p.act, p.act_limit, p.act_alpha);
-                            out[s * p.ldo] = __float2bfloat16_rn(y * sc);
-                        }
+                        g[q] = up ? other : mine;
+                        u[q] = up ? mine : other;
+                        sc[q] = p.scale && t < at.count ? __ldcg(p.scale + (size_t)(at.t0 + t) * p.scale_stride) : 1.f;
+                    }
+                    if (p.act == 2) gate_eight<2>(g, u, p.act_limit, p.act_alpha, sc);
+                    else if (p.act == 3) gate_eight<3>(g, u, p.act_limit, p.act_alpha, sc);
+                    else gate_eight<1>(g, u, p.act_limit, p.act_alpha, sc);
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) {
+                        const int t = c + (up ? 8 + q : q);
+                        if (t < at.count && row < p.N) out[(size_t)(at.t0 + t) * p.ldo] = __float2bfloat16_rn(sc[q]);
                     }
                 } else {
                     const int n = row + quad * 32 + lane;
