@@ -57,7 +57,7 @@ __device__ __forceinline__ void load8(const float* p, float (&v)[8]) {
 // The same for rows of eights: a CTA takes four rows by eight experts, its four warps every fourth run of 256 k, a lane
 // eight neighbouring k of a run.  An expert's values are converted once for four rows, a row's once for eight experts.
 // The lanes' sums meet by halves (31 shuffles for 32 logits) and the warps' in their order: a fixed order per logit,
-// whatever the batch.  2,048 rows of 4,096, 16 experts: 64 us a warp a (row, expert) -> 8 us; eight rows 11 -> 5 us.
+// whatever the batch.  2,048 rows of 4,096, 16 experts: 64 us a warp a (row, expert) -> 17 us; eight rows 11 -> 5 us.
 template <typename TX, typename TW>
 __global__ void __launch_bounds__(128) router_logits_tile_kernel(const TX* __restrict__ x, int ldx, const TW* __restrict__ w,
                                                                  int ldw, float* __restrict__ z, int n_rows, int E, int K) {

@@ -258,7 +258,7 @@ __device__ __forceinline__ void conv_silu_rows(const T* __restrict__ x, int x_st
 }
 
 // The same for prompts, whose scan goes in chunks (scan_chunk.cu): B and C of a token one after the other, bc [groups]
-// [rows][2][state].  2,048 rows of 2,304 channels 48 us -> 29 us.
+// [rows][2][state].  2,048 rows of 2,304 channels 48 us -> 18 us.
 template <typename T>
 __global__ void __launch_bounds__(128)
 ssd_prepare_rows_kernel(const T* __restrict__ x, int x_stride, const float* __restrict__ w, const float* __restrict__ b,

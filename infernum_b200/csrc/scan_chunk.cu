@@ -15,8 +15,8 @@
 // Decays are multiplied, never divided (a decay may be 0), and a token's result is made from what comes before it only:
 // what a later token brings is left out of the sum, not multiplied by zero.  A chunk's tokens are counted from the entry's
 // first row of the step: a prompt cut elsewhere rounds otherwise.
-// Bound by the multiply-adds (as many as token by token).  2,048 tokens, 32 heads of 128 x 64: 414 us by scan.cu, 36 + 28 +
-// 67 us here.
+// Bound by the multiply-adds (as many as token by token).  2,048 tokens, 32 heads of 128 x 64: 414 us by scan.cu, 36 + 30 +
+// 58 us here.
 #include "common.cuh"
 
 using namespace ib;
@@ -397,7 +397,8 @@ __global__ void __launch_bounds__(128) chunk_out_kernel(const SsdParams p) {
 //   chunk_out           every chunk at once: o
 // The walk is the only part that waits for the chunk before: 32 columns a CTA, so that there are four for a head of 128,
 // and the next chunk's operands come while one is worked on.  Two entries of 750 tokens, 16 heads of 128 x 128 on eight key
-// heads: 376 us by scan.cu, 20 + 32 + 113 + 51 us here.
+// heads: 376 us by scan.cu, 16 + 32 + 110 + 49 us here; the walk is bound by
+// what shared memory hands its small tiles (a 2 x 4 and a 4 x 4 of products a thread).
 struct DeltaParams {
     SsdParams o;           // what chunk_out reads: x is `u`, bc the k and q, cb the q_t.k_s, carry the states before the chunks
     const float* v;        // [heads][rows][P]

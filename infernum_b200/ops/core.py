@@ -558,8 +558,7 @@ def choose_f32_splits(max_rows_per_entry: int, n_rows: int, heads: int, kv_heads
                       sm_count: int) -> int:
     """How ``attention_f32`` spreads a step: 0 for tiles of 64 packed rows, or into how many slices (the CTAs of a
     cluster: 1, 2, 4 or 8) the keys of every row are cut.  Up to four rows an entry go row by row: a tile would be
-    filled to a quarter at most with four query heads a key/value head, and its keys walked by one CTA (eight decoded
-    rows of the 1B shape at 500 keys: 12 us by rows in eight slices).  Slices as long as the SMs hold CTAs to take
+    filled to a quarter at most with four query heads a key/value head, and its keys walked by one CTA.  Slices as long as the SMs hold CTAs to take
     them, and a slice keeps 64 keys."""
     if max_rows_per_entry > 4:
         return 0
