@@ -450,6 +450,7 @@ def test_scans_in_chunks_against_one_token_at_a_time(rule, heads, groups, rows, 
         return out, state
 
     assert scan.in_chunks(ctx, N, rows, cols, 0, tail + 8) and not scan.in_chunks(ctx, N, rows, cols, 0, tail + 9)
+    assert not scan.in_chunks(ctx, N, rows, cols, 0, tail + 8, heads=1 << 17)  # (more scratch than it may have)
     out, state = walk(x, tail + 8)
     ref, ref_state = walk(x, tail + 9)
     assert rel_err(out, ref) < 1e-5 and rel_err(state[:E, :size], ref_state[:E, :size]) < 1e-5
