@@ -263,7 +263,10 @@ attention_expanded_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
     const int rows_e = p.cu_rows[e + 1] - row0;
     const int pos0 = p.q_start[e];
     const int r_begin = ((int)gridDim.z - 1 - (int)blockIdx.z) * BM;
-    if (r_begin >= rows_e) return;
+    if (r_begin >= rows_e) {
+        pdl_wait();  // a CTA without rows too: this grid is not complete before the ones before it are
+        return;
+    }
     const int r_count = min(BM, rows_e - r_begin);
     const int kv_hi = pos0 + r_begin + r_count;             // keys of this row tile end here
     const int lo = p.window > 0 ? max(0, pos0 + r_begin - p.window + 1) : 0;   // the first row's first key

@@ -776,7 +776,10 @@ attention_split_tma_kernel(const Params p, const __grid_constant__ CUtensorMap m
     const int row0 = p.cu_rows[e];
     const int rows_e = p.cu_rows[e + 1] - row0;
     const int pos0 = p.q_start[e];
-    if (rows_e * gs > p.small_rows) return;  // tile mode takes this entry (the whole block leaves)
+    if (rows_e * gs > p.small_rows) {  // tile mode takes this entry (the whole block leaves)
+        pdl_wait();  // (this grid must not be complete before the ones before it are)
+        return;
+    }
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int gid = lane >> 2, tig = lane & 3;

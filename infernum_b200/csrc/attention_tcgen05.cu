@@ -305,14 +305,21 @@ __device__ __forceinline__ void attention_body(const CUtensorMap& map_q, const C
     const int rows_e = p.cu_rows[e + 1] - row0;
     const int pos0 = p.q_start[e];
     const int gs_split = G < 8 ? G : 8;
-    if (rows_e * gs_split <= p.small_rows) return;  // split mode takes this entry
+    // (CTAs without work wait too: this grid must not be complete before the ones before it are)
+    if (rows_e * gs_split <= p.small_rows) {  // split mode takes this entry
+        pdl_wait();
+        return;
+    }
     // The CTAs of a cluster (p.splits of them, consecutive in x) share one row tile
     // and take a slice of its key tiles each; they are merged at the end.
     const int S = SPLIT ? p.splits : 1;
     const int rank = (int)blockIdx.x % S;
     const int g = (int)blockIdx.x / S;
     const int r_begin = ((int)gridDim.z - 1 - (int)blockIdx.z) * rq;
-    if (r_begin >= rows_e) return;  // (the whole cluster leaves)
+    if (r_begin >= rows_e) {  // (the whole cluster leaves)
+        pdl_wait();
+        return;
+    }
     const int r_count = min(rq, rows_e - r_begin);
     const int kv_hi = pos0 + r_begin + r_count;
     const int all_tiles = (kv_hi + BN - 1) / BN;

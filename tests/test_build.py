@@ -1,5 +1,9 @@
 """The kernel build helper, as far as it goes without a GPU or a compiler run."""
+import os
+import re
 from concurrent.futures import ThreadPoolExecutor
+
+import pytest
 
 from infernum_b200.csrc import build
 
@@ -21,3 +25,14 @@ def test_module_hash_follows_sources_and_flags():
     assert a == build._hash_module(["elementwise.cu"], [], "nvcc")
     assert a != build._hash_module(["elementwise.cu"], ["-DIB_HD=64"], "nvcc")
     assert a != build._hash_module(["sampling.cu"], [], "nvcc")
+
+
+@pytest.mark.parametrize("name", sorted(f for f in os.listdir(build.CSRC_DIR) if f.endswith(".cu")))
+def test_no_thread_leaves_a_kernel_begun_early_without_waiting(name):
+    """Between a kernel's ``pdl_trigger()`` and its first ``pdl_wait()`` nothing returns: a grid whose CTAs all left there
+    would be complete before the grids before it are, and the kernel behind it would begin on what they still write."""
+    with open(os.path.join(build.CSRC_DIR, name), encoding="utf-8") as fh:
+        source = re.sub(r"//[^\n]*", "", fh.read())
+    for m in re.finditer(r"pdl_trigger\(\);", source):
+        before = source[m.end():].split("pdl_wait();")[0]
+        assert not re.search(r"\breturn;", before), f"{name}: line {source.count(chr(10), 0, m.start()) + 1}"
