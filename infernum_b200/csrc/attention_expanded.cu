@@ -510,6 +510,9 @@ gather_latents_kernel(const bf16* __restrict__ pool, bf16* __restrict__ out, con
     pdl_wait();
     const int at = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (at >= out_rows) return;
+    // (keys without a row would be zeros to the attention, which reads nothing behind the buffer: reported)
+    if (at == out_rows - 1 && lane == 0 && buffer_row(cu_rows, q_start, n_entries, window) > out_rows)
+        atomicOr(err, IB_FLAG_KEYS_LOST);
     int e = 0, left = at, key = -1;
     for (; e < n_entries; ++e) {
         const int rows = cu_rows[e + 1] - cu_rows[e];
@@ -571,7 +574,7 @@ IB_EXPORT int ib_attention_expanded_sizes() { return D * 1000000 + R * 1000 + VD
 
 // pool [num_pages][page_size][width] -> out [out_rows, width]: the keys of entry 0 that any of its rows sees (from the
 // multiple of 128 before the first row's window on), then those of entry 1, ...; rows behind the last key are left as they
-// are.  width a multiple of 8.
+// are, and keys that find no row set IB_FLAG_KEYS_LOST.  width a multiple of 8.
 IB_EXPORT int ib_gather_latents(const void* pool, void* out, const int* cu_rows, const int* q_start, const int* tables,
                                 int max_blocks, int n_entries, int page_size, int num_pages, int window, int width,
                                 int out_rows, unsigned* err, void* stream) {

@@ -22,6 +22,7 @@
 #define IB_FLAG_BAD_TOKEN 1u      // token id outside the vocabulary
 #define IB_FLAG_BAD_PAGE 2u       // block-table entry outside the pool
 #define IB_FLAG_WAIT_TIMEOUT 4u   // a bounded wait on a barrier gave up
+#define IB_FLAG_KEYS_LOST 8u      // a step's keys do not fit the buffer made for them
 // Which wait gave up: bit 8 + site is set beside IB_FLAG_WAIT_TIMEOUT.
 #define IB_SITE_GEMM_PRODUCER 0      // gemm_tcgen05: TMA producer
 #define IB_SITE_GEMM_MMA 1           // gemm_tcgen05: MMA issuer

@@ -203,7 +203,8 @@ class DecodeRunner:
                 # costs nothing, and a step whose portion ends its prompt needs no recording of its own)
                 logit_rows=view("logit", size + K),
                 block_tables=[tables[g] for g in range(G)],
-                # (for launch geometry: one portion at its longest, the entries behind it empty)
+                # (one way the rows may fall to the entries, for launch geometry: the first portion has all of
+                # them, the entries behind it none)
                 host_cu_rows=list(range(size + 1)) + [rows] * (K + 1), host_kv_len=[], max_rows_per_entry=portion,
                 max_kv_len=kv_cap, all_decode=False)
         n_sel = size + K   # rows whose token is selected

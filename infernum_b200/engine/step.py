@@ -53,9 +53,11 @@ class StepContext:
     belong to no request - while the host-side fields below stay as they were
     when the step was recorded.  Those describe the step's *shape* and serve
     for launch geometry only: ``n_rows``, ``n_entries``; ``max_rows_per_entry``
-    and ``max_kv_len``, upper bounds; ``host_cu_rows``, which in a recorded step
-    gives every entry the most rows it may have (not the rows it has);
-    ``all_decode``, one row per entry.  ``scratch`` lives as long as the
+    and ``max_kv_len``, upper bounds; ``host_cu_rows`` and ``host_kv_len``, exact
+    in a step that is not recorded, while in a recorded one ``host_kv_len`` is
+    empty and ``host_cu_rows`` is one way out of many of giving the entries their
+    rows (all rows of the portions to the first of them), so that a sum over it is
+    no bound; ``all_decode``, one row per entry.  ``scratch`` lives as long as the
     recording: a part may keep a plan or a buffer there."""
 
     n_rows: int

@@ -54,17 +54,21 @@ def lib_for(dim: int, rot_dim: int, vdim: int) -> ctypes.CDLL:
 def plan(ctx, n_rows: int, window: int, bytes_per_key: int) -> int:
     """Rows of the buffers that hold the step's keys (at least as many as there are: a recorded step knows bounds only), or
     0 when the step runs over the latents.  Every entry has to bring rows enough on average, and the keys made must not
-    be many times the rows that read them (portions far behind in long contexts, recordings with room for many)."""
+    be many times the rows that read them (portions far behind in long contexts, recordings with room for many).
+    Behind a window an entry's keys begin at the last multiple of ``KEY_TILE`` that its first row sees, at most
+    ``window + KEY_TILE - 2`` before that row."""
     if n_rows < MIN_ROWS_PER_ENTRY * ctx.n_entries:
         return 0
-    lens, most = list(getattr(ctx, "host_kv_len", None) or ()), 16 * n_rows
-    if len(lens) != ctx.n_entries:  # (a recording: its buffers, for the longest cache it may meet, stay with it)
-        most = 8 * n_rows
-        lens = [ctx.max_kv_len] * ctx.n_entries
-    if window > 0:
-        cu = ctx.host_cu_rows
-        lens = [min(n, window + cu[i + 1] - cu[i] + KEY_TILE) for i, n in enumerate(lens)]
-    keys = sum(lens)
+    lens, reach = list(getattr(ctx, "host_kv_len", None) or ()), window + KEY_TILE - 2
+    if len(lens) == ctx.n_entries:
+        most, cu = 16 * n_rows, ctx.host_cu_rows
+        keys = sum(min(n, cu[i + 1] - cu[i] + reach) if window > 0 else n for i, n in enumerate(lens))
+    else:
+        # a recording: lengths up to the bound, the rows among the entries in any way (``host_cu_rows`` does not say);
+        # its buffers stay with it
+        most, keys = 8 * n_rows, ctx.n_entries * ctx.max_kv_len
+        if window > 0:
+            keys = min(keys, n_rows + ctx.n_entries * reach)
     if keys > most or keys * bytes_per_key > MAX_KEY_BYTES:
         return 0
     return keys

@@ -99,3 +99,54 @@ def test_token_groups_are_even_and_bounded():
     assert gemm_tc.choose_token_group(2048, 4096) == 8      # one group: as before there were groups
     assert gemm_tc.choose_token_group(2048, 14336) == 8
     assert gemm_tc.choose_token_group(8192, 14336) == 8     # four groups of 2,048 tokens
+
+
+def _portion_step(rng):
+    """A recorded step's shape as ``DecodeRunner`` describes it, and one way the rows of a replay may fall to its entries:
+    (context, rows, [(cached before, rows) of each entry])."""
+    cap = rng.choice([256, 1024, 4096])
+    size, K = rng.choice([0, 0, 0, 1, 4]), rng.choice([1, 3, 12])
+    portion = rng.choice([64, 192, 512, 1024, 1536, 2048])
+    rows = size + portion
+    ctx = SimpleNamespace(n_entries=size + K + 1, host_kv_len=[], max_kv_len=cap,
+                          host_cu_rows=list(range(size + 1)) + [rows] * (K + 1))
+    parts = min(K, rng.randint(1, K))
+    most = min(cap, 512)
+    shares = [min(most, max(2, rng.choice([portion // parts, rng.randint(2, most)]))) for _ in range(parts)]
+    while sum(shares) > portion:
+        shares.pop()
+    left = portion - sum(shares)
+    entries = [(rng.randint(0, cap - 1), 1) for _ in range(size)]
+    entries += [(rng.choice([cap - n, (cap - n) // 2, rng.randint(0, cap - n)]), n) for n in shares]
+    entries += [(0, 0)] * (K - len(shares)) + [(0, min(left, cap))]
+    return ctx, rows, entries
+
+
+def test_made_keys_find_room_however_a_recorded_step_spreads_its_rows():
+    """Wherever ``plan`` sends a step over made keys, its buffer holds them: those of an entry begin at the last multiple
+    of 128 in front of its first row's window.  Lengths known on the host give a bound too, and a tighter one."""
+    import random
+
+    from infernum_b200.ops import attention_expanded as ae
+
+    def needed(entries, window):
+        return sum(q + n - (max(0, q - window + 1) // 128 * 128 if window > 0 else 0) for q, n in entries if n > 0)
+
+    # three portions of 512 behind 512 cached tokens, in the engine's default limits
+    ctx = SimpleNamespace(n_entries=4, host_kv_len=[], max_kv_len=1024, host_cu_rows=[0, 1536, 1536, 1536, 1536])
+    for window in (128, 256, 512):
+        assert ae.plan(ctx, 1536, window, 1) >= needed([(512, 512)] * 3, window)
+    rng, taken = random.Random(5), 0
+    for _ in range(4000):
+        ctx, rows, entries = _portion_step(rng)
+        window = rng.choice([0, 1, 37, 128, 129, 512, 700, 4096])
+        got = ae.plan(ctx, rows, window, 1)
+        assert got == 0 or got >= needed(entries, window), (vars(ctx), window, entries)
+        taken += got > 0
+        entries = [(q, n) for q, n in entries if n > 0]
+        cu = [sum(n for _, n in entries[:i]) for i in range(len(entries) + 1)]
+        known = SimpleNamespace(n_entries=len(entries), host_kv_len=[q + n for q, n in entries], host_cu_rows=cu,
+                                max_kv_len=max(q + n for q, n in entries))
+        got = ae.plan(known, cu[-1], window, 1)
+        assert got == 0 or needed(entries, window) <= got <= needed(entries, window) + (256 if window else 0) * len(entries)
+    assert taken > 400

@@ -410,6 +410,25 @@ def test_latent_attention_over_made_keys_against_the_plain_kernel(heads, window,
     assert outs[0].isfinite().all() and rel_err(outs[0], outs[1]) < TOL[torch.bfloat16]
 
 
+@pytest.mark.parametrize("short", [0, 1, 200])
+def test_keys_that_find_no_row_in_the_buffer_are_reported(short):
+    """The gathered latents end with the buffer: one that is too small sets the error word and is written to its end only."""
+    from infernum_b200.ops import attention_expanded, core
+
+    lib, i32 = attention_expanded.lib_for(128, 64, 128), lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)  # noqa: E731
+    pool = torch.randn(40, 1, 16, 128, device=DEV).to(torch.bfloat16)
+    tables, cu, start = i32([list(range(20)), list(range(20, 40))]), i32([0, 70, 170]), i32([230, 0])
+    keys = (300 - 128) + 100  # (a window of 90: the first entry's first row sees keys from 141 on, its buffer begins at 128)
+    out = torch.full((keys + 3, 128), 7.0, dtype=torch.bfloat16, device=DEV)
+    err = core.new_error_word(DEV)
+    core.check(lib.ib_gather_latents(pool.data_ptr(), out.data_ptr(), cu.data_ptr(), start.data_ptr(), tables.data_ptr(), 20, 2,
+                                     16, 40, 90, 128, keys - short, err.data_ptr(), core.stream_ptr(out)), "gather_latents")
+    want = torch.cat([torch.zeros(13, 128, device=DEV), pool.view(-1, 128)[141:300].float(), pool.view(-1, 128)[320:420].float()])
+    assert torch.equal(out[: keys - short].float(), want[: keys - short]) and bool((out[keys - short:] == 7.0).all())
+    assert int(err.item()) == (core.FLAG_KEYS_LOST if short else 0)
+    assert "buffer made for them" in core.describe_flags(core.FLAG_KEYS_LOST)
+
+
 @pytest.mark.parametrize("rule, heads, groups, rows, cols", [("ssd", 4, 2, 128, 64), ("ssd", 3, 1, 64, 128),
                                                              ("delta", 4, 2, 128, 128), ("delta", 3, 3, 64, 64),
                                                              ("delta", 2, 1, 128, 192)])

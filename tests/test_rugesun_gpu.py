@@ -317,6 +317,29 @@ def test_command_line_generate(models, tmp_path):
     assert "Generated 4 tokens" in out.stdout
 
 
+def test_portions_of_three_prompts_behind_a_window_from_a_recording(tmp_path):
+    """Three prompts of 1,024 tokens in portions of 512, windows of 512 and 200, heads whose keys and values prompts make:
+    the second step, replayed from a recording, against the same engine with the plain attention kernel (bfloat16
+    both: what the two round differently stays below the tolerance of this file)."""
+    import infernum_b200 as ib
+    from rugesun_cases import DENSE, layer, mixer
+    config = {"architecture": "Rugesun", "vocab": 211, "width": 128, "postln_alpha": 1.5, "logit_softcap": 20.0,
+              "norm": {"eps": 1e-6}, "embedding": {"bigram": {"buckets": 97, "mul_prev": 7, "mul_cur": 13}},
+              "layers": [layer(mixer(2, 128, 64, 128, 64, 64, 0.1, 512), DENSE(128)),
+                         layer(mixer(3, 128, 64, 128, 64, 64, 0.1, 200), DENSE(128))]}
+    folder = make_folder(str(tmp_path), config, seed=5, sharpen=4.0)
+    prompts, logits = [random_tokens(1024, 211, 7 + i) for i in range(3)], []
+    for options in ({}, {"attention": "plain"}):
+        model = ib.load_model(folder, dtype="bfloat16", options=options)
+        engine = ib.Engine(model, ib.BatchConfig(max_batch_size=3, num_blocks=256))
+        handles = [engine.submit(p, ib.GenerateOptions(max_new_tokens=1)) for p in prompts]
+        engine.run_until_done(handles)
+        assert all(h.seq.finish_reason != ib.FinishReason.ERROR for h in handles), handles[0].seq.error
+        assert engine.decoder.counts["replayed"] + engine.decoder.counts["recorded"] >= 1
+        logits.append(engine.decoder.last.logits[:3].double())
+    assert rel_err(logits[0], logits[1]) < TOL16
+
+
 # ---- mechanisms alone -------------------------------------------------------------------
 def step_context(cache, requests, tokens=None):
     from types import SimpleNamespace
