@@ -470,7 +470,7 @@ attention_expanded_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
         if (!ok && lane == 0) atomicOr(p.err, IB_TIMEOUT_AT(IB_SITE_EXPANDED_SOFTMAX));
         float inv = inv_denominator(p.sink, h, m_run * p.scale_log2, l_run);
         if (p.gate && valid)
-            inv *= 1.f / (1.f + expf(-to_f32(p.gate[(size_t)(row0 + r_begin + m) * p.gate_stride + h])));
+            inv *= 1.f / (1.f + expf(-load1(p.gate + (size_t)(row0 + r_begin + m) * p.gate_stride + h)));
         bf16* dst = valid ? p.out + (size_t)(row0 + r_begin + m) * p.out_stride + (size_t)h * VD : nullptr;
 #pragma unroll
         for (int c = 0; c < VD; c += 16) {

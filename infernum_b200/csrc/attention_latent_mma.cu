@@ -381,7 +381,7 @@ __global__ void latent_combine_kernel(const float* __restrict__ part_o, const fl
     float wa = a.x > -INFINITY ? __expf(a.x - mx) : 0.f, wb = b.x > -INFINITY ? __expf(b.x - mx) : 0.f;
     const float denom = warp_sum(wa * a.y + wb * b.y);
     float inv = denom > 0.f ? 1.f / denom : 0.f;
-    if (gate) inv *= gate_factor(gate[(size_t)r * gate_rs + h]);
+    if (gate) inv *= gate_factor(__ldcg(gate + (size_t)r * gate_rs + h));
     wa *= inv;
     wb *= inv;
     // four columns a thread, 16 bytes a load (KV is a multiple of 32, the scratch 16-byte aligned)

@@ -154,7 +154,9 @@ template <typename T> __device__ __forceinline__ T from_f32(float v);
 template <> __device__ __forceinline__ float from_f32<float>(float v) { return v; }
 template <> __device__ __forceinline__ bf16 from_f32<bf16>(float v) { return __float2bfloat16_rn(v); }
 
-// Four neighbouring values, past the L1 (a kernel begun under its predecessor's tail may meet an older line there).
+// One value, or four neighbouring ones, past the L1 (a kernel begun under its predecessor's tail may meet an older line there).
+__device__ __forceinline__ float load1(const float* p) { return __ldcg(p); }
+__device__ __forceinline__ float load1(const bf16* p) { return __bfloat162float(__ldcg(p)); }
 __device__ __forceinline__ float4 load4(const float* p) { return __ldcg(reinterpret_cast<const float4*>(p)); }
 __device__ __forceinline__ float4 load4(const bf16* p) {
     const uint2 r = __ldcg(reinterpret_cast<const uint2*>(p));

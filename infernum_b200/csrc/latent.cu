@@ -133,11 +133,11 @@ latent_prepare_fours_kernel(const TI* __restrict__ lat, int lat_stride, int q_ra
         T* to = dst + kv_rank;
         if (i < half) {
             const int a = adjacent ? 2 * i : i, b = adjacent ? 2 * i + 1 : i + half;
-            const float u = to_f32(rt[a]), r = to_f32(rt[b]);
+            const float u = load1(rt + a), r = load1(rt + b);
             to[a] = from_f32<T>(u * cs - r * sn);
             to[b] = from_f32<T>(r * cs + u * sn);
         } else {
-            to[i + half] = from_f32<T>(to_f32(rt[i + half]));
+            to[i + half] = from_f32<T>(load1(rt + i + half));
         }
     }
     __syncthreads();
@@ -240,11 +240,11 @@ __global__ void latent_q_rotate_kernel(const T* __restrict__ q, int q_stride, in
         if (i < half) {
             const int a = adjacent ? 2 * i : i, b = adjacent ? 2 * i + 1 : i + half;
             const float2 t = i < ROTATE_PAIRS ? turn[i] : angle(i);
-            const float u = to_f32(src[a]), v = to_f32(src[b]);
+            const float u = load1(src + a), v = load1(src + b);
             dst[a] = from_f32<T>(u * t.y - v * t.x);
             dst[b] = from_f32<T>(v * t.y + u * t.x);
         } else {
-            dst[i + half] = src[i + half];
+            dst[i + half] = from_f32<T>(load1(src + i + half));
         }
     }
 }

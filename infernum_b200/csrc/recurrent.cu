@@ -274,7 +274,7 @@ ssd_prepare_rows_kernel(const T* __restrict__ x, int x_stride, const float* __re
     if (blockIdx.y == gridDim.y - 1) {   // the gates of the heads
         for (int i = threadIdx.x; i < heads * (r1 - r0); i += blockDim.x) {
             const int h = i % heads, row = r0 + i / heads;
-            const float raw = to_f32(dt_raw[(size_t)row * dt_stride + h]) + dt_bias[h];
+            const float raw = load1(dt_raw + (size_t)row * dt_stride + h) + dt_bias[h];
             const float dt = raw > 20.f ? raw : log1pf(expf(raw));
             dd[(size_t)h * n_rows + row] = make_float2(dt, expf(-expf(a_log[h]) * dt));
         }
@@ -900,8 +900,8 @@ delta_prepare_rows_kernel(const T* __restrict__ x, int x_stride, int c_off, int 
     if (blockIdx.y == gridDim.y - 1) {   // the gates of the heads
         for (int i = threadIdx.x; i < H * (r1 - r0); i += blockDim.x) {
             const int h = i % H, row = r0 + i / H;
-            const float b = to_f32(x[(size_t)row * x_stride + b_off + h]);
-            const float a = to_f32(x[(size_t)row * x_stride + a_off + h]) + dt_bias[h];
+            const float b = load1(x + (size_t)row * x_stride + b_off + h);
+            const float a = load1(x + (size_t)row * x_stride + a_off + h) + dt_bias[h];
             const float sp = a > 20.f ? a : log1pf(expf(a));
             dd[(size_t)h * n_rows + row] = make_float4(1.f / (1.f + expf(-b)), expf(-expf(a_log[h]) * sp), 0.f, 0.f);
         }
