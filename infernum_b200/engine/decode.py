@@ -122,8 +122,11 @@ class DecodeRunner:
         w = max(list(windows) + [1])
         return -(-w // cls.RECENT_WIDTH) * cls.RECENT_WIDTH
     # Buffers and graphs are kept for this many (bucket, cache-length class, sampling, feed,
-    # portion) keys; beyond it the one unused for longest is dropped (a graph holds its own
-    # activations: some 65 KB a row at the 8B layer sizes, 35 MB for a portion of 512).
+    # portion) keys; beyond it the one unused for longest is dropped.  A recording keeps its input
+    # buffers and its logits (4 bytes a selected row and token of the vocabulary, valid until the next
+    # step runs).  Activations and the kernels' scratch - a prompt's keys made of latents or its states
+    # before the chunks of a scan may take a GiB each - lie in one pool that all recordings share:
+    # steps follow one another on one stream, so it holds as much as the largest of them needs.
     MAX_RECORDED = 256
     # Entries a recorded step may hold for prompt portions: the smallest of these that takes the
     # step's portions (a step with more runs kernel by kernel).  Part of a recording's key.
@@ -144,6 +147,7 @@ class DecodeRunner:
         self._slots: Dict[tuple, _Slot] = {}
         self._pinned: Optional[Tuple[tuple, List[RequestCache]]] = None
         self.last: Optional[_Slot] = None
+        self._pool = None  # of the recordings' memory
         # results of launched steps on their way to the host, oldest first
         self._reads: collections.deque = collections.deque(maxlen=4)
         # how the steps so far ran: kernel by kernel, recorded (and replayed at once), replayed
@@ -302,7 +306,9 @@ class DecodeRunner:
             collecting = gc.isenabled()
             gc.disable()
             try:
-                with torch.cuda.graph(graph, capture_error_mode="thread_local"):
+                if self._pool is None:
+                    self._pool = torch.cuda.graph_pool_handle()
+                with torch.cuda.graph(graph, pool=self._pool, capture_error_mode="thread_local"):
                     self._body(slot, device_feed)
             finally:
                 if collecting:

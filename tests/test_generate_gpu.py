@@ -681,3 +681,42 @@ def test_profile_mode_times_every_operation(folders, monkeypatch):
     text = core.profile_report()
     assert "share" in text and "add_rmsnorm" in text
     core._profile_totals.clear()
+
+
+def test_recordings_share_one_pool_of_memory():
+    """Recorded steps keep their buffers and logits; what a step allocates while it runs lies in one pool, as large as the
+    largest step's, and steps replayed in any order do not disturb one another's results."""
+    import infernum_b200 as ib
+
+    def private():
+        sizes = {}
+        for seg in torch.cuda.memory_snapshot():
+            if tuple(seg["segment_pool_id"]) != (0, 0):
+                sizes[tuple(seg["segment_pool_id"])] = sizes.get(tuple(seg["segment_pool_id"]), 0) + seg["total_size"]
+        return sizes
+
+    config = {"model_type": "llama", "num_hidden_layers": 2, "hidden_size": 1024, "num_attention_heads": 8,
+              "num_key_value_heads": 2, "head_dim": 128, "intermediate_size": 4096, "vocab_size": 1000, "rope_theta": 10000.0,
+              "rms_norm_eps": 1e-5, "tie_word_embeddings": False, "max_position_embeddings": 4096}
+    model = ib.random_model(config, seed=3, dtype="bfloat16", device="cuda:0")
+    engine = ib.Engine(model, ib.BatchConfig(max_batch_size=1, max_prefill_tokens=2048, num_blocks=256))
+    prompts = {n: random_tokens(n, 1000, n) for n in (1900, 1700, 1500, 1300, 1100, 900, 60)}
+    opts, others = ib.GenerateOptions(max_new_tokens=1), set(private())
+
+    def logits(n):
+        engine.generate(prompts[n], opts)
+        return engine.decoder.last.logits.clone()
+
+    first, largest = {}, 0
+    for n in prompts:
+        logits(n)             # kernel by kernel
+        first[n] = logits(n)  # recorded and replayed
+        mine = {k: v for k, v in private().items() if k not in others}
+        assert len(mine) == 1
+        largest = largest or sum(mine.values())
+    recorded = engine.decoder.counts["recorded"]
+    assert recorded >= len(prompts)
+    assert sum(mine.values()) <= 1.5 * largest
+    for n in sorted(prompts):
+        assert torch.equal(logits(n), first[n]), n
+    assert engine.decoder.counts["recorded"] == recorded and engine.decoder.counts["replayed"] >= len(prompts)
