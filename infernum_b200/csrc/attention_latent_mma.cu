@@ -362,8 +362,10 @@ __global__ void __launch_bounds__(128 * RG) latent_attention_kernel(const Latent
 // out[row, head, :] = sum_s exp(m_s - M) O_s / sum_s exp(m_s - M) l_s over the splits.
 // One block per (row, head): every warp turns the splits' maxima and denominators into one weight
 // per split (a lane two splits), and every thread then sums its columns over the splits in split
-// order, sixteen loads in flight.  Bound by the chain of two loads.  (27 splits of 256 rows and
-// heads, KV 512, with the weights made by one thread: 13.6 us; 7.9 us here.)
+// order, eight loads in flight: with few blocks bound by the chain of two loads, with thousands by
+// the bytes, for which an SM has to hold many blocks (sixteen loads take the registers of half of
+// them).  With the attention before it, KV 512, the weights made by one thread / sixteen loads /
+// eight: 27 splits of 256 rows and heads 25.2 / 23.1 / 21.8 us, 3 splits of 6,144 83.1 / 103.2 / 80.9.
 __global__ void latent_combine_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
                                       bf16* __restrict__ out, int o_rs, int o_hs, int n_rows, int heads,
                                       int splits, const bf16* __restrict__ gate, int gate_rs) {
@@ -389,13 +391,13 @@ __global__ void latent_combine_kernel(const float* __restrict__ part_o, const fl
         const int c = c0 + threadIdx.x * 4;
         float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
         const float* src = part_o + (size_t)pr * KV + (c < KV ? c : 0);
-        for (int s0 = 0; s0 < splits; s0 += 16) {
-            float4 v[16];
+        for (int s0 = 0; s0 < splits; s0 += 8) {
+            float4 v[8];
 #pragma unroll
-            for (int k = 0; k < 16; ++k)
+            for (int k = 0; k < 8; ++k)
                 if (s0 + k < splits) v[k] = __ldcg(reinterpret_cast<const float4*>(src + (size_t)(s0 + k) * stride * KV));
 #pragma unroll
-            for (int k = 0; k < 16; ++k)
+            for (int k = 0; k < 8; ++k)
                 if (s0 + k < splits) {
                     const float w = __shfl_sync(0xffffffffu, s0 < 32 ? wa : wb, (s0 + k) & 31);
                     acc.x += w * v[k].x;
