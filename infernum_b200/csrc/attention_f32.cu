@@ -255,7 +255,7 @@ __global__ void __launch_bounds__(128) attention_f32_tile_kernel(const F32Params
             corr = expf(m[i] - top);
             l[i] = l[i] * corr + expf(sk - top);
         }
-        const float inv = l[i] > 0.f ? corr / l[i] : 0.f;
+        const float inv = corr / l[i];   // (a row sees its own key: a sum of 0, or NaN, is NaN in the result)
         float* op = p.out + (size_t)(first + pr / group) * p.out_stride + (size_t)head * HD + lx * 4;
 #pragma unroll
         for (int c = 0; c < HD / 32; ++c)
@@ -395,7 +395,8 @@ __global__ void __launch_bounds__(128) attention_f32_rows_kernel(const F32Params
                     sum = fmaf(peer(&all_l[h], r), corr, sum);
                     a = fmaf(peer(&all_acc[h][d], r), corr, a);
                 }
-            p.out[(size_t)row * p.out_stride + (size_t)head * HD + d] = sum > 0.f ? a / sum : 0.f;
+            // (with keys a sum of 0 - every score -inf - or NaN is NaN in the result)
+            p.out[(size_t)row * p.out_stride + (size_t)head * HD + d] = n > 0 || sum > 0.f ? a / sum : 0.f;
         }
     }
     asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");   // the shares are read

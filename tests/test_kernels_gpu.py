@@ -399,6 +399,25 @@ def test_attention_in_32_bit_tiles_and_rows(nh, nkv, hd, ps, lens, rows, window,
     assert rel_err(out[rest], ref[rest]) < 2e-6 and not bool(out[rows[0] - 1].isfinite().any())
 
 
+@pytest.mark.parametrize("lens, rows", [([130, 3, 40], [130, 3, 20]), ([700, 1, 129], [1, 1, 1]), ([30, 17], [4, 2])])
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("value", [float("nan"), float("inf"), float("-inf")])
+def test_attention_in_32_bit_hides_no_nan(lens, rows, hd, value):
+    """A query with a NaN, and one whose scores are all infinite, give NaN as they do in the plain kernel (with -inf no key
+    is left to divide by), and the other rows do not change."""
+    c, nh, nkv = core(), 8, 2
+    q, kp, vp, tables, ctx, _ = paged_case(lens, rows, nh, nkv, hd, 16, torch.float32, 3, poison=True)
+    kp[..., 0] = kp[..., 0].abs() + 0.1
+    err, ref, out = c.new_error_word(DEV), torch.empty_like(q), torch.empty_like(q)
+    q[rows[0] - 1, 3 * hd] = value   # (head 3 of the first entry's last row)
+    q[-1, 0] = value
+    c.attention_plain(q, kp, vp, ref, ctx.positions, ctx.row_entry, tables, nh, hd ** -0.5, 0, err)
+    assert c.attention_f32(q, kp, vp, out, ctx, tables, nh, hd ** -0.5, 0, err)
+    assert err.item() == 0 and int(ref.isnan().sum()) == 2 * hd
+    assert torch.equal(out.isnan(), ref.isnan())
+    assert rel_err(out.nan_to_num(), ref.nan_to_num()) < 2e-6
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_attention_plain_finds_a_far_key(dtype):
     """Among hundreds of keys one far key carries the answer."""
