@@ -584,7 +584,8 @@ def attention_f32(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, o
             or not k_pool.is_contiguous() or not v_pool.is_contiguous() or q.stride(1) != 1 or out.stride(1) != 1 \
             or q.stride(0) % 4 or out.stride(0) % 4 or q.shape[1] < n_heads * hd or out.shape[1] < n_heads * hd \
             or any(t.data_ptr() % 16 for t in (q, k_pool, v_pool, out)) \
-            or max(q.shape[0], ctx.n_entries, n_heads) > 65535:
+            or max(q.shape[0], ctx.n_entries, n_heads) > 65535 \
+            or ctx.max_rows_per_entry * (n_heads // nkv) > 65535 * 64:  # (tiles of 64 rows and heads, on the grid's z)
         return False
     require_cuda(q, k_pool, v_pool, out, ctx.positions, ctx.row_entry, block_tables, err, sink)
     for t, name in ((ctx.positions, "positions"), (ctx.row_entry, "row_entry"), (ctx.cu_rows, "cu_rows"),

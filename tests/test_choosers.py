@@ -3,9 +3,10 @@ checked without a GPU against the properties the kernels rely on."""
 from types import SimpleNamespace
 
 import numpy as np
+import torch
 
 from infernum_b200.cache import CacheManager
-from infernum_b200.ops import attention_fast, gemm_tc
+from infernum_b200.ops import attention_fast, core, gemm_tc
 from infernum_b200.parts.base import PagedCacheSpec
 
 
@@ -150,3 +151,13 @@ def test_made_keys_find_room_however_a_recorded_step_spreads_its_rows():
         got = ae.plan(known, cu[-1], window, 1)
         assert got == 0 or needed(entries, window) <= got <= needed(entries, window) + (256 if window else 0) * len(entries)
     assert taken > 400
+
+
+def test_steps_of_more_row_tiles_than_a_grid_holds_are_left_to_the_plain_kernel():
+    """65 query heads a key/value head and 65,000 rows of one entry: 66,016 tiles of 64."""
+    rows, heads, hd = 65000, 65, 64
+    q = torch.empty(1, heads * hd).expand(rows, heads * hd)
+    pool = torch.empty(2, 1, 16, hd)
+    ctx = SimpleNamespace(n_entries=1, max_rows_per_entry=rows, max_kv_len=rows)
+    assert not core.attention_f32(q, pool, pool, q, ctx, torch.zeros(1, 1, dtype=torch.int32), heads, 1.0, 0,
+                                  torch.zeros(1, dtype=torch.int32))
