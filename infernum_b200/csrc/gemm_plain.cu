@@ -399,7 +399,8 @@ static int launch_f32(const void* A, int lda, const void* W, int ldw, void* C, i
     auto rounds = [&](int t) {
         return (double)(((long long)((M + t - 1) / t) * ((N + t - 1) / t) * batch + 147) / 148);
     };
-    return rounds(32) * 0.25 * SMALL_TILE_COST < rounds(64) ? IB_F32((launch_tile<32, 32, 4, 4>))
+    // (the rows' tiles are on the grid's y; small ones are cheaper at any number of rows where N <= 32)
+    return (M + 31) / 32 <= 65535 && rounds(32) * 0.25 * SMALL_TILE_COST < rounds(64) ? IB_F32((launch_tile<32, 32, 4, 4>))
                                                             : IB_F32((launch_tile<64, 64, 8, 4>));
 #undef IB_F32
 }

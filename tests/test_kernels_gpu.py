@@ -216,6 +216,17 @@ def test_gemm_plain_in_32_bit_gives_the_same_bits_by_every_kernel(M, N, K):
     assert torch.equal(even, ref)
 
 
+def test_gemm_plain_in_32_bit_takes_more_rows_than_small_tiles_on_a_grid():
+    """2,097,121 rows: 65,536 tiles of 32, one more than a grid's y holds."""
+    c, M, N, K = core(), 65535 * 32 + 1, 3, 4
+    a, w = torch.randn(M, K, device=DEV), torch.randn(N, K, device=DEV)
+    out, ref = torch.empty(M, N, device=DEV), torch.empty(100, N, device=DEV)
+    c.gemm_plain(a, w, out)
+    for at in (0, M - 100):
+        c.gemm_plain(a[at: at + 100], w, ref)
+        assert torch.equal(out[at: at + 100], ref)
+
+
 def test_argmax_lowest_index_wins():
     c = core()
     x = torch.randn(6, 1000)
