@@ -72,12 +72,14 @@ def chunk_lib_for(rows: int) -> ctypes.CDLL:
     return lib
 
 
-def in_chunks(ctx, n_rows: int, rows: int, cols: int, state_ptr: int, state_stride: int, heads: int = 1) -> bool:
-    """Whether a step's scan runs in chunks of 64 tokens: where a request brings a prompt (below some hundred tokens the
-    walk token by token is over before three or four launches are), and not for its sake alone beside many decoded tokens, each
-    of which would be a chunk.  The states before the chunks are kept for the results: up to 1 GiB of them (34 MB for
-    2,048 tokens of 32 heads of 128 x 64); beyond, the walk needs none."""
-    if (n_rows // 64 + ctx.n_entries) * heads * rows * cols * 4 > CHUNK_MAX_BYTES:
+def in_chunks(ctx, n_rows: int, rows: int, cols: int, state_ptr: int, state_stride: int, heads: int = 1, groups: int = 1,
+              delta: bool = False) -> bool:
+    """Whether a step's scan can run in chunks of 64 tokens: where a request brings a prompt, and not for its sake alone
+    beside many decoded tokens, each of which would be a chunk.  What the kernels pass one another - the states before the
+    chunks, their keys' products, a delta rule's two solutions - takes up to 1 GiB (36 MB for 2,048 tokens of 32 heads
+    of 128 x 64); beyond, the walk token by token needs none."""
+    floats = (n_rows // 64 + ctx.n_entries) * (heads * (rows * cols + 1) + 4 + (2 if delta else 1) * groups * 64 * 64)
+    if 4 * (floats + (heads * n_rows * (rows + cols) if delta else 0)) > CHUNK_MAX_BYTES:
         return False
     most = getattr(ctx, "max_rows_per_entry", n_rows)
     return (rows in CHUNK_ROWS and cols % 64 == 0 and state_ptr % 16 == 0 and state_stride % 4 == 0
@@ -233,7 +235,7 @@ def ssd_scan(xbc: torch.Tensor, dt: torch.Tensor, dt_bias: torch.Tensor, a_log: 
         conv_ptr, conv_stride = _state_ptr(state, conv_offset)
     ptr, stride = _state_ptr(state, state_offset)
     # (prompts in chunks read B and C one after the other, which the pass for rows of fours with four taps writes)
-    chunked = in_chunks(ctx, N, state_rows, vdim, ptr, stride, heads) and out.data_ptr() % 16 == 0 and taps == 4 \
+    chunked = in_chunks(ctx, N, state_rows, vdim, ptr, stride, heads, groups) and out.data_ptr() % 16 == 0 and taps == 4 \
         and conv_ptr % 16 == 0 and xbc.stride(0) % 4 == 0 and xbc.data_ptr() % (4 * xbc.element_size()) == 0 \
         and w.data_ptr() % 16 == 0 and (b is None or b.data_ptr() % 16 == 0)
     prepare = core.core_lib().ib_ssd_prepare_rows if chunked else core.core_lib().ib_ssd_prepare
@@ -296,7 +298,7 @@ def delta_scan(proj: torch.Tensor, c_off: int, b_off: int, a_off: int, conv_w: O
     dd = torch.empty((heads, N, 4), dtype=torch.float32, device=dev)
     conv_ptr, conv_stride = _state_ptr(state, conv_offset)
     ptr, stride = _state_ptr(state, state_offset)
-    chunked = in_chunks(ctx, N, dim, vdim, ptr, stride, heads) and out.data_ptr() % 16 == 0
+    chunked = in_chunks(ctx, N, dim, vdim, ptr, stride, heads, kv_heads, delta=True) and out.data_ptr() % 16 == 0
     core.check(core.core_lib().ib_delta_prepare(
         proj.data_ptr(), proj.stride(0), core.dtype_code(proj.dtype), int(c_off), int(b_off), int(a_off),
         conv_w.data_ptr() if conv_w is not None else None, taps, conv_ptr, conv_stride, ctx.row_entry.data_ptr(),

@@ -6,7 +6,7 @@ import numpy as np
 import torch
 
 from infernum_b200.cache import CacheManager
-from infernum_b200.ops import attention_fast, core, gemm_tc
+from infernum_b200.ops import attention_fast, core, gemm_tc, scan
 from infernum_b200.parts.base import PagedCacheSpec
 
 
@@ -161,3 +161,21 @@ def test_steps_of_more_row_tiles_than_a_grid_holds_are_left_to_the_plain_kernel(
     ctx = SimpleNamespace(n_entries=1, max_rows_per_entry=rows, max_kv_len=rows)
     assert not core.attention_f32(q, pool, pool, q, ctx, torch.zeros(1, 1, dtype=torch.int32), heads, 1.0, 0,
                                   torch.zeros(1, dtype=torch.int32))
+
+
+def test_scratch_of_chunked_scans_is_counted_whole():
+    """As many floats as the kernels' own count, within the few that round up a chunk; a delta rule's two solutions are as
+    much again as the states before the chunks."""
+    def most_rows(heads, groups, rows, cols, delta):
+        ctx = SimpleNamespace(n_entries=1, max_rows_per_entry=0)
+        low, high = 96, 1 << 24
+        while low < high:
+            ctx.max_rows_per_entry = mid = (low + high + 1) // 2
+            low, high = (mid, high) if scan.in_chunks(ctx, mid, rows, cols, 0, 4, heads, groups, delta) else (low, mid - 1)
+        return low
+
+    for heads, groups, rows, cols, delta in [(32, 1, 128, 64, False), (16, 8, 128, 128, True), (64, 64, 64, 64, True)]:
+        n = most_rows(heads, groups, rows, cols, delta)
+        chunks = n // 64 + 1
+        floats = chunks * (heads * rows * cols + groups * 4096 * (1 + delta)) + (heads * n * (rows + cols) if delta else 0)
+        assert 0.98 * scan.CHUNK_MAX_BYTES < 4 * floats <= scan.CHUNK_MAX_BYTES
