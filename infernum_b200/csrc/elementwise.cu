@@ -38,12 +38,11 @@ __global__ void embed_kernel(const int* __restrict__ ids, const TW* __restrict__
     for (int i = threadIdx.x; i < H; i += blockDim.x) o[i] = to_f32(src[i]) * scale;
 }
 
-// The same, eight elements a thread and access: 16 bytes of a bf16 table's row (32 of a float32 one's) to two 16-byte
-// stores.  Bound by the stores.  bf16 rows, before and after: 64 of 4,096 10.3 -> 3.5 us, 2,048 of 4,096 18.9 -> 12.7 us, one of
-// 2,048 5.6 -> 3.8 us (single launches from a cold cache).
+// The same in fours: 8 bytes of a bf16 table's row (16 of a float32 one's) to one 16-byte store, four of them in flight a
+// thread, so that a warp's store fills whole sectors.  Bound by the stores.
 template <typename TW>
-__global__ void embed_vec_kernel(const int* __restrict__ ids, const TW* __restrict__ table, float* __restrict__ out, int H,
-                                 int V, float scale, unsigned* __restrict__ err) {
+__global__ void embed_fours_kernel(const int* __restrict__ ids, const TW* __restrict__ table, float* __restrict__ out, int H,
+                                   int V, float scale, unsigned* __restrict__ err) {
     pdl_trigger();
     pdl_wait();
     const int row = blockIdx.x;
@@ -51,26 +50,22 @@ __global__ void embed_vec_kernel(const int* __restrict__ ids, const TW* __restri
     const bool known = id >= 0 && id < V;
     if (!known && threadIdx.x == 0) atomicOr(err, IB_FLAG_BAD_TOKEN);
     const TW* src = table + (size_t)(known ? id : 0) * H;
-    float4* o = reinterpret_cast<float4*>(out + (size_t)row * H);
-    for (int i = threadIdx.x; i < (H >> 3); i += blockDim.x) {
-        float v[8];
-        if (sizeof(TW) == 2) {
-            const uint4 raw = reinterpret_cast<const uint4*>(src)[i];
-            const __nv_bfloat162* pair = reinterpret_cast<const __nv_bfloat162*>(&raw);
+    float* o = out + (size_t)row * H;
+    constexpr int AHEAD = 4;
+    for (int i0 = threadIdx.x * 4; i0 < H; i0 += AHEAD * blockDim.x * 4) {
+        float4 v[AHEAD];
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const float2 f = __bfloat1622float2(pair[k]);
-                v[2 * k] = f.x;
-                v[2 * k + 1] = f.y;
-            }
-        } else {
-            *reinterpret_cast<float4*>(v) = reinterpret_cast<const float4*>(src)[2 * i];
-            *reinterpret_cast<float4*>(v + 4) = reinterpret_cast<const float4*>(src)[2 * i + 1];
+        for (int k = 0; k < AHEAD; ++k) {
+            const int i = i0 + k * blockDim.x * 4;
+            if (i < H) v[k] = load4(src + i);
         }
 #pragma unroll
-        for (int k = 0; k < 8; ++k) v[k] = known ? v[k] * scale : 0.f;
-        o[2 * i] = *reinterpret_cast<const float4*>(v);
-        o[2 * i + 1] = *reinterpret_cast<const float4*>(v + 4);
+        for (int k = 0; k < AHEAD; ++k) {
+            const int i = i0 + k * blockDim.x * 4;
+            if (i < H)
+                store4(o + i, known ? make_float4(v[k].x * scale, v[k].y * scale, v[k].z * scale, v[k].w * scale)
+                                    : make_float4(0.f, 0.f, 0.f, 0.f));
+        }
     }
 }
 
@@ -82,8 +77,8 @@ IB_EXPORT int ib_embed_scaled(const int* ids, const void* table, int table_dtype
     if (H % 8 == 0 && (table_dtype == 0 || table_dtype == 1) && !(((uintptr_t)table | (uintptr_t)out) & 15)) {
         const int threads = H >= 2048 ? 256 : H >= 1024 ? 128 : 64;
         const cudaError_t le = table_dtype == 0
-            ? launch_kernel(embed_vec_kernel<float>, dim3(n_rows), dim3(threads), 0, s, ids, (const float*)table, out, H, V, scale, err)
-            : launch_kernel(embed_vec_kernel<bf16>, dim3(n_rows), dim3(threads), 0, s, ids, (const bf16*)table, out, H, V, scale, err);
+            ? launch_kernel(embed_fours_kernel<float>, dim3(n_rows), dim3(threads), 0, s, ids, (const float*)table, out, H, V, scale, err)
+            : launch_kernel(embed_fours_kernel<bf16>, dim3(n_rows), dim3(threads), 0, s, ids, (const bf16*)table, out, H, V, scale, err);
         if (le != cudaSuccess) return (int)le;
         IB_LAUNCH_CHECK();
         return IB_OK;
