@@ -1,7 +1,7 @@
 """Chooses the attention kernel for a step.
 
 ``float32`` engines take the 32-bit tile and row kernels when keys and values
-have 64 or 128 elements, and the plain kernel (one warp per row and head)
+have 64 or 128 elements and there are more than a handful of keys, and the plain kernel (one warp per row and head)
 otherwise, 32-bit throughout.  ``bfloat16`` engines take the tensor-core prefill kernel
 and the split-KV decode kernel when the head size has a compiled variant, and
 the plain kernel otherwise; ``rt.options["attention"] = "plain"`` forces the
@@ -33,9 +33,10 @@ def paged_attention(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor,
         if attention_fast.run(q, k_pool, v_pool, out, ctx, tables, n_heads, scale, window, rt, sink=sink,
                               keep_first=keep_first):
             return
-    if q.dtype == torch.float32 and impl != "plain" and core.attention_f32(
-            q, k_pool, v_pool, out, ctx, tables, n_heads, scale, window, rt.err, sink=sink, keep_first=keep_first,
-            sm_count=rt.options.get("sm_count") or 148):
+    if q.dtype == torch.float32 and impl != "plain" \
+            and not core.f32_few_keys(ctx.max_rows_per_entry, ctx.max_kv_len, k_pool.shape[3]) and core.attention_f32(
+                q, k_pool, v_pool, out, ctx, tables, n_heads, scale, window, rt.err, sink=sink, keep_first=keep_first,
+                sm_count=rt.options.get("sm_count") or 148):
         return
     core.attention_plain(q, k_pool, v_pool, out, ctx.positions, ctx.row_entry, tables, n_heads,
                          scale, window, rt.err, sink=sink, keep_first=keep_first)

@@ -573,6 +573,13 @@ def choose_f32_splits(max_rows_per_entry: int, n_rows: int, heads: int, kv_heads
     return splits
 
 
+def f32_few_keys(max_rows_per_entry: int, max_kv_len: int, hd: int) -> bool:
+    """Whether a float32 step sees so few keys that the plain kernel, a key after the other, is done before
+    ``attention_f32``: 3.2 us with one key against 3.3 to 4.8 row by row (3.7 and 3.3 to 4.8 with two, 4.8 and 3.2 to 5.2
+    with three); against tiles 11.9 us with 13 keys of 64 (12.3) and 17.6 with 18 of 128 (17.6)."""
+    return max_kv_len <= (2 if max_rows_per_entry <= 4 else 13 if hd == 64 else 18)
+
+
 def attention_f32(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, out: torch.Tensor, ctx,
                   block_tables: torch.Tensor, n_heads: int, scale: float, window: int, err: torch.Tensor,
                   sink: Optional[torch.Tensor] = None, keep_first: int = 0, sm_count: int = 148) -> bool:

@@ -179,3 +179,9 @@ def test_scratch_of_chunked_scans_is_counted_whole():
         chunks = n // 64 + 1
         floats = chunks * (heads * rows * cols + groups * 4096 * (1 + delta)) + (heads * n * (rows + cols) if delta else 0)
         assert 0.98 * scan.CHUNK_MAX_BYTES < 4 * floats <= scan.CHUNK_MAX_BYTES
+
+
+def test_a_handful_of_keys_in_32_bit_is_left_to_the_plain_kernel():
+    few = core.f32_few_keys
+    assert few(1, 1, 64) and few(4, 2, 128) and not few(1, 3, 64)
+    assert few(5, 5, 64) and few(13, 13, 64) and not few(5, 14, 64) and few(16, 18, 128) and not few(16, 19, 128)
