@@ -86,6 +86,18 @@ def in_chunks(ctx, n_rows: int, rows: int, cols: int, state_ptr: int, state_stri
             and most >= CHUNK_MIN_ROWS and n_rows >= CHUNK_MIN_MEAN * ctx.n_entries)
 
 
+# Most rows of an entry from which the chunks pay: (where the heads of all rows are few, where they fill the SMs).
+CHUNK_PAY_ROWS = {"ssd": (160, 128), "delta": (256, 160)}
+
+
+def chunks_pay(rule: str, n_rows: int, most: int, heads: int, rt) -> bool:
+    """Whether the chunks are quicker than the walk for a longest entry of ``most`` rows: the walk's time is that entry's,
+    and grows with the heads once they fill the SMs (some 32 heads of entries as long); the chunks' begins with three or four more
+    launches.  ``rt.options["scan"]`` = "chunks" takes them wherever they can run."""
+    few, many = CHUNK_PAY_ROWS[rule]
+    return most >= (many if heads * n_rows >= 32 * most else few) or rt.options.get("scan") == "chunks"
+
+
 def choose_col_slices(n_entries: int, heads: int, cols: int, split: int, sm_count: int) -> int:
     """Into how many CTAs the columns of a head's state are cut.  The warps of a
     scan are as many as its columns times the lanes of a column, whatever the
@@ -235,7 +247,8 @@ def ssd_scan(xbc: torch.Tensor, dt: torch.Tensor, dt_bias: torch.Tensor, a_log: 
         conv_ptr, conv_stride = _state_ptr(state, conv_offset)
     ptr, stride = _state_ptr(state, state_offset)
     # (prompts in chunks read B and C one after the other, which the pass for rows of fours with four taps writes)
-    chunked = in_chunks(ctx, N, state_rows, vdim, ptr, stride, heads, groups) and out.data_ptr() % 16 == 0 and taps == 4 \
+    chunked = in_chunks(ctx, N, state_rows, vdim, ptr, stride, heads, groups) \
+        and chunks_pay("ssd", N, ctx.max_rows_per_entry, heads, rt) and out.data_ptr() % 16 == 0 and taps == 4 \
         and conv_ptr % 16 == 0 and xbc.stride(0) % 4 == 0 and xbc.data_ptr() % (4 * xbc.element_size()) == 0 \
         and w.data_ptr() % 16 == 0 and (b is None or b.data_ptr() % 16 == 0)
     prepare = core.core_lib().ib_ssd_prepare_rows if chunked else core.core_lib().ib_ssd_prepare
@@ -298,7 +311,8 @@ def delta_scan(proj: torch.Tensor, c_off: int, b_off: int, a_off: int, conv_w: O
     dd = torch.empty((heads, N, 4), dtype=torch.float32, device=dev)
     conv_ptr, conv_stride = _state_ptr(state, conv_offset)
     ptr, stride = _state_ptr(state, state_offset)
-    chunked = in_chunks(ctx, N, dim, vdim, ptr, stride, heads, kv_heads, delta=True) and out.data_ptr() % 16 == 0
+    chunked = in_chunks(ctx, N, dim, vdim, ptr, stride, heads, kv_heads, delta=True) \
+        and chunks_pay("delta", N, ctx.max_rows_per_entry, heads, rt) and out.data_ptr() % 16 == 0
     core.check(core.core_lib().ib_delta_prepare(
         proj.data_ptr(), proj.stride(0), core.dtype_code(proj.dtype), int(c_off), int(b_off), int(a_off),
         conv_w.data_ptr() if conv_w is not None else None, taps, conv_ptr, conv_stride, ctx.row_entry.data_ptr(),

@@ -441,7 +441,7 @@ def test_scans_in_chunks_against_one_token_at_a_time(rule, heads, groups, rows, 
 
     from infernum_b200.ops import scan
 
-    rt, N, E = runtime(torch.float32), sum(lens), len(lens)
+    rt, N, E = runtime(torch.float32, scan="chunks"), sum(lens), len(lens)  # (also where they do not pay)
     g = torch.Generator(device=DEV).manual_seed(N + rows)
     rnd = lambda *s: torch.randn(*s, generator=g, device=DEV)  # noqa: E731
     i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)  # noqa: E731
