@@ -240,7 +240,9 @@ class MixtureOfExperts(FeedForward):
         from ..ops import gemm_tc
 
         if self.block == 64 and gemm_tc.grouped_suits(x, self.gate_up.weight, self.down.weight, self.expert_size,
-                                                      self.experts, self.top, self.activation):
+                                                      self.experts, self.top, self.activation) \
+                and (self.rt.options.get("experts") == "grouped" or gemm_tc.grouped_pays(
+                    x.shape[0], self.hidden_size, self.expert_size, self.experts, self.top)):
             return self.grouped(x, ids, wts, gate)
         act = torch.empty((x.shape[0], gate.shape[1] * self.expert_size), dtype=x.dtype, device=x.device)
         fused = False

@@ -195,3 +195,13 @@ def test_scans_of_short_prompts_are_walked():
     assert not pays("ssd", 1, 96, 32) and not pays("ssd", 1, 128, 16) and pays("ssd", 1, 160, 16) and pays("ssd", 1, 128, 32)
     assert not pays("delta", 1, 224, 8) and not pays("delta", 2, 192, 8) and pays("delta", 1, 256, 8)
     assert not pays("delta", 4, 128, 16) and pays("delta", 2, 160, 16) and pays("delta", 1, 96, 4, scan="chunks")
+
+
+def test_experts_run_alone_where_that_saves_more_than_it_costs():
+    """At sizes where the two ways were measured a sixth or more apart."""
+    for hidden, ff, experts, top, rows, alone in [
+            (512, 256, 8, 2, 400, False), (512, 256, 32, 4, 700, True),
+            (1024, 512, 16, 4, 128, False), (1024, 512, 16, 2, 700, True), (2048, 1024, 8, 4, 256, False),
+            (2048, 1024, 8, 4, 512, False), (2048, 512, 8, 2, 100, False), (4096, 256, 32, 4, 65, False),
+            (4096, 1792, 16, 2, 2048, True), (4096, 3584, 16, 4, 2048, True), (2048, 768, 64, 6, 1400, True)]:
+        assert gemm_tc.grouped_pays(rows, hidden, ff, experts, top) == alone, (hidden, ff, experts, top, rows)
