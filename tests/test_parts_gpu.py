@@ -363,9 +363,10 @@ def test_router_logits_of_rows_of_eights(rows, experts, hidden, dx, dw):
 
 @pytest.mark.parametrize("heads, window, sink, gate, q_rank", [(4, 0, False, False, 64), (3, 100, True, True, 0),
                                                                (8, 300, True, False, 64)])
+@pytest.mark.parametrize("dim, vdim", [(128, 128), (128, 64), (64, 128), (64, 64)])
 @pytest.mark.parametrize("past, new, page", [([0], [64], 16), ([0], [129], 4), ([0, 77, 300], [200, 65, 128], 16),
                                              ([513, 0], [300, 31], 32), ([128], [256], 128)])
-def test_latent_attention_over_made_keys_against_the_plain_kernel(heads, window, sink, gate, q_rank, past, new, page):
+def test_latent_attention_over_made_keys_against_the_plain_kernel(heads, window, sink, gate, q_rank, dim, vdim, past, new, page):
     """Prompts of many rows make every head's keys and values; the plain kernel attends over the latents in 32-bit.  Both
     round a handful of intermediate rows to bfloat16, other ones: bfloat16's tolerance of these tests.  Every page
     and slot without a token is NaN."""
@@ -379,7 +380,7 @@ def test_latent_attention_over_made_keys_against_the_plain_kernel(heads, window,
     for options in ({}, {"attention": "plain"}):
         rt = runtime(torch.bfloat16, **options)
         part = build_part("mixer", PartSpec("latent_attention", dict(
-            hidden_size=hidden, num_heads=heads, dim=128, rot_dim=64, vdim=128, q_rank=q_rank, kv_rank=64, scale=0.08,
+            hidden_size=hidden, num_heads=heads, dim=dim, rot_dim=64, vdim=vdim, q_rank=q_rank, kv_rank=64, scale=0.08,
             window=window, eps=1e-5, theta=10000.0, sink="sink" if sink else None, gate="g" if gate else None)), rt)
         gen = torch.Generator(device=DEV).manual_seed(heads + page)
         part.bind({n: (torch.randn(s.shape, generator=gen, device=DEV) * (1.0 if "norm" in n or n == "sink" else 0.15)).to(
