@@ -8,7 +8,8 @@
 // (infernum-cuda/src/inner/cuda/ops/matmul.rs:68-116) on its f32 path.
 //
 // Three kernels with one arithmetic, so that all of them give the same bits:
-//   gemm_rows_kernel   float32, at most 64 rows (decode): the weights stream through shared memory once
+//   gemm_rows_kernel   float32, at most 64 rows, 32 where N x batch >= 8,192 (decode): the weights stream through shared
+//                      memory once
 //   gemm_tile_kernel   float32, more rows: register tiles, two tile sizes
 //   gemm_plain_kernel  any operand types, strides and alignments
 #include "common.cuh"

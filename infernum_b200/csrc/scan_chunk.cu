@@ -397,8 +397,8 @@ __global__ void __launch_bounds__(128) chunk_out_kernel(const SsdParams p) {
 //   chunk_out           every chunk at once: o
 // The walk is the only part that waits for the chunk before: 32 columns a CTA, so that there are four for a head of 128,
 // and the next chunk's operands come while one is worked on.  Two entries of 750 tokens, 16 heads of 128 x 128 on eight key
-// heads: 376 us by scan.cu, 16 + 32 + 110 + 49 us here; the walk is bound by
-// what shared memory hands its small tiles (a 2 x 4 and a 4 x 4 of products a thread).
+// heads: 376 us by scan.cu, 16 + 32 + 110 + 49 us here; the walk is bound by its chain of chunks, two small products between
+// barriers each (a mapping of them with a third of the reads of shared memory: 113 -> 110 us).
 struct DeltaParams {
     SsdParams o;           // what chunk_out reads: x is `u`, bc the k and q, cb the q_t.k_s, carry the states before the chunks
     const float* v;        // [heads][rows][P]

@@ -13,7 +13,7 @@ values, the activation (in that product's epilogue where it can be) multiplies e
 the token's weight for that expert (0 where it was not chosen), and the down
 product sums over all experts at once: ``sum_e Wd_e (w_e a_e)`` is one product
 with the concatenated vector.  What a token did not choose is multiplied by an exact 0.
-Steps of many tokens run each token through the experts it chose only (``grouped``).
+Steps of many tokens run each token through the experts it chose only (``grouped``), where that is quicker.
 
 Parameters: ``hidden_size``, ``expert_size`` (ff), ``experts``, ``top``,
 ``activation`` ("silu" | "gelu_tanh" | "clamped_swish" with ``limit`` and ``alpha``), ``prefix``, ``expert_names`` (format of
