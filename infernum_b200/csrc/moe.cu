@@ -54,11 +54,27 @@ __device__ __forceinline__ void load8(const float* p, float (&v)[8]) {
     v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
 }
 
-// A lane's share of four rows by N experts from e0 on (a row's last ones repeat where there are fewer), v[row][expert].
+// The same for rows of eights: a CTA takes four rows by N experts (eight, where there are more than four), its four warps every fourth run of 256 k, a lane
+// eight neighbouring k of a run.  An expert's values are converted once for four rows, a row's once for N experts.
+// The lanes' sums meet by halves (31 shuffles for 32 logits) and the warps' in their order: a fixed order per logit,
+// whatever the batch.  2,048 rows of 4,096, 16 experts: 64 us a warp a (row, expert) -> 17 us; eight rows 11 -> 5 us.
+// N is 1, 2 or 4 where there are no more experts: one as eight took three times a warp a row (float32, 2,048 rows of
+// 4,096: 22.6 us against 7.2; 8.1 as one, and 3.5 against 6.2 for eight rows).  Which N it is does not change a logit's order.
 template <int N, typename TX, typename TW>
-__device__ __forceinline__ void router_shares(const TX* const (&xr)[4], const TW* __restrict__ w, int ldw, int e0, int E, int k0,
-                                              int K, float (&v)[32]) {
-    for (int k = k0; k < K; k += 1024) {
+__global__ void __launch_bounds__(128) router_logits_tile_kernel(const TX* __restrict__ x, int ldx, const TW* __restrict__ w,
+                                                                 int ldw, float* __restrict__ z, int n_rows, int E, int K) {
+    pdl_trigger();
+    pdl_wait();
+    __shared__ float sums[4][32];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int row0 = blockIdx.x * 4, e0 = blockIdx.y * N;
+    const TX* xr[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) xr[r] = x + (size_t)min(row0 + r, n_rows - 1) * ldx;
+    float v[32];   // [row][expert]
+#pragma unroll
+    for (int i = 0; i < 32; ++i) v[i] = 0.f;
+    for (int k = warp * 256 + lane * 8; k < K; k += 1024) {
         float a[4][8];
 #pragma unroll
         for (int r = 0; r < 4; ++r) load8(xr[r] + k, a[r]);
@@ -72,33 +88,6 @@ __device__ __forceinline__ void router_shares(const TX* const (&xr)[4], const TW
                 for (int i = 0; i < 8; ++i) v[r * 8 + e] = fmaf(a[r][i], b[i], v[r * 8 + e]);
         }
     }
-}
-
-// The same for rows of eights: a CTA takes four rows by eight experts, its four warps every fourth run of 256 k, a lane
-// eight neighbouring k of a run.  An expert's values are converted once for four rows, a row's once for eight experts.
-// The lanes' sums meet by halves (31 shuffles for 32 logits) and the warps' in their order: a fixed order per logit,
-// whatever the batch.  2,048 rows of 4,096, 16 experts: 64 us a warp a (row, expert) -> 17 us; eight rows 11 -> 5 us.
-// What is left of the experts takes a loop of one, two or four where that holds it: one expert as eight was 2.3 times the
-// time of a warp a row (float32, 2,048 rows of 4,096: 7.2 us against 22.6).
-template <typename TX, typename TW>
-__global__ void __launch_bounds__(128) router_logits_tile_kernel(const TX* __restrict__ x, int ldx, const TW* __restrict__ w,
-                                                                 int ldw, float* __restrict__ z, int n_rows, int E, int K) {
-    pdl_trigger();
-    pdl_wait();
-    __shared__ float sums[4][32];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int row0 = blockIdx.x * 4, e0 = blockIdx.y * 8;
-    const TX* xr[4];
-#pragma unroll
-    for (int r = 0; r < 4; ++r) xr[r] = x + (size_t)min(row0 + r, n_rows - 1) * ldx;
-    float v[32];   // [row][expert]
-#pragma unroll
-    for (int i = 0; i < 32; ++i) v[i] = 0.f;
-    const int k0 = warp * 256 + lane * 8;
-    if (E - e0 > 4) router_shares<8>(xr, w, ldw, e0, E, k0, K, v);
-    else if (E - e0 > 2) router_shares<4>(xr, w, ldw, e0, E, k0, K, v);
-    else if (E - e0 == 2) router_shares<2>(xr, w, ldw, e0, E, k0, K, v);
-    else router_shares<1>(xr, w, ldw, e0, E, k0, K, v);
     int o = 1;
 #pragma unroll
     for (int n = 16; n >= 1; n >>= 1, o <<= 1) {
@@ -113,9 +102,19 @@ __global__ void __launch_bounds__(128) router_logits_tile_kernel(const TX* __res
     __syncthreads();
     if (warp == 0) {
         const int row = row0 + lane / 8, e = e0 + lane % 8;
-        if (row < n_rows && e < E)
+        if (row < n_rows && lane % 8 < N && e < E)
             z[(size_t)row * E + e] = ((sums[0][lane] + sums[1][lane]) + sums[2][lane]) + sums[3][lane];
     }
+}
+
+template <typename TX, typename TW>
+static cudaError_t launch_router_tiles(const void* x, int ldx, const void* w, int ldw, float* z, int n_rows, int E, int K,
+                                       cudaStream_t s) {
+    const int n = E > 4 ? 8 : E > 2 ? 4 : E;
+    const dim3 grid((n_rows + 3) / 4, (E + n - 1) / n);
+    auto kernel = n == 8 ? router_logits_tile_kernel<8, TX, TW> : n == 4 ? router_logits_tile_kernel<4, TX, TW>
+                : n == 2 ? router_logits_tile_kernel<2, TX, TW> : router_logits_tile_kernel<1, TX, TW>;
+    return launch_kernel(kernel, grid, dim3(128), 0, s, (const TX*)x, ldx, (const TW*)w, ldw, z, n_rows, E, K);
 }
 
 template <typename TX, typename TW>
@@ -130,24 +129,20 @@ IB_EXPORT int ib_router_logits(const void* x, int x_dtype, int ldx, const void* 
     if (!x || !w || !z || E <= 0 || K <= 0 || ldx < K || ldw < K) return IB_ERR_BAD_ARG;
     const long long warps = (long long)n_rows * E;
     const unsigned blocks = (unsigned)((warps + 7) / 8);
-    const dim3 tiles((n_rows + 3) / 4, (E + 7) / 8);
     cudaStream_t s = (cudaStream_t)stream;
     cudaError_t le;
     if (x_dtype == 0 && w_dtype == 0 && rows_of_eights<float, float>(x, ldx, w, ldw, K))
-        le = launch_kernel(router_logits_tile_kernel<float, float>, tiles, dim3(128), 0, s, (const float*)x, ldx,
-                           (const float*)w, ldw, z, n_rows, E, K);
+        le = launch_router_tiles<float, float>(x, ldx, w, ldw, z, n_rows, E, K, s);
     else if (x_dtype == 0 && w_dtype == 0)
         le = launch_kernel(router_logits_kernel<float, float>, dim3(blocks), dim3(256), 0, s, (const float*)x, ldx,
                            (const float*)w, ldw, z, n_rows, E, K);
     else if (x_dtype == 1 && w_dtype == 1 && rows_of_eights<bf16, bf16>(x, ldx, w, ldw, K))
-        le = launch_kernel(router_logits_tile_kernel<bf16, bf16>, tiles, dim3(128), 0, s, (const bf16*)x, ldx,
-                           (const bf16*)w, ldw, z, n_rows, E, K);
+        le = launch_router_tiles<bf16, bf16>(x, ldx, w, ldw, z, n_rows, E, K, s);
     else if (x_dtype == 1 && w_dtype == 1)
         le = launch_kernel(router_logits_kernel<bf16, bf16>, dim3(blocks), dim3(256), 0, s, (const bf16*)x, ldx,
                            (const bf16*)w, ldw, z, n_rows, E, K);
     else if (x_dtype == 1 && w_dtype == 0 && rows_of_eights<bf16, float>(x, ldx, w, ldw, K))
-        le = launch_kernel(router_logits_tile_kernel<bf16, float>, tiles, dim3(128), 0, s, (const bf16*)x, ldx,
-                           (const float*)w, ldw, z, n_rows, E, K);
+        le = launch_router_tiles<bf16, float>(x, ldx, w, ldw, z, n_rows, E, K, s);
     else if (x_dtype == 1 && w_dtype == 0)
         le = launch_kernel(router_logits_kernel<bf16, float>, dim3(blocks), dim3(256), 0, s, (const bf16*)x, ldx,
                            (const float*)w, ldw, z, n_rows, E, K);

@@ -344,7 +344,7 @@ def test_experts_of_the_chosen_tokens_only_against_every_expert_for_every_token(
     assert torch.equal(got, again)
 
 
-@pytest.mark.parametrize("rows, experts, hidden", [(1, 1, 8), (3, 17, 264), (8, 16, 2048), (70, 9, 1032), (2049, 16, 320)])
+@pytest.mark.parametrize("rows, experts, hidden", [(1, 1, 8), (3, 17, 264), (5, 2, 264), (6, 3, 1032), (9, 4, 64), (11, 12, 264), (8, 16, 2048), (70, 9, 1032), (2049, 16, 320)])
 @pytest.mark.parametrize("dx, dw", [(torch.bfloat16,) * 2, (torch.float32,) * 2, (torch.bfloat16, torch.float32)])
 def test_router_logits_of_rows_of_eights(rows, experts, hidden, dx, dw):
     """32-bit sums of ``hidden`` products in a fixed order: within sqrt(hidden) roundings of the sum of their sizes, and
